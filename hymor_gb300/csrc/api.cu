@@ -727,6 +727,9 @@ int hymor_ctx_create(const hymor_config* cfg, const hymor_mesh* mesh, hymor_ctx*
   d.step_ffv = 1;
   d.expm_ff = 1;
   d.cfl_screen = 1;
+  d.lanes = 1;
+  d.lane_stride = 0;
+  d.spl_shared = 0;
   d.flux_rows = 4;  // the split tiling
   d.flux_spare = 1;
   d.tma = make_flux_maps(d);

@@ -25,6 +25,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <vector>
 
 #include "ff.cuh"
 #include "kernels.h"
@@ -419,7 +420,16 @@ struct SplineArgs {
   double* ws;
   double lam;
   int n, copy_pts;
+  long lane;  // offset of the next lane's ws and pts (grid z; kernels.h, DevCtx::lane_stride)
 };
+
+// the shock points of lane `off` doubles further
+__device__ __forceinline__ ShockPts lane_pts(const ShockPts& p, long off) {
+  return ShockPts{p.x + off, p.y + off, p.chi + off, p.eta + off};
+}
+__device__ __forceinline__ Cons lane_cons(const Cons& q, long off) {
+  return Cons{q.rho + off, q.ru + off, q.rv + off, q.rE + off};
+}
 
 // Per-row bands of A = R + lam Q^T Q, right-hand sides Q^T y and interval reciprocals,
 // one thread per row (the rows are independent), after copying the shock points of S
@@ -428,24 +438,26 @@ __global__ void __launch_bounds__(128) k_spline_rows(SplineArgs A) {
   const int n = A.n;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double* xs = A.ws;
+  const long off = blockIdx.z * A.lane;
+  const ShockPts pts = lane_pts(A.pts, off);
+  double* xs = A.ws + off;
   double* yx = xs + n;
   double* yy = yx + n;
-  double* d0 = A.ws + 7 * n;
+  double* d0 = xs + 7 * n;
   double* d1 = d0 + n;
   double* d2 = d1 + n;
   double* rx = d2 + n;
   double* ry = rx + n;
-  double* ih = A.ws + 15 * n;  // 1 / (x[k+1] - x[k])
-  const ShockPts& src = A.copy_pts ? A.pS : A.pts;
+  double* ih = xs + 15 * n;  // 1 / (x[k+1] - x[k])
+  const ShockPts& src = A.copy_pts ? A.pS : pts;
   const double lam = A.lam;
   auto X = [&](int k) { return src.chi[k]; };
   xs[i] = src.chi[i];
   yx[i] = src.x[i];
   yy[i] = src.y[i];
   if (A.copy_pts) {
-    A.pts.x[i] = A.pS.x[i]; A.pts.y[i] = A.pS.y[i];
-    A.pts.chi[i] = A.pS.chi[i]; A.pts.eta[i] = A.pS.eta[i];
+    pts.x[i] = A.pS.x[i]; pts.y[i] = A.pS.y[i];
+    pts.chi[i] = A.pS.chi[i]; pts.eta[i] = A.pS.eta[i];
   }
   if (i + 1 < n) ih[i] = 1.0 / (X(i + 1) - X(i));
   const int m = n - 2;
@@ -692,14 +704,15 @@ __global__ void __launch_bounds__(kSplineThreads) k_spline_fit(SplineArgs A) {
   float* shf = reinterpret_cast<float*>(shf4);
   const int n = A.n, m = n - 2, tid = threadIdx.x, nt = blockDim.x;
   const int mp = spline_stride(n);
-  double* xs = A.ws;
+  double* const ws = A.ws + blockIdx.z * A.lane;
+  double* xs = ws;
   double* yx = xs + n;
   double* yy = yx + n;
   double* cx = yy + n;
   double* cy = cx + n;
   double* gx = cy + n;
   double* gy = gx + n;
-  const double* d0 = A.ws + 7 * n;
+  const double* d0 = ws + 7 * n;
   const double* d1 = d0 + n;
   const double* d2 = d1 + n;
   const double* rx = d2 + n;
@@ -725,7 +738,7 @@ __global__ void __launch_bounds__(kSplineThreads) k_spline_fit(SplineArgs A) {
     for (int i = tid; i < n; i += nt) { gx[i] = yx[i]; gy[i] = yy[i]; }
     return;
   }
-  const double* ih = A.ws + 15 * n;
+  const double* ih = ws + 15 * n;
   float qloc = 0.f, yloc = 0.f;  // max 2 (1/h_{k-1} + 1/h_k) and max |y| over this thread's rows
   for (int j = tid; j < m; j += nt) {
     fd0[j] = (float)d0[j]; fd1[j] = (float)d1[j]; fd2[j] = (float)d2[j];
@@ -801,7 +814,7 @@ __global__ void __launch_bounds__(kSplineThreads) k_spline_fit(SplineArgs A) {
   }
   if (direct) {
     if (tid == 0)
-      chol_solve_f64(m, d0, d1, d2, rx, ry, A.ws + 12 * n, A.ws + 13 * n, A.ws + 14 * n, cx, cy);
+      chol_solve_f64(m, d0, d1, d2, rx, ry, ws + 12 * n, ws + 13 * n, ws + 14 * n, cx, cy);
     __syncthreads();
   }
   // fitted values g = y - lam Q gamma
@@ -830,6 +843,7 @@ struct ColArgs {
   double vmag, cph, sph;                  // its speed and flow-angle cosine / sine
   // gas constants of the jump relations: (g+1)/(g-1), 1/(g-1), 2/(g-1)
   double gp1_gm1, igm1, two_igm1;
+  long lane, ws_lane;  // offsets of the next lane's buffers and spline workspace (grid z)
 };
 
 // value and slope of the fitted spline at t (Linear() extrapolation outside the knots)
@@ -894,12 +908,16 @@ __global__ void __launch_bounds__(kColThreads) k_shock_columns(ColArgs A) {
   const int lane = threadIdx.x % kColCols, w = threadIdx.x / kColCols;
   const int i = blockIdx.x * kColCols + lane;
   const bool act = i < nchi;
-  const double* xs = A.ws;
-  const double* cxs = A.ws + 3 * nchi;
-  const double* cys = A.ws + 4 * nchi;
-  const double* gxs = A.ws + 5 * nchi;
-  const double* gys = A.ws + 6 * nchi;
-  const double* ih = A.ws + 15 * nchi;
+  const long off = blockIdx.z * A.lane;
+  const double* xs = A.ws + blockIdx.z * A.ws_lane;
+  const double* cxs = xs + 3 * nchi;
+  const double* cys = xs + 4 * nchi;
+  const double* gxs = xs + 5 * nchi;
+  const double* gys = xs + 6 * nchi;
+  const double* ih = xs + 15 * nchi;
+  const ShockPts pts = lane_pts(A.pts, off);
+  const Cons q = lane_cons(A.tgt, off);
+  double* const P = A.p + off;
   const int I = i + 1;
   // phase 1. LEAST_SQUARES_SHOCK_POINTS.jl:60-70, COMPUTE_BETA.jl:37-50: the fitted spline
   // and its slope at the column's abscissa
@@ -924,11 +942,11 @@ __global__ void __launch_bounds__(kColThreads) k_shock_columns(ColArgs A) {
       sh.i01[lane] = frsqrt(dx01 * dx01 + dy01 * dy01);  // 1 / dist01
       sh.i12[lane] = i12;
       const int g1 = gidx(I, sc - 1, nchi), g2 = gidx(I, sc - 2, nchi);
-      const double p_1 = A.p[g1];
-      double p_2 = A.p[g2];
+      const double p_1 = P[g1];
+      double p_2 = P[g2];
       if (sc - 2 == 0 && c.bc_eta0 == HYMOR_BC_NO_SLIP_ISOTHERMAL)
-        p_2 = 2 * A.p[gidx(I, 1, nchi)] - A.p[gidx(I, 2, nchi)];  // UPDATE_THERMODYNAMIC_PROPERTIES.jl:28-31
-      const double* arr[4] = {A.tgt.rho, A.tgt.ru, A.tgt.rv, A.tgt.rE};
+        p_2 = 2 * P[gidx(I, 1, nchi)] - P[gidx(I, 2, nchi)];  // UPDATE_THERMODYNAMIC_PROPERTIES.jl:28-31
+      const double* arr[4] = {q.rho, q.ru, q.rv, q.rE};
       sh.q1[4][lane] = p_1;
       sh.q2[4][lane] = p_2;
       sh.sl[0][lane] = (p_1 - p_2) * i12;
@@ -947,18 +965,17 @@ __global__ void __launch_bounds__(kColThreads) k_shock_columns(ColArgs A) {
   if (w == 0) {
     double ch, et;
     element_space(c, xv, yv, ch, et);
-    A.pts.chi[i] = ch;
-    A.pts.eta[i] = et;
+    pts.chi[i] = ch;
+    pts.eta[i] = et;
     return;
   }
   // phase 2, warp 1
   const double xd = sh.xd[lane], yd = sh.yd[lane];
   const double t = A.scal[kT], dt = A.scal[kDt];
-  Cons q = A.tgt;
-  A.pts.x[i] = xv; A.pts.y[i] = yv;
+  pts.x[i] = xv; pts.y[i] = yv;
   double p_inf = A.p_inf, u_inf = A.u_inf, v_inf = A.v_inf, rho_inf = A.rho_inf;
   const bool local_up = A.disturbed || A.up_cols || (c.axisymmetric && i == 0);
-  if (local_up) upstream(c, t, xv, yv, i == 0, p_inf, u_inf, v_inf, rho_inf, A.up_cols, i);
+  if (local_up) upstream(c, t, xv, yv, i == 0, p_inf, u_inf, v_inf, rho_inf, A.up_cols ? A.up_cols + off : nullptr, i);
   const double cross = xd * v_inf - yd * u_inf;
   const double dot = xd * u_inf + yd * v_inf;
   // beta = atan2(|cross|, |dot|) enters only through its sine and cosine, |cross| / r and |dot| / r
@@ -1006,7 +1023,7 @@ __global__ void __launch_bounds__(kColThreads) k_shock_columns(ColArgs A) {
   const double temp2 = yr * Acoef + 1;
   const double temp3 = p_inf * (yr - 1) * frcp(rho_inf);
   const double rel = -vn_inf + sqrt(temp3 * temp2 * frcp(temp1));
-  A.rel[i] = rel;
+  A.rel[off + i] = rel;
   const double vt_s = ca * vmag;
   const double vn_s = -rel + rho_inf * irho_s * (rel + vn_inf);
   double spx, spy;
@@ -1018,8 +1035,8 @@ __global__ void __launch_bounds__(kColThreads) k_shock_columns(ColArgs A) {
     spx = sx - sy * (cb * frcp(sb));  // tan(pi/2 - beta) = cos(beta) / sin(beta)
     spy = 0.0;
   }
-  A.speed_x[i] = spx;
-  A.speed_y[i] = spy;
+  A.speed_x[off + i] = spx;
+  A.speed_y[off + i] = spy;
   const double ru_s = rho_s * (vn_s * sb + vt_s * cb);
   const double rv_s = rho_s * (-vn_s * cb + vt_s * sb);
   const double rE_s = e_s * rho_s + (ru_s * ru_s + rv_s * rv_s) * (0.5 * irho_s);
@@ -1030,7 +1047,7 @@ __global__ void __launch_bounds__(kColThreads) k_shock_columns(ColArgs A) {
   v0[2] = -sh.sl[3][lane] * dist0s + rv_s;
   v0[3] = -sh.sl[4][lane] * dist0s + rE_s;
   v0[4] = -slope_p * dist0s + p_s;
-  double* arr[5] = {q.rho, q.ru, q.rv, q.rE, A.p};
+  double* arr[5] = {q.rho, q.ru, q.rv, q.rE, P};
   const int i1 = gidx(I, sc + 1, nchi), i2 = gidx(I, sc + 2, nchi);
 #pragma unroll
   for (int v = 0; v < 5; ++v) arr[v][g0] = v0[v];
@@ -1058,7 +1075,7 @@ __global__ void __launch_bounds__(kColThreads) k_shock_columns(ColArgs A) {
     }
   }
   // MOVE_SHOCK; the symmetry copy pts_x[1] -> pts_x[0] runs in k_bc_edges
-  if (A.move) move_shock_point(c, A.pS, A.pts, A.on_S, A.cY, A.cS, dt, spx, spy, i);
+  if (A.move) move_shock_point(c, A.pS, pts, A.on_S, A.cY, A.cS, dt, spx, spy, i);
 }
 
 // MOVE_SHOCK on its own, after a k_shock_columns launch without it: one CTA moves every
@@ -1095,6 +1112,7 @@ struct BcArgs {
   int phase;     // 0: chi edges, 1: eta edges
   int fix_pts;   // MOVE_SHOCK symmetry copy (phase 0, thread 0)
   int on_S;
+  long lane;     // offset of the next lane's q, p, T, a_bc (grid z)
 };
 
 // point t of the two edges of one phase (0: chi edges, 1: eta edges)
@@ -1107,13 +1125,15 @@ __device__ __forceinline__ void bc_edge_point(const BcArgs& A, int phase, int t)
   const int bc = edge == 0 ? c.bc_chi0 : edge == 1 ? c.bc_chi1 : edge == 2 ? c.bc_eta0 : c.bc_eta1;
   if (bc == HYMOR_BC_SHOCK) return;
   EdgeCtx e{edge, bc, NI, NJ, nchi, neta};
-  edge_bc_point(c, e, A.m, A.q, A.p, A.T, A.a_bc, k, len);
+  const long off = blockIdx.z * A.lane;
+  const Cons q = lane_cons(A.q, off);
+  edge_bc_point(c, e, A.m, q, A.p + off, A.T + off, A.a_bc + off, k, len);
   if (bc == HYMOR_BC_SYMMETRY) {
     // ends of the ghost line copy their neighbours along the line
-    if (k == 1) { A.q.ru[at(e, 0, 0)] = A.q.ru[at(e, 0, 1)]; A.q.rv[at(e, 0, 0)] = A.q.rv[at(e, 0, 1)]; }
+    if (k == 1) { q.ru[at(e, 0, 0)] = q.ru[at(e, 0, 1)]; q.rv[at(e, 0, 0)] = q.rv[at(e, 0, 1)]; }
     if (k == len - 2) {
-      A.q.ru[at(e, 0, len - 1)] = A.q.ru[at(e, 0, len - 2)];
-      A.q.rv[at(e, 0, len - 1)] = A.q.rv[at(e, 0, len - 2)];
+      q.ru[at(e, 0, len - 1)] = q.ru[at(e, 0, len - 2)];
+      q.rv[at(e, 0, len - 1)] = q.rv[at(e, 0, len - 2)];
     }
   }
 }
@@ -1154,6 +1174,7 @@ struct FluxArgs {
   const int* list;
   const int* count;
   int tiles_x;
+  long lane;  // offset of the next lane's inputs and outputs (grid z, the linearisation's launches)
 };
 
 // Tile classes of the RK step, once per step (the shocked rows are fixed within a step):
@@ -1311,6 +1332,8 @@ __device__ __forceinline__ bool flux_tile(const FluxArgs& a, const FluxMaps& tm,
   ff* fTc = reinterpret_cast<ff*>(s_Tc);
 
   const int nchi = a.nchi, neta = a.neta;
+  // the lane of a batched launch (the linearisation's FP64 residuals)
+  const long off = FFV ? 0 : blockIdx.z * a.lane;
   const int i0 = bx * TX, j0 = by * TYV;  // first interior cell (0-based)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // shared index of halo cell (hx, hy) = ghosted (i0 + hx, j0 + hy); with TMA the staged rows
@@ -1344,7 +1367,7 @@ __device__ __forceinline__ bool flux_tile(const FluxArgs& a, const FluxMaps& tm,
     if (j0 + 1 >= sc) {
       const int ci = i0 + lane, cj = j0 + warp;
       if (lane < TX && ci < nchi && cj < neta) {
-        const long c = (long)ci + (long)cj * nchi;
+        const long c = off + (long)ci + (long)cj * nchi;
         a.o0[c] = 0; a.o1[c] = 0; a.o2[c] = 0; a.o3[c] = 0;
       }
       return true;
@@ -1387,7 +1410,7 @@ __device__ __forceinline__ bool flux_tile(const FluxArgs& a, const FluxMaps& tm,
       if (TMA) {
         r = s_r[h]; ru = s_ru[h]; rv = s_rv[h]; T = s_T[h];
       } else {
-        const long g = (long)gi + (long)gj * (nchi + 2);
+        const long g = off + (long)gi + (long)gj * (nchi + 2);
         r = a.rho[g]; ru = a.ru[g]; rv = a.rv[g];
         s_r[h] = r; s_ru[h] = ru; s_rv[h] = rv; s_rE[h] = a.rE[g];
         s_p[h] = a.p[g];
@@ -1588,7 +1611,8 @@ __device__ __forceinline__ bool flux_tile(const FluxArgs& a, const FluxMaps& tm,
         r2 = v2 * rv;
         r3 = (dl[3] + f_bt[3 * G::NBTF + s] - f_bt[3 * G::NBTF + n]) * rv;
       }
-      a.o0[c] = r0; a.o1[c] = r1; a.o2[c] = r2; a.o3[c] = r3;
+      const long o = off + c;
+      a.o0[o] = r0; a.o1[o] = r1; a.o2[o] = r2; a.o3[o] = r3;
     }
   }
   return true;
@@ -2357,8 +2381,9 @@ void launch_spline(const DevCtx& d, bool on_S, bool copy_pts, cudaStream_t st) {
   sa.lam = (1 - c.spline_param) / c.spline_param;
   sa.n = d.nchi;
   sa.copy_pts = copy_pts;
-  k_spline_rows<<<(d.nchi + 127) / 128, 128, 0, st>>>(sa);
-  k_spline_fit<<<1, kSplineThreads, sizeof(float) * kSplineArrays * spline_stride(d.nchi), st>>>(sa);
+  sa.lane = d.lane_stride;
+  k_spline_rows<<<dim3((d.nchi + 127) / 128, 1, d.lanes), 128, 0, st>>>(sa);
+  k_spline_fit<<<dim3(1, 1, d.lanes), kSplineThreads, sizeof(float) * kSplineArrays * spline_stride(d.nchi), st>>>(sa);
 }
 
 void launch_columns_bc(const DevCtx& d, bool on_S, bool move, double cY, double cS, int a_mode, bool do_shock,
@@ -2405,7 +2430,9 @@ void launch_columns_bc(const DevCtx& d, bool on_S, bool move, double cY, double 
     ca.gp1_gm1 = (c.gamma + 1) / (c.gamma - 1);
     ca.igm1 = 1.0 / (c.gamma - 1);
     ca.two_igm1 = 2 / (c.gamma - 1);
-    k_shock_columns<<<(d.nchi + kColCols - 1) / kColCols, kColThreads, 0, st>>>(ca);
+    ca.lane = d.lane_stride;
+    ca.ws_lane = d.spl_shared ? 0 : d.lane_stride;
+    k_shock_columns<<<dim3((d.nchi + kColCols - 1) / kColCols, 1, d.lanes), kColThreads, 0, st>>>(ca);
   }
   const bool fix = shock && move && c.bc_chi0 == HYMOR_BC_SYMMETRY;
   if (do_bc || fix) {
@@ -2425,12 +2452,13 @@ void launch_columns_bc(const DevCtx& d, bool on_S, bool move, double cY, double 
       ba.cfg.bc_chi0 = HYMOR_BC_SHOCK;
       ba.cfg.bc_chi1 = HYMOR_BC_SHOCK;
     }
+    ba.lane = d.lane_stride;
     ba.phase = 0;
-    k_bc_edges<<<(2 * d.NJ + 255) / 256, 256, 0, st>>>(ba);
+    k_bc_edges<<<dim3((2 * d.NJ + 255) / 256, 1, d.lanes), 256, 0, st>>>(ba);
     if (do_bc) {
       ba.phase = 1;
       ba.fix_pts = 0;
-      k_bc_edges<<<(2 * d.NI + 255) / 256, 256, 0, st>>>(ba);
+      k_bc_edges<<<dim3((2 * d.NI + 255) / 256, 1, d.lanes), 256, 0, st>>>(ba);
     }
   }
 }
@@ -2502,14 +2530,44 @@ void launch_classify_tiles(const DevCtx& d, cudaStream_t st) {
                                                    flux_rows(d), flux_split(d), flux_list0_cap(d));
 }
 
+// The tiles that hold the cells (i, sc_i - 1) of the shocked rows `rows` (host copy) as the
+// class-1 list (halves in the split tiling), and the ghosted rows jlo <= j < jhi that those
+// tiles and the jump kernel read (rows sc_i - 2 .. sc_i + 2 of every column included). The
+// class-0 list is left empty.
+void launch_band_tiles(const DevCtx& d, const int* rows, int& jlo, int& jhi, cudaStream_t st) {
+  const int ty = flux_split(d) ? TY / 2 : flux_rows(d), tx = flux_tiles_x(d);
+  std::vector<int> list{0, 0};
+  std::vector<char> hit((size_t)tx * ((d.neta + ty - 1) / ty), 0);
+  jlo = d.NJ;
+  jhi = 0;
+  for (int i = 0; i < d.nchi; ++i) {
+    const int t = i / TX, by = (rows[i] - 2) / ty;  // cell row sc - 1, 0-based sc - 2
+    if (!hit[(size_t)by * tx + t]) {
+      hit[(size_t)by * tx + t] = 1;
+      list.push_back(by * tx + t);
+    }
+    jlo = std::min(jlo, std::min(by * ty, rows[i] - 2));
+    jhi = std::max(jhi, std::max(by * ty + ty + 2, rows[i] + 3));
+  }
+  jlo = std::max(jlo, 0);
+  jhi = std::min(jhi, d.NJ);
+  list[1] = (int)list.size() - 2;
+  cudaMemcpyAsync(d.tiles, list.data(), 2 * sizeof(int), cudaMemcpyHostToDevice, st);
+  cudaMemcpyAsync(d.tiles + 2 + flux_list0_cap(d), list.data() + 2, list[1] * sizeof(int), cudaMemcpyHostToDevice, st);
+}
+
 template <bool AXI, bool SUTH, bool FFV, int TYV, bool TMA>
 void flux_launch_rows(const FluxArgs& a, const FluxMaps& tm, int tile_class, dim3 grid, const DevCtx& d,
                       cudaStream_t st) {
   const size_t smem = flux_smem<AXI, SUTH, TYV, TMA>();
+  grid.z = d.lanes;
   if (tile_class == 1 && a.list) {
     // the shock/boundary class: a persistent grid of one block per SM over its few tiles (two
     // of the half-height tiles)
-    k_flux<AXI, SUTH, TYV, FFV, TMA><<<d.sms * (TYV == TY / 2 ? 2 : 1), 32 * TYV, smem, st>>>(a, tm);
+    // over many lanes, as many blocks as tiles at most: the lanes fill the SMs
+    const int per = d.sms * (TYV == TY / 2 ? 2 : 1);
+    const int bx = d.lanes > 1 ? std::min(per, std::max(1, 4 * per / d.lanes)) : per;
+    k_flux<AXI, SUTH, TYV, FFV, TMA><<<dim3(bx, 1, d.lanes), 32 * TYV, smem, st>>>(a, tm);
   } else {
     k_flux<AXI, SUTH, TYV, FFV, TMA><<<grid, 32 * TYV, smem, st>>>(a, tm);
   }
@@ -2545,6 +2603,7 @@ void launch_flux_class(const DevCtx& d, bool on_S, double* const out[4], int til
   a.cell_idx = d.cell_idx;
   a.m = d.m;
   a.err = d.err;
+  a.lane = d.lane_stride;
   // the split tiling's classes: half-height tiles, halo by thread loads
   const bool half = flux_split(d) && tile_class >= 0 && d.tiles;
   const int rows = half ? TY / 2 : flux_rows(d);

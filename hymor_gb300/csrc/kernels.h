@@ -82,6 +82,13 @@ struct DevCtx {
   // by thread.
   CUtensorMap tmS[2][4], tmY[2][4], tmP[2], tmT[2];
   int tma;
+  // residuals of several perturbed states in one launch per kernel (the linearisation): the
+  // grid's z runs over `lanes` copies of the lane-owned arrays (Y, p, T, aY, spl, the shock
+  // speeds, Yp, up_cols, the flux), lane_stride doubles apart. 1 and 0 everywhere else.
+  // spl_shared: the lanes read one spline workspace (their shock points are the same).
+  int lanes;
+  long lane_stride;
+  int spl_shared;
 };
 
 // Unknowns of the linearised operator: 4N, plus Nchi with the shock blocks.
@@ -118,6 +125,9 @@ void launch_flux_class(const DevCtx& d, bool on_S, double* const out[4], int til
                        int spare = 0, bool ffv = false);
 // Classifies the flux tiles of the current shocked rows into d.tiles.
 void launch_classify_tiles(const DevCtx& d, cudaStream_t st);
+// The tiles that hold the cells (i, sc_i - 1) (rows: sc_i on the host) as d.tiles' class 1, and
+// the ghosted rows jlo <= j < jhi their flux reads.
+void launch_band_tiles(const DevCtx& d, const int* rows, int& jlo, int& jhi, cudaStream_t st);
 int flux_tiles(const DevCtx& d);
 int flux_tiles_max(const DevCtx& d);  // the tile count of the smallest tile height (list sizes)
 // UPDATE_FLOW_CELLS part 1: detect shocked cells, upstream fill, extrapolation (on S).

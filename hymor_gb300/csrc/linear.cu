@@ -67,6 +67,9 @@ Wrap make_wrap(const hymor_config& c) {
 // raised by flow_cells * eps; then p, T of Y. shock_row = j > 0 raises instead the
 // cell (i, sc_i - j) of every column by eps (the flow-to-shock-speed perturbations,
 // :140-258).
+// Lane z of a batched launch (DevCtx::lane_stride) evaluates the perturbation `first + z`:
+// colour and variable of the A11 colours (var * 9 + colour - 1, when `colours`), else the
+// members as they are.
 struct PertArgs {
   Cons S, Y;
   double *p, *T;
@@ -75,15 +78,29 @@ struct PertArgs {
   const int* cell_idx;
   double eps, gm1;
   int nchi, neta, var, colour, shock, shock_row;
+  int j0, j1;        // rows written, j0 <= j < j1 (ghosted)
+  long lane;
+  int first, batch;  // batch: 0 one perturbation; 1 the A11 colours; 2 the A21 rows (j, var)
 };
 
 __global__ void k_perturb_thermo(PertArgs a) {
+  const long off = blockIdx.z * a.lane;
+  a.Y.rho += off; a.Y.ru += off; a.Y.rv += off; a.Y.rE += off;
+  a.p += off; a.T += off; a.aY += off;
+  const int id = a.first + blockIdx.z;
+  if (a.batch == 1) {
+    a.var = id / 9;
+    a.colour = id % 9 + 1;
+  } else if (a.batch == 2) {
+    a.shock_row = id / 4 + 1;
+    a.var = id % 4;
+  }
   const int NI = a.nchi + 2;
-  const long G = (long)NI * (a.neta + 2);
+  const long G = (long)NI * a.j1;
   const int si = (a.colour % 3 == 0) ? 3 : a.colour % 3;  // 1-based start in chi
   const int sj = (a.colour + 2) / 3;                       // 1-based start in eta
-  for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < G; k += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(k % NI), j = (int)(k / NI);
+  for (long k = (long)NI * a.j0 + blockIdx.x * (long)blockDim.x + threadIdx.x; k < G; k += (long)gridDim.x * blockDim.x) {
+    const int j = (int)((unsigned)k / (unsigned)NI), i = (int)((unsigned)k - (unsigned)j * (unsigned)NI);
     double v[4] = {a.S.rho[k], a.S.ru[k], a.S.rv[k], a.S.rE[k]};
     if (a.var >= 0 && i >= 1 && i <= a.nchi && j >= 1 && j <= a.neta) {
       if (a.shock_row) {
@@ -109,41 +126,74 @@ __global__ void k_perturb_thermo(PertArgs a) {
   }
 }
 
-// coef[plane(q, vo, var)][m] = (Fp[vo][m] - Fb[vo][m]) / eps for every slot q whose
-// input cell m + offset(q) has the perturbed colour (GET_OUTPUT_INDEXING_A11,
-// LINEARIZE_EQUATIONS_NO_DISCONTINUITY.jl:306-788; REMOVE_BASE_OUTPUT :935-946).
+// coef[plane(q, vo, var)][m] = (Fp[vo][m] - Fb[vo][m]) / eps with Fp the residual of the colour
+// of slot q's input cell m + offset(q) (GET_OUTPUT_INDEXING_A11,
+// LINEARIZE_EQUATIONS_NO_DISCONTINUITY.jl:306-788; REMOVE_BASE_OUTPUT :935-946), for one
+// variable (grid z: first_var + z) whose nine colours are nine consecutive lanes. A thread
+// takes a cell and loops over its slots, so that a warp writes whole rows of a plane and its
+// reads of the three colours of a row of slots share their lines in L1; one colour at a time
+// every warp wrote a third of the sectors of three planes. Linearisation at 600 x 300: 3.29 ms
+// with a pass per colour, 2.70 ms so.
 struct ScatArgs {
   const double* Fp[4];
   const double* Fb[4];
   double* coef;
   Wrap w;
-  double inv_eps_dummy;
-  double eps;
-  int var, colour;
+  double eps, inv_eps;  // inv_eps: the rounded reciprocal of eps, 0 to divide
   long N;
+  long lane;
+  int first_var;
 };
 
-__global__ void k_scatter(ScatArgs a) {
-  const long N = a.N;
-  const int si = (a.colour % 3 == 0) ? 3 : a.colour % 3;
-  const int sj = (a.colour + 2) / 3;
+// d / eps, correctly rounded. The FP64 division of the compiler takes ~25 FP64 instructions
+// and this GPU issues one per ~70 cycles, so that the four quotients of a cell bounded the
+// scatter. With y = RN(1 / eps): q0 = d y is within two ulps; one residual correction
+// (r = d - eps q0 exact by FMA) makes it faithful, and by Markstein's theorem (IBM J. Res.
+// Dev. 34 (1990) 111-119) the second gives the rounded quotient: five instructions. Outside
+// the exponents where every step is exact (d below 2^-500, infinite or NaN) it divides; the
+// host gives inv_eps = 0 for an eps whose reciprocal the theorem leaves out (significand of
+// all ones) or whose exponent is extreme. 600 x 300, one colour's scatter: 35.7 -> 25.4 us.
+__device__ __forceinline__ double div_eps(double d, double eps, double y) {
+  const unsigned e = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
+  if (y != 0.0) {
+    if ((__double_as_longlong(d) << 1) == 0) return d;  // +-0 / eps, eps > 0
+    if (e - 523u < 1000u) {
+      double q = d * y;
+      q = fma(fma(-eps, q, d), y, q);
+      return fma(fma(-eps, q, d), y, q);
+    }
+  }
+  return d / eps;
+}
+// the rounded reciprocal of eps for div_eps, or 0
+double div_eps_reciprocal(double eps) {
+  int ex = 0;
+  const double m = std::frexp(std::fabs(eps), &ex);
+  if (!(eps > 0) || !(m < 1) || ex < -200 || ex > 200 || m == 1.0 - 0x1p-53) return 0.0;
+  return 1.0 / eps;
+}
+
+__global__ void __launch_bounds__(256) k_scatter(ScatArgs a) {
+  const long N = a.N, off = 9L * blockIdx.z * a.lane;
+  const int var = a.first_var + blockIdx.z;
+  const unsigned nchi_u = (unsigned)a.w.nchi;
   for (long m = blockIdx.x * (long)blockDim.x + threadIdx.x; m < N; m += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(m % a.w.nchi), j = (int)(m / a.w.nchi);
-    double d[4];
+    const int j = (int)((unsigned)m / nchi_u), i = (int)((unsigned)m - (unsigned)j * nchi_u);
+    double fb[4];
 #pragma unroll
-    for (int vo = 0; vo < 4; ++vo) d[vo] = (a.Fp[vo][m] - a.Fb[vo][m]) / a.eps;
+    for (int vo = 0; vo < 4; ++vo) fb[vo] = a.Fb[vo][m];
 #pragma unroll
     for (int b = -1; b <= 1; ++b)
 #pragma unroll
       for (int aa = -1; aa <= 1; ++aa) {
         const long n = a.w.nbr(i, j, aa, b);
         if (n < 0) continue;
-        const int ni = (int)(n % a.w.nchi) + 1, nj = (int)(n / a.w.nchi) + 1;  // 1-based
-        const bool hit = (ni >= si) && ((ni - si) % 3 == 0) && (nj >= sj) && ((nj - sj) % 3 == 0);
-        if (!hit) continue;
+        const unsigned nj = (unsigned)n / nchi_u, ni = (unsigned)n - nj * nchi_u;
+        const long o = off + (long)(3 * (nj % 3u) + ni % 3u) * a.lane + m;  // the input cell's colour
         const int q = (b + 1) * 3 + (aa + 1);
 #pragma unroll
-        for (int vo = 0; vo < 4; ++vo) a.coef[((long)(q * 4 + vo) * 4 + a.var) * N + m] = d[vo];
+        for (int vo = 0; vo < 4; ++vo)
+          a.coef[((long)(q * 4 + vo) * 4 + var) * N + m] = div_eps(a.Fp[vo][o] - fb[vo], a.eps, a.inv_eps);
       }
   }
 }
@@ -788,11 +838,15 @@ __global__ void k_shock_dir(const double* beta, double* dir, int nchi, double cp
 }
 
 // Y's shock points = S's, point p displaced by eps along its PERTURB_SHOCK direction.
-__global__ void k_perturb_point(ShockPts S, ShockPts Y, const double* dir, int nchi, int p, double eps) {
+// Lane z of a batched launch displaces point first + z.
+__global__ void k_perturb_point(ShockPts S, ShockPts Y, const double* dir, int nchi, int first, double eps,
+                                long lane) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nchi) return;
+  const long off = blockIdx.z * lane;
+  Y = ShockPts{Y.x + off, Y.y + off, Y.chi + off, Y.eta + off};
   double x = S.x[i], y = S.y[i];
-  if (i == p) {
+  if (i == first + (int)blockIdx.z) {
     x = x + eps * dir[i];
     y = y + eps * dir[nchi + i];
   }
@@ -804,10 +858,11 @@ __global__ void k_perturb_point(ShockPts S, ShockPts Y, const double* dir, int n
 
 // A21 column (j, var) of every point: (speed_i(x + eps e) - speed_i(x)) / eps
 // (GET_OUTPUT_INDEXING_A21, :800-820; REMOVE_BASE_OUTPUT, :935-946)
-__global__ void k_gather_a21(const double* rel, const double* rel_b, double* a21, int nchi, int col, double eps) {
+__global__ void k_gather_a21(const double* rel, const double* rel_b, double* a21, int nchi, int first, double eps,
+                             long lane) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nchi) return;
-  a21[i * 8 + col] = (rel[i] - rel_b[i]) / eps;
+  a21[i * 8 + first + blockIdx.z] = (rel[blockIdx.z * lane + i] - rel_b[i]) / eps;
 }
 
 // A12 and A22 columns of point p (GET_OUTPUT_INDEXING_A12_A22, :854-903): the flux of the
@@ -816,13 +871,15 @@ struct Flux4 {
   const double* v[4];
 };
 __global__ void k_gather_a12(Flux4 Fp, Flux4 Fb, const double* rel, const double* rel_b, const int* rows,
-                             double* a12, double* a22, int nchi, int p, double eps) {
+                             double* a12, double* a22, int nchi, int first, double eps, long lane) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nchi) return;
+  const long off = blockIdx.z * lane;
+  const int p = first + blockIdx.z;
   const long m = i + (long)(rows[i] - 2) * nchi;
 #pragma unroll
-  for (int v = 0; v < 4; ++v) a12[((long)v * nchi + i) * nchi + p] = (Fp.v[v][m] - Fb.v[v][m]) / eps;
-  a22[(long)i * nchi + p] = (rel[i] - rel_b[i]) / eps;
+  for (int v = 0; v < 4; ++v) a12[((long)v * nchi + i) * nchi + p] = (Fp.v[v][off + m] - Fb.v[v][m]) / eps;
+  a22[(long)i * nchi + p] = (rel[off + i] - rel_b[i]) / eps;
 }
 
 // out (cols x rows) = in (rows x cols) transposed, both row-major
@@ -923,10 +980,16 @@ __global__ void __launch_bounds__(kShockThreads) k_shock_mv(ShockMvArgs a) {
 
 // Per-column upstream state: the freestream, with variable `var` of the columns i = colour
 // (mod 3) raised by eps (LINEARIZE_B.jl:49-70; var < 0: the unperturbed state).
+// Lane z of a batched launch (lane > 0) raises variable (first + z) / 3 of colour (first + z) % 3.
 __global__ void k_up_cols(double* cols, int nchi, double r0, double ru0, double rv0, double rE0, int var,
-                          int colour, double eps) {
+                          int colour, double eps, int first = 0, long lane = 0) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nchi) return;
+  cols += blockIdx.z * lane;
+  if (lane) {
+    var = (first + (int)blockIdx.z) / 3;
+    colour = (first + (int)blockIdx.z) % 3;
+  }
   const double f[4] = {r0, ru0, rv0, rE0};
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
@@ -939,9 +1002,11 @@ __global__ void k_up_cols(double* cols, int nchi, double r0, double ru0, double 
 // column m is the one of this colour; its entries are the flux change of the cell
 // (m, sc_m - 1) and the change of speed m over eps.
 __global__ void k_gather_b(Flux4 Fp, Flux4 Fb, const double* rel, const double* rel_b, const int* rows, double* bq,
-                           double* bs, int nchi, int var, int colour, double eps) {
+                           double* bs, int nchi, int first, double eps, long lane) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= nchi) return;
+  const long off = blockIdx.z * lane;
+  const int var = (first + (int)blockIdx.z) / 3, colour = (first + (int)blockIdx.z) % 3;
   int d = 2;  // the offset in -1..1 whose column has this colour
   for (int dd = -1; dd <= 1; ++dd)
     if (((m + dd) % 3 + 3) % 3 == colour) d = dd;
@@ -950,8 +1015,8 @@ __global__ void k_gather_b(Flux4 Fp, Flux4 Fb, const double* rel, const double* 
   const long cell = m + (long)(rows[m] - 2) * nchi;
 #pragma unroll
   for (int vo = 0; vo < 4; ++vo)
-    bq[((m * 3 + d + 1) * 4 + vo) * 4 + var] = (Fp.v[vo][cell] - Fb.v[vo][cell]) / eps;
-  if (bs) bs[(m * 3 + d + 1) * 4 + var] = (rel[m] - rel_b[m]) / eps;
+    bq[((m * 3 + d + 1) * 4 + vo) * 4 + var] = (Fp.v[vo][off + cell] - Fb.v[vo][cell]) / eps;
+  if (bs) bs[(m * 3 + d + 1) * 4 + var] = (rel[off + m] - rel_b[m]) / eps;
 }
 
 struct RecArgs {
@@ -1254,57 +1319,85 @@ void launch_expm(const DevCtx& d, int k, double dt, int nsteps, int order, const
 
 // Workspaces of the perturbed residuals of a linearisation (the A11 colours, the shock-point
 // residuals, LINEARIZE_B's columns): each lane has its own stage array, p, T, edge sound
-// speed, shock points, spline workspace, shock speeds, prescribed upstream columns and flux,
-// and its own stream, so that the residuals of different perturbations run concurrently. The
-// base state, the mesh, the base flux and the assembled blocks are shared: read-only, or
-// written at entries no other perturbation writes, with the same arithmetic as one after
-// another, so the result does not depend on the lanes.
-constexpr int kJacLanes = 8;
+// speed, shock points, spline workspace, shock speeds, prescribed upstream columns and flux.
+// The lanes form two groups with a stream each; a group evaluates one perturbation per lane,
+// every kernel launched once for all its lanes (grid z), and the other group's launches run
+// beside it. The base state, the mesh, the base flux and the assembled blocks are shared:
+// read-only, or written at entries no other perturbation writes, with the same arithmetic as
+// one after another, so the result does not depend on the lanes.
+// One launch per kernel and group instead of one per residual, because the ~9 launches of a
+// residual cost the host ~2 us each: the assembly with the shock unknowns at 200 x 100 (245
+// residuals) took 4.2 ms, bound by them, and takes 1.06 ms so (with its point residuals on the
+// shock band's tiles only). Lanes per group: enough cells to fill the GPU (1.2 M), at least 9
+// and at most 32; the 36 colours take 9 or 18 at a time (one or two variables).
+constexpr int kLaneGroups = 2;
+constexpr int kMaxGroupLanes = 32;
 static PertArgs pert_args(const DevCtx& d);
 struct JacLane {
-  cudaStream_t st = nullptr;
-  cudaEvent_t done = nullptr;
-  double* mem = nullptr;
   Cons Y;
   double *p, *T, *aY, *spl, *speed_x, *speed_y, *rel, *cols;
   ShockPts Yp;
   double* F[4];
 };
 struct JacLanes {
-  std::vector<JacLane> lane;
+  JacLane first[kLaneGroups];  // the first lane of each group; the next is `stride` doubles on
+  cudaStream_t st[kLaneGroups] = {};
+  cudaEvent_t done[kLaneGroups] = {};
   cudaEvent_t fork = nullptr;
+  double* mem = nullptr;
+  long stride = 0;
+  int per_group = 0;
 };
+int lanes_per_group(long N) {
+  const long want = (1200000 + N - 1) / N;
+  for (int g : {9, 18})
+    if (want <= g) return g;
+  return kMaxGroupLanes;
+}
 
-// The lane's view of the context: its own buffers in place of the shared ones. TMA
-// descriptors name the context's own stage array, so a lane loads its halo thread by thread
-// (the same values, the same arithmetic).
-DevCtx lane_ctx(const DevCtx& d, const JacLane& l) {
+// The group's view of the context: its lanes' buffers in place of the shared ones, `count` of
+// them. TMA descriptors name the context's own stage array, so a lane loads its halo thread by
+// thread (the same values, the same arithmetic). own_fit: each lane fits its own shock points
+// (else they are S's, and all read the fit that the base residual left in the context's
+// workspace).
+DevCtx lane_ctx(const DevCtx& d, const JacLanes& L, int group, int count, bool own_fit = false) {
   DevCtx ld = d;
+  const JacLane& l = L.first[group];
   ld.Y = l.Y;
   ld.p = l.p;
   ld.T = l.T;
   ld.aY = l.aY;
-  ld.spl = l.spl;
+  if (own_fit) ld.spl = l.spl;
+  ld.spl_shared = !own_fit;
   ld.speed_x = l.speed_x;
   ld.speed_y = l.speed_y;
   ld.rel = l.rel;
   ld.Yp = l.Yp;
   ld.tma = 0;
   if (d.up_cols) ld.up_cols = l.cols;
+  ld.lanes = count;
+  ld.lane_stride = L.stride;
   return ld;
 }
 
-// every lane waits for the work enqueued on st so far
+// every group waits for the work enqueued on st so far
 void lanes_fork(JacLanes& L, cudaStream_t st) {
   cudaEventRecord(L.fork, st);
-  for (JacLane& l : L.lane) cudaStreamWaitEvent(l.st, L.fork, 0);
+  for (cudaStream_t s : L.st) cudaStreamWaitEvent(s, L.fork, 0);
 }
-// st waits for every lane
+// st waits for every group
 void lanes_join(JacLanes& L, cudaStream_t st) {
-  for (JacLane& l : L.lane) {
-    cudaEventRecord(l.done, l.st);
-    cudaStreamWaitEvent(st, l.done, 0);
+  for (int g = 0; g < kLaneGroups; ++g) {
+    cudaEventRecord(L.done[g], L.st[g]);
+    cudaStreamWaitEvent(st, L.done[g], 0);
   }
+}
+// run(first perturbation, group, lanes) over n perturbations, at most `most` at a time
+template <class Run>
+static void for_groups(const JacLanes& L, int n, int most, Run run) {
+  const int g = std::min(most, L.per_group);
+  int group = 0;
+  for (int q = 0; q < n; q += g, group = (group + 1) % kLaneGroups) run(q, group, std::min(g, n - q));
 }
 
 // The shock-position blocks (perturb_shock), after the A11 assembly has left the base
@@ -1317,49 +1410,52 @@ void lanes_join(JacLanes& L, cudaStream_t st) {
 //     a column are exact zeros. 8 residuals (j = 1, 2; 4 variables), no flux needed.
 //   A12, A22 (:262-274): one residual per shock point, the point moved by eps along the
 //     PERTURB_SHOCK direction (the smoothing spline couples every point to every other).
-void launch_shock_assemble(DevCtx& d, const double* const Fb[4], PertArgs pa, JacLanes& L, cudaStream_t st) {
+//     Only the flux of the cells (i, sc_i - 1) and the speeds are read: the residuals cover the
+//     tiles that hold those cells (launch_band_tiles; the same per-cell arithmetic as the whole
+//     grid) and copy only the rows those tiles read; what the boundary kernels make of the
+//     other rows is not used. hrows: the shocked rows on the host.
+void launch_shock_assemble(DevCtx& d, const double* const Fb[4], JacLanes& L, const int* hrows, cudaStream_t st) {
   const hymor_config& c = d.cfg;
   const int nchi = d.nchi;
   const int cb = (nchi + 127) / 128;
   const double eps = c.perturbation_magnitude;
   const double h = std::hypot(c.rho_u_0, c.rho_v_0);
-  const int K = (int)L.lane.size();
   k_shock_dir<<<cb, 128, 0, st>>>(d.beta, d.sj.dir, nchi, c.rho_u_0 / h, c.rho_v_0 / h);
   cudaMemcpyAsync(d.sj.rows, d.cell_idx, sizeof(int) * nchi, cudaMemcpyDeviceToDevice, st);
-  // only the flux of the cells (i, sc_i - 1) is read: the tiles whose halo the shock and
-  // boundary kernels write (class 1 of the step's tile lists) hold them all, and compute
-  // them with the same per-cell arithmetic as the whole grid
-  launch_classify_tiles(d, st);
+  int jlo = 0, jhi = 0;
+  launch_band_tiles(d, hrows, jlo, jhi, st);
   lanes_fork(L, st);
-  int q = 0;
-  for (int j = 1; j <= 2; ++j)
-    for (int var = 0; var < 4; ++var, ++q) {
-      const JacLane& l = L.lane[q % K];
-      const DevCtx ld = lane_ctx(d, l);
-      PertArgs pl = pert_args(ld);
-      pl.var = var;
-      pl.shock_row = j;
-      k_perturb_thermo<<<grid_for(d.G, 256), 256, 0, l.st>>>(pl);
-      launch_shock_bc_flags(ld, false, true, true, false, 0, l.st);
-      k_gather_a21<<<cb, 128, 0, l.st>>>(ld.rel, d.sj.rel_b, d.sj.a21, nchi, (j - 1) * 4 + var, eps);
-    }
+  for_groups(L, 8, 4, [&](int q, int group, int n) {
+    const DevCtx ld = lane_ctx(d, L, group, n);
+    cudaStream_t ls = L.st[group];
+    PertArgs pl = pert_args(ld);
+    pl.first = q;
+    pl.batch = 2;
+    pl.j0 = jlo;
+    pl.j1 = jhi;
+    k_perturb_thermo<<<dim3(grid_for((long)d.NI * (jhi - jlo), 256), 1, n), 256, 0, ls>>>(pl);
+    launch_columns_bc(ld, false, false, 0, 0, 0, true, false, ls);
+    k_gather_a21<<<dim3(cb, 1, n), 128, 0, ls>>>(ld.rel, d.sj.rel_b, d.sj.a21, nchi, q, eps, L.stride);
+  });
   Flux4 fb;
   for (int v = 0; v < 4; ++v) fb.v[v] = Fb[v];
-  for (int p = 0; p < nchi; ++p, ++q) {
-    const JacLane& l = L.lane[q % K];
-    const DevCtx ld = lane_ctx(d, l);
-    PertArgs pl = pert_args(ld);
-    pl.var = -1;
-    pl.shock_row = 0;
+  for_groups(L, nchi, kMaxGroupLanes, [&](int q, int group, int n) {
+    const DevCtx ld = lane_ctx(d, L, group, n, true);
+    cudaStream_t ls = L.st[group];
+    const JacLane& l = L.first[group];
     Flux4 fp;
     for (int v = 0; v < 4; ++v) fp.v[v] = l.F[v];
     double* const Fp[4] = {l.F[0], l.F[1], l.F[2], l.F[3]};
-    k_perturb_thermo<<<grid_for(d.G, 256), 256, 0, l.st>>>(pl);
-    k_perturb_point<<<cb, 128, 0, l.st>>>(d.Sp, ld.Yp, d.sj.dir, nchi, p, eps);
-    launch_shock_bc_flags(ld, false, false, true, true, 0, l.st);
-    launch_flux_class(ld, false, Fp, 1, l.st);
-    k_gather_a12<<<cb, 128, 0, l.st>>>(fp, fb, ld.rel, d.sj.rel_b, d.sj.rows, d.sj.a12, d.sj.a22, nchi, p, eps);
-  }
+    PertArgs pl = pert_args(ld);
+    pl.j0 = jlo;
+    pl.j1 = jhi;
+    k_perturb_thermo<<<dim3(grid_for((long)d.NI * (jhi - jlo), 256), 1, n), 256, 0, ls>>>(pl);
+    k_perturb_point<<<dim3(cb, 1, n), 128, 0, ls>>>(d.Sp, ld.Yp, d.sj.dir, nchi, q, eps, L.stride);
+    launch_shock_bc_flags(ld, false, false, true, true, 0, ls);
+    launch_flux_class(ld, false, Fp, 1, ls);
+    k_gather_a12<<<dim3(cb, 1, n), 128, 0, ls>>>(fp, fb, ld.rel, d.sj.rel_b, d.sj.rows, d.sj.a12, d.sj.a22, nchi, q,
+                                                 eps, L.stride);
+  });
   lanes_join(L, st);
   k_transpose<<<grid_for(4L * nchi * nchi, 256), 256, 0, st>>>(d.sj.a12, d.sj.a12t, 4L * nchi, nchi);
   k_transpose<<<grid_for((long)nchi * nchi, 256), 256, 0, st>>>(d.sj.a22, d.sj.a22t, nchi, nchi);
@@ -1384,10 +1480,15 @@ static PertArgs pert_args(const DevCtx& d) {
              ((c.bc_eta0 == HYMOR_BC_OUTFLOW_NRCBC) << 2) | ((c.bc_eta1 == HYMOR_BC_OUTFLOW_NRCBC) << 3);
   pa.var = -1;
   pa.colour = 1;
+  pa.j0 = 0;
+  pa.j1 = d.NJ;
+  pa.lane = d.lane_stride;
+  pa.first = 0;
+  pa.batch = 0;
   return pa;
 }
 
-void launch_jacobian_assemble(DevCtx& d, cudaStream_t st, JacLanes& L) {
+void launch_jacobian_assemble(DevCtx& d, cudaStream_t st, JacLanes& L, const int* hrows) {
   ++d.coef_version;
   const hymor_config& c = d.cfg;
   const long N = d.N;
@@ -1407,30 +1508,30 @@ void launch_jacobian_assemble(DevCtx& d, cudaStream_t st, JacLanes& L) {
   sa.coef = d.coef;
   sa.w = make_wrap(c);
   sa.eps = c.perturbation_magnitude;
+  sa.inv_eps = div_eps_reciprocal(sa.eps);
   sa.N = N;
-  // the 36 colour x variable residuals, spread over the lanes
-  const int K = (int)L.lane.size();
+  sa.lane = L.stride;
+  // the 36 colour x variable residuals over the lanes; the shock points of all are S's, so
+  // the smoothing-spline fit of the base residual serves them
   lanes_fork(L, st);
-  int q = 0;
-  for (int var = 0; var < 4; ++var)
-    for (int colour = 1; colour <= 9; ++colour, ++q) {
-      const JacLane& l = L.lane[q % K];
-      const DevCtx ld = lane_ctx(d, l);
-      PertArgs pl = pert_args(ld);
-      pl.var = var;
-      pl.colour = colour;
-      double* const Fp[4] = {l.F[0], l.F[1], l.F[2], l.F[3]};
-      k_perturb_thermo<<<grid_for(d.G, 256), 256, 0, l.st>>>(pl);
-      launch_shock_bc_flags(ld, false, true, c.shock_enabled, true, 0, l.st);
-      launch_flux(ld, false, Fp, l.st);
-      ScatArgs sl = sa;
-      for (int v = 0; v < 4; ++v) sl.Fp[v] = l.F[v];
-      sl.var = var;
-      sl.colour = colour;
-      k_scatter<<<grid_for(N, 256), 256, 0, l.st>>>(sl);
-    }
+  for_groups(L, 36, L.per_group >= 18 ? 18 : 9, [&](int q, int group, int n) {
+    const DevCtx ld = lane_ctx(d, L, group, n);
+    cudaStream_t ls = L.st[group];
+    const JacLane& l = L.first[group];
+    PertArgs pl = pert_args(ld);
+    pl.first = q;
+    pl.batch = 1;
+    double* const Fp[4] = {l.F[0], l.F[1], l.F[2], l.F[3]};
+    k_perturb_thermo<<<dim3(grid_for(d.G, 256), 1, n), 256, 0, ls>>>(pl);
+    launch_columns_bc(ld, false, false, 0, 0, 0, c.shock_enabled, true, ls);
+    launch_flux(ld, false, Fp, ls);
+    ScatArgs sl = sa;
+    for (int v = 0; v < 4; ++v) sl.Fp[v] = l.F[v];
+    sl.first_var = q / 9;
+    k_scatter<<<dim3(grid_for(N, 256), 1, n / 9), 256, 0, ls>>>(sl);
+  });
   lanes_join(L, st);
-  if (shock_blocks) launch_shock_assemble(d, Fb, pa, L, st);
+  if (shock_blocks) launch_shock_assemble(d, Fb, L, hrows, st);
 }
 
 // LINEARIZE_B (Freestream_receptivity/LINEARIZE_B.jl:40-170): the residual with a prescribed
@@ -1460,24 +1561,23 @@ void launch_b_assemble(DevCtx& d, cudaStream_t st, JacLanes& L) {
   launch_shock_bc_flags(d, false, true, true, true, 0, st);
   launch_flux(d, false, Fb, st);
   cudaMemcpyAsync(rel_b, d.rel, sizeof(double) * nchi, cudaMemcpyDeviceToDevice, st);
-  // one residual per variable and colour of columns, spread over the lanes (each with its own
-  // upstream columns)
-  const int K = (int)L.lane.size();
+  // one residual per variable and colour of columns, over the lanes (each with its own upstream
+  // columns; the shock points are S's, so the base residual's fit serves them all)
   lanes_fork(L, st);
-  int q = 0;
-  for (int var = 0; var < 4; ++var)
-    for (int colour = 0; colour < 3; ++colour, ++q) {
-      const JacLane& l = L.lane[q % K];
-      const DevCtx ld = lane_ctx(d, l);
-      Flux4 fp;
-      for (int v = 0; v < 4; ++v) fp.v[v] = l.F[v];
-      double* const Fp[4] = {l.F[0], l.F[1], l.F[2], l.F[3]};
-      k_up_cols<<<cb, 128, 0, l.st>>>(l.cols, nchi, c.rho_0, c.rho_u_0, c.rho_v_0, c.rho_E_0, var, colour, eps);
-      k_perturb_thermo<<<grid_for(d.G, 256), 256, 0, l.st>>>(pert_args(ld));
-      launch_shock_bc_flags(ld, false, true, true, true, 0, l.st);
-      launch_flux(ld, false, Fp, l.st);
-      k_gather_b<<<cb, 128, 0, l.st>>>(fp, fb, ld.rel, rel_b, d.brows, d.bq, d.bs, nchi, var, colour, eps);
-    }
+  for_groups(L, 12, 6, [&](int q, int group, int n) {
+    const DevCtx ld = lane_ctx(d, L, group, n);
+    cudaStream_t ls = L.st[group];
+    const JacLane& l = L.first[group];
+    Flux4 fp;
+    for (int v = 0; v < 4; ++v) fp.v[v] = l.F[v];
+    double* const Fp[4] = {l.F[0], l.F[1], l.F[2], l.F[3]};
+    k_up_cols<<<dim3(cb, 1, n), 128, 0, ls>>>(l.cols, nchi, c.rho_0, c.rho_u_0, c.rho_v_0, c.rho_E_0, 0, 0, eps, q,
+                                              L.stride);
+    k_perturb_thermo<<<dim3(grid_for(d.G, 256), 1, n), 256, 0, ls>>>(pert_args(ld));
+    launch_columns_bc(ld, false, false, 0, 0, 0, true, true, ls);
+    launch_flux(ld, false, Fp, ls);
+    k_gather_b<<<dim3(cb, 1, n), 128, 0, ls>>>(fp, fb, ld.rel, rel_b, d.brows, d.bq, d.bs, nchi, q, eps, L.stride);
+  });
   lanes_join(L, st);
   d.up_cols = nullptr;
 }
@@ -1611,36 +1711,49 @@ LinearState& linear_state(hymor_ctx* ctx) {
 }
 ExpmCache& expm_cache(hymor_ctx* ctx) { return linear_state(ctx).expm; }
 
-// The linearisation lanes, made on first use (kJacLanes x ~(7 G + 4 N) doubles).
+// The linearisation lanes, made on first use (2 groups of 9 to 32 x ~(11 N + 7 ..) doubles).
 int ensure_lanes(hymor_ctx* ctx, JacLanes** out) {
   JacLanes& L = linear_state(ctx).lanes;
   *out = &L;
-  if (!L.lane.empty()) return 0;
+  if (L.mem) return 0;
   const DevCtx& d = ctx_dev(ctx);
   const size_t G = d.G, N = d.N, n = d.nchi;
   auto pad = [](size_t k) { return (k + 31) & ~size_t(31); };  // 256-byte aligned parts
   const size_t total = 7 * pad(G) + 4 * pad(N) + 4 * pad(n) + pad(17 * n + 16) + 3 * pad(n) + pad(4 * n);
-  if (cudaEventCreateWithFlags(&L.fork, cudaEventDisableTiming) != cudaSuccess)
+  const int per = lanes_per_group(N);
+  if (!L.fork && cudaEventCreateWithFlags(&L.fork, cudaEventDisableTiming) != cudaSuccess)
     return ctx_fail(ctx, HYMOR_ERR_CUDA, "linearisation lane event");
-  L.lane.resize(kJacLanes);
-  for (JacLane& l : L.lane) {
-    if (cudaStreamCreateWithFlags(&l.st, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming) != cudaSuccess ||
-        cudaMalloc(&l.mem, sizeof(double) * total) != cudaSuccess)
-      return ctx_fail(ctx, HYMOR_ERR_CUDA, "linearisation lane allocation failed");
-    cudaMemset(l.mem, 0, sizeof(double) * total);
-    double* b = l.mem;
+  for (int g = 0; g < kLaneGroups; ++g)
+    if ((!L.st[g] && cudaStreamCreateWithFlags(&L.st[g], cudaStreamNonBlocking) != cudaSuccess) ||
+        (!L.done[g] && cudaEventCreateWithFlags(&L.done[g], cudaEventDisableTiming) != cudaSuccess))
+      return ctx_fail(ctx, HYMOR_ERR_CUDA, "linearisation lane stream");
+  double* mem = nullptr;
+  const size_t bytes = sizeof(double) * total * per * kLaneGroups;
+  if (cudaMalloc(&mem, bytes) != cudaSuccess) return ctx_fail(ctx, HYMOR_ERR_CUDA, "linearisation lane allocation failed");
+  if (cudaMemsetAsync(mem, 0, bytes, ctx_stream(ctx)) != cudaSuccess) {
+    cudaFree(mem);
+    return ctx_fail(ctx, HYMOR_ERR_CUDA, "linearisation lane allocation failed");
+  }
+  L.mem = mem;
+  L.stride = (long)total;
+  L.per_group = per;
+  for (int g = 0; g < kLaneGroups; ++g) {
+    JacLane& l = L.first[g];
+    double* b = mem + total * per * g;
     auto take = [&](size_t k) {
       double* r = b;
       b += pad(k);
       return r;
     };
-    l.Y = Cons{take(G), take(G), take(G), take(G)};
+    double* y[4];
+    for (double*& v : y) v = take(G);
+    l.Y = Cons{y[0], y[1], y[2], y[3]};
     l.p = take(G);
     l.T = take(G);
     l.aY = take(G);
     for (int v = 0; v < 4; ++v) l.F[v] = take(N);
-    l.Yp = ShockPts{take(n), take(n), take(n), take(n)};
+    for (double*& v : y) v = take(n);
+    l.Yp = ShockPts{y[0], y[1], y[2], y[3]};
     l.spl = take(17 * n + 16);
     l.speed_x = take(n);
     l.speed_y = take(n);
@@ -1774,11 +1887,11 @@ void linear_state_release(void* p) {
   if (!p) return;
   LinearState* s = static_cast<LinearState*>(p);
   if (s->expm.buf) cudaFree(s->expm.buf);
-  for (JacLane& l : s->lanes.lane) {
-    if (l.st) cudaStreamDestroy(l.st);
-    if (l.done) cudaEventDestroy(l.done);
-    if (l.mem) cudaFree(l.mem);
+  for (int g = 0; g < kLaneGroups; ++g) {
+    if (s->lanes.st[g]) cudaStreamDestroy(s->lanes.st[g]);
+    if (s->lanes.done[g]) cudaEventDestroy(s->lanes.done[g]);
   }
+  if (s->lanes.mem) cudaFree(s->lanes.mem);
   if (s->lanes.fork) cudaEventDestroy(s->lanes.fork);
   delete s;  // the Krylov buffers are context allocations, freed with the context
 }
@@ -1805,15 +1918,16 @@ int hymor_linearize(hymor_ctx* ctx) {
   launch_update_thermo(d, 3, 0, 0, st);
   launch_sound_cmax(d, true, st);
   launch_shock_bc_flags(d, true, false, false, true, 1, st);
+  std::vector<int> rows;
   if (shock_blocks) {
-    std::vector<int> rows(d.nchi);
+    rows.resize(d.nchi);
     cudaMemcpyAsync(rows.data(), d.cell_idx, sizeof(int) * d.nchi, cudaMemcpyDeviceToHost, st);
     if ((r = cuda_check(ctx, cudaStreamSynchronize(st)))) return r;
     if ((r = check_shock_rows_for_blocks(ctx, rows.data(), d.nchi, d.neta))) return r;
   }
   JacLanes* L = nullptr;
   if ((r = ensure_lanes(ctx, &L))) return r;
-  launch_jacobian_assemble(d, st, *L);
+  launch_jacobian_assemble(d, st, *L, rows.data());
   if ((r = cuda_check(ctx, cudaGetLastError()))) return r;
   if ((r = cuda_check(ctx, cudaStreamSynchronize(st)))) return r;
   d.sj.on = shock_blocks;
