@@ -916,6 +916,7 @@ __host__ __device__ inline long shock_mv_smem(int nchi, int transpose) {
 // pipe, not the loads, bounds these rows; partial sums would add FP64 instructions)
 __device__ __forceinline__ double lane_dot(const double* __restrict__ a, const double* b, int n, int lane) {
   double t = 0;
+#pragma unroll 8
   for (int p = lane; p < n; p += 32) t = fma(a[p], b[p], t);
   return t;
 }
@@ -1116,6 +1117,232 @@ int grid_for(long n, int threads) {
   return (int)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
+// ---------------------------------------------------------------------------
+// The Taylor propagation of the extended operators (the shock-position unknowns, the
+// receptivity operator, or both) in one cooperative launch, FP64: per term one pass over all
+// outputs and one grid barrier, instead of three or four launches (stencil, shock rows,
+// receptivity rows, accumulation) that each wait for the last.
+//
+// So that a term needs a single pass, every output is formed whole by one owner: a thread per
+// (cell, component, vector) for the stencil outputs, as matvec_one, and a warp for each output
+// with a long row: the cells (i, sc_i - 1) that A12 and B write (their 36 stencil products and
+// the row's products shared over the lanes), the shock speeds, and the adjoint's tails. The
+// warps take the long rows first. What bounds it: the FP64 pipe (144 FMA per cell and vector,
+// 4.6 us at 160 x 97) and the latency of one pass and a barrier per term; 8 warps per SM keep
+// that pipe busy (a dependent FP64 instruction waits about as long as one issues) and leave
+// room for the propagations of other contexts (two blocks per SM: a single context's term 20 %
+// faster, three contexts' 1.8 times slower). A term of one context alone, and of three at once
+// per context: adjoint with the shock unknowns, 160 x 97, 17.0 -> 11.7 us and 10.8 -> 6.3;
+// receptivity 98 x 73 with 24 frequencies 38.6 -> 17.6 and 22.1 -> 8.0.
+struct ExtArgs {
+  const double* coef;
+  ShockJac sj;
+  const double *bq, *bs, *w;  // receptivity: B and the frequencies (w null: no receptivity)
+  const int* brows;
+  Wrap wr;
+  long N, ld, nop;  // ld: vector stride; nop: start of the freestream blocks
+  double dt;
+  int nchi, k, nw, shock, divide;  // k real vectors; divide: EXPONENTIAL!'s term / j recurrence
+};
+
+struct ExtTerm {
+  const double* X;
+  double* Y;
+  double* acc;         // the running sum, or null (the first term is added one term late)
+  const double* prev;  // the previous term, added first, or null
+  double c, c_prev;
+};
+
+__device__ __forceinline__ void ext_out(const ExtArgs& a, const ExtTerm& t, long o, double y) {
+  double val = a.dt * y;
+  if (a.divide) val *= t.c;
+  t.Y[o] = val;
+  if (!t.acc) return;
+  double r = t.acc[o];
+  if (a.divide) {
+    if (t.prev) r += t.prev[o];
+    t.acc[o] = r + val;
+  } else {
+    if (t.prev) r = fma(t.prev[o], t.c_prev, r);
+    t.acc[o] = fma(val, t.c, r);
+  }
+}
+
+// the lane's share of the stencil row of output component c of cell m = (i, j)
+__device__ __forceinline__ double ext_stencil_lane(const ExtArgs& a, const double* x, int c, long m, int i, int j,
+                                                   int lane, double s) {
+  for (int e = lane; e < 36; e += 32) {
+    const int q = e >> 2, v = e & 3;
+    const long n = a.wr.nbr(i, j, q % 3 - 1, q / 3 - 1);
+    if (n >= 0) s = fma(a.coef[(long)(q * 16 + c * 4 + v) * a.N + m], x[v * a.N + n], s);
+  }
+  return s;
+}
+
+// the lane's share of Σ_d Σ_vin b[d * db + vin] Σ_k u_k,vin(n + d): a row of B on the freestream
+// blocks u of x (b at its column's first entry)
+__device__ __forceinline__ double ext_upstream_lane(const ExtArgs& a, const double* x, const double* b, int db, int m,
+                                                    int lane, double s) {
+  const int p4 = 4 * a.nchi;
+#pragma unroll 4
+  for (int e = lane; e < 12 * a.nw; e += 32) {
+    const int kk = e / 12, r = e - 12 * kk, d = r >> 2, vin = r & 3, n = m + d - 1;
+    if (n >= 0 && n < a.nchi) s = fma(b[d * db + vin], x[a.nop + (long)kk * p4 + vin * a.nchi + n], s);
+  }
+  return s;
+}
+
+template <bool T>
+__device__ __forceinline__ void ext_pass(const ExtArgs& a, const ExtTerm& t) {
+  const int lane = threadIdx.x & 31;
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  const int nchi = a.nchi, p4 = 4 * nchi;
+  const long N = a.N;
+  const unsigned N_u = (unsigned)N, nchi_u = (unsigned)nchi;
+  const bool rec = a.w != nullptr;
+  // the warps' items: rows of the shock speeds, rows of A12 (forward), rows of B (forward),
+  // freestream entries (by 32; the adjoint: a warp per entry of a block, lanes over the
+  // frequencies), stencil outputs (by 32)
+  const int r_spd = a.shock ? a.k * nchi : 0;
+  const int r_a12 = !T && a.shock ? a.k * p4 : 0;
+  const int r_b = !T && rec ? a.k * p4 : 0;
+  const int per_free = T ? p4 : (a.nw * p4 + 31) / 32;
+  const int r_free = rec ? a.k * per_free : 0;
+  const int b0 = r_spd, b1 = b0 + r_a12, b2 = b1 + r_b, b3 = b2 + r_free;
+  const unsigned outs = 4u * N_u;
+  const int items = b3 + (int)((outs * (unsigned)a.k + 31) / 32);
+  for (int it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < items; it += warps) {
+    if (it >= b3) {
+      const unsigned g = (unsigned)(it - b3) * 32 + lane;
+      if (g >= outs * (unsigned)a.k) continue;
+      const unsigned vec = g / outs, w = g - vec * outs, comp = w / N_u, m = w - comp * N_u;
+      const int j = (int)(m / nchi_u), i = (int)(m - (unsigned)j * nchi_u);
+      if (!T && ((a.shock && j == a.sj.rows[i] - 2) || (rec && j == a.brows[i] - 2))) continue;
+      const double* x = t.X + vec * a.ld;
+      double y = 0, B[2][4], V[2][4];
+      bool ok[2];
+      auto load = [&](int q, int slot) {
+        const int b = q / 3 - 1, aa = q % 3 - 1;
+        const long n = T ? a.wr.nbr(i, j, -aa, -b) : a.wr.nbr(i, j, aa, b);
+        const long cell = T ? n : (long)m;
+        ok[slot] = n >= 0;
+        if (n >= 0) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const long plane = T ? q * 16 + e * 4 + (int)comp : q * 16 + (int)comp * 4 + e;
+            B[slot][e] = a.coef[plane * N + cell];
+            V[slot][e] = x[e * N + n];
+          }
+        }
+      };
+      load(0, 0);
+#pragma unroll
+      for (int q = 0; q < 9; ++q) {
+        const int c = q & 1;
+        if (q + 1 < 9) load(q + 1, c ^ 1);
+        if (!ok[c]) continue;
+        y = fma(B[c][0], V[c][0], fma(B[c][1], V[c][1], fma(B[c][2], V[c][2], fma(B[c][3], V[c][3], y))));
+      }
+      if (T && a.shock) {  // A21^T r into the two cells below the shocked cell
+        const int d = a.sj.rows[i] - 2 - j;
+        if (d == 0 || d == 1) y = fma(a.sj.a21[i * 8 + d * 4 + comp], x[4 * N + i], y);
+      }
+      ext_out(a, t, vec * a.ld + w, y);
+    } else if (it < b0) {
+      const int vec = it / nchi, i = it - vec * nchi;
+      const double* x = t.X + vec * a.ld;
+      const double* xr = x + 4 * N;
+      double s;
+      if (!T) {  // A22 r + A21 q (+ B's speed rows)
+        s = lane_dot(a.sj.a22 + (long)i * nchi, xr, nchi, lane);
+        if (lane < 8)
+          s = fma(a.sj.a21[i * 8 + lane], x[(lane & 3) * N + i + (long)(a.sj.rows[i] - 2 - (lane >> 2)) * nchi], s);
+        if (rec) s = ext_upstream_lane(a, x, a.bs + i * 12, 4, i, lane, s);
+      } else {  // A12^T q + A22^T r
+        s = lane_dot(a.sj.a22t + (long)i * nchi, xr, nchi, lane);
+        const double* row = a.sj.a12t + (long)i * p4;
+#pragma unroll 2
+        for (int p = lane; p < nchi; p += 32) {
+          const double* xp = x + p + (long)(a.sj.rows[p] - 2) * nchi;
+#pragma unroll
+          for (int v = 0; v < 4; ++v) s = fma(row[v * nchi + p], xp[v * N], s);
+        }
+      }
+      s = warp_sum(s);
+      if (lane == 0) ext_out(a, t, vec * a.ld + 4 * N + i, s);
+    } else if (it < b2) {
+      const bool sh = it < b1;  // a row of A12 (with B's when both write the cell), or of B alone
+      const int r = it - (sh ? b0 : b1), vec = r / p4, e = r - vec * p4, v = e / nchi, i = e - v * nchi;
+      const bool both = a.shock && rec && a.sj.rows[i] == a.brows[i];
+      if (!sh && both) continue;
+      const int j = (sh ? a.sj.rows[i] : a.brows[i]) - 2;
+      const long m = i + (long)j * nchi;
+      const double* x = t.X + vec * a.ld;
+      double s = sh ? lane_dot(a.sj.a12 + (long)e * nchi, x + 4 * N, nchi, lane) : 0.0;
+      if (!sh || both) s = ext_upstream_lane(a, x, a.bq + (i * 12 + v) * 4, 16, i, lane, s);
+      s = warp_sum(ext_stencil_lane(a, x, v, m, i, j, lane, s));
+      if (lane == 0) ext_out(a, t, vec * a.ld + v * N + m, s);
+    } else if (!T) {  // freestream rows -i w u of real vectors (re, im)
+      const int r = it - b2, vec = r / per_free, f = (r - vec * per_free) * 32 + lane;
+      if (f >= a.nw * p4) continue;
+      const long idx = a.nop + f;
+      const double sg = (vec & 1) ? -1.0 : 1.0;
+      ext_out(a, t, vec * a.ld + idx, sg * a.w[f / p4] * t.X[(vec ^ 1) * a.ld + idx]);
+    } else {  // every freestream block gets B^T q + i w u
+      const int r = it - b2, vec = r / p4, e = r - vec * p4, vin = e / nchi, n = e - vin * nchi;
+      const double* x = t.X + vec * a.ld;
+      const double* xo = t.X + (vec ^ 1) * a.ld;
+      // lanes 0 .. 14: the products of three columns and their speeds, then summed
+      double bt = 0;
+      const int d = lane / 5, vo = lane - 5 * d, m = n + d - 1;
+      if (lane < 15 && m >= 0 && m < nchi) {
+        const int slot = (m * 3 + (n - m) + 1) * 4;
+        if (vo < 4) bt = a.bq[(slot + vo) * 4 + vin] * x[vo * N + m + (long)(a.brows[m] - 2) * nchi];
+        else if (a.shock) bt = a.bs[slot + vin] * x[4 * N + m];
+      }
+      bt = warp_sum(bt);
+      const double sg = (vec & 1) ? 1.0 : -1.0;
+      for (int kk = lane; kk < a.nw; kk += 32) {
+        const long idx = a.nop + (long)kk * p4 + e;
+        ext_out(a, t, vec * a.ld + idx, fma(sg * a.w[kk], xo[idx], bt));
+      }
+    }
+  }
+}
+
+// k_expm_coop's schedule (the first term added one term late, degree 1 with a pass of its own)
+// over ext_pass; sum holds the input when the steps begin.
+template <bool T>
+__global__ void __launch_bounds__(kMvThreads, 3) k_expm_ext(ExtArgs a, int nsteps, int order, const double* xin,
+                                                            double* sum, double* t1, double* t2) {
+  cg::grid_group grid = cg::this_grid();
+  const long n = a.ld * (long)a.k;
+  if (xin != sum) {
+    for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) sum[q] = xin[q];
+    grid.sync();
+  }
+  for (int s = 0; s < nsteps; ++s) {
+    ExtTerm t{sum, nullptr, nullptr, nullptr, 0, 0};
+    long fact = 1;
+    for (int j = 1; j <= order; ++j) {
+      fact *= j;
+      t.Y = (j % 2) ? t1 : t2;
+      t.acc = j == 1 ? nullptr : sum;
+      t.c = 1.0 / (double)(a.divide ? j : fact);
+      ext_pass<T>(a, t);
+      grid.sync();
+      t.X = t.Y;
+      t.prev = j == 1 ? t.Y : nullptr;
+      t.c_prev = t.c;
+    }
+    if (order == 1) {
+      for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x)
+        sum[q] = sum[q] + t1[q];
+      grid.sync();
+    }
+  }
+}
+
 }  // namespace
 
 void launch_shock_mv(const DevCtx& d, int k, const double* X, double* Y, int transpose, double scale,
@@ -1306,8 +1533,48 @@ static void launch_expm_body(const DevCtx& d, int k, double dt, int nsteps, int 
   }
 }
 
+
+// The extended operators' propagation in one cooperative launch (k_expm_ext): from as many
+// launches as the stencil operator's, on grids whose thread-per-output pass is the better one
+// (mv_one; above it a term is long enough to hide its launches, and a batch reads the blocks
+// once for four vectors).
+constexpr int kExpmCoopMinLaunches = 16;
+static bool expm_ext_fits(const DevCtx& d, int k, int nsteps, int order) {
+  return (long)nsteps * (order + 1) >= kExpmCoopMinLaunches && mv_one(d.N, k, d.sms);
+}
+static ExtArgs ext_args(const DevCtx& d, int k, double dt) {
+  ExtArgs a;
+  a.coef = d.coef;
+  a.sj = d.sj;
+  a.bq = a.bs = a.w = nullptr;
+  a.brows = nullptr;
+  a.wr = make_wrap(d.cfg);
+  a.N = d.N;
+  a.ld = a.nop = op_size(d);
+  a.dt = dt;
+  a.nchi = d.nchi;
+  a.k = k;
+  a.nw = 0;
+  a.shock = d.sj.on;
+  a.divide = 0;
+  return a;
+}
+// work: 2 x k x ld doubles
+static cudaError_t launch_expm_ext(const DevCtx& d, const ExtArgs& a, int transpose, int nsteps, int order,
+                                   const double* dX, double* dY, double* work, cudaStream_t st) {
+  double *t1 = work, *t2 = work + a.ld * (long)a.k;
+  const int grid = (int)std::min<long>((4 * d.N * a.k / 32 + a.k * d.nchi + 7) / 8, d.sms);
+  void* args[] = {(void*)&a, &nsteps, &order, (void*)&dX, &dY, &t1, &t2};
+  return cudaLaunchCooperativeKernel(transpose ? (const void*)k_expm_ext<true> : (const void*)k_expm_ext<false>,
+                                     std::max(grid, 1), kMvThreads, args, 0, st);
+}
+
 void launch_expm(const DevCtx& d, int k, double dt, int nsteps, int order, const double* X, double* Yout,
                  int transpose, double* work, cudaStream_t st, bool graph_ok) {
+  if (d.sj.on && expm_ext_fits(d, k, nsteps, order)) {
+    launch_expm_ext(d, ext_args(d, k, dt), transpose, nsteps, order, X, Yout, work, st);
+    return;
+  }
   const long n = op_size(d) * (long)k;
   double* v = work;
   double* t1 = work + n;
@@ -1762,7 +2029,7 @@ int ensure_lanes(hymor_ctx* ctx, JacLanes** out) {
   }
   return 0;
 }
-constexpr int kExpmCoopMinLaunches = 16;
+
 // grids from this many cells take the thread-per-component float-float batch
 constexpr long kFfCompCells = 65536;
 
@@ -2091,8 +2358,8 @@ int hymor_expm_apply_dev(hymor_ctx* ctx, int k, double dt, int nsteps, int order
   DevCtx& d = ctx_dev(ctx);
   if (!d.coef) return ctx_fail(ctx, HYMOR_ERR_NOT_READY, "no Jacobian: call hymor_linearize or hymor_jacobian_set");
   cudaStream_t st = ctx_stream(ctx);
-  // the cooperative kernel covers the stencil operator; with the shock blocks each term
-  // is a launch sequence (launch_expm_body)
+  // the stencil operator in one cooperative launch, and with the shock blocks the extended one
+  // (launch_expm); else each term is a launch sequence (launch_expm_body)
   if (!d.sj.on && (long)nsteps * (order + 1) >= kExpmCoopMinLaunches)
     return expm_cooperative(ctx, k, dt, nsteps, order, dX, dY, transpose);
   const size_t n = op_size(d) * (size_t)k;
@@ -2312,6 +2579,24 @@ int hymor_recept_expm_dev(hymor_ctx* ctx, int k, int nw, const double* w, double
   if (r) return r;
   DevCtx& d = ctx_dev(ctx);
   cudaStream_t st = ctx_stream(ctx);
+  // (k_expm_ext counts its items in 32 bits)
+  if (expm_ext_fits(d, 2 * k, nsteps, order) && 8L * k * d.nchi * nw < (1L << 30)) {
+    ExtArgs a = ext_args(d, 2 * k, dt);
+    a.bq = d.bq;
+    a.bs = d.bs;
+    a.w = dw;
+    a.brows = d.brows;
+    a.ld = recept_size(d, nw);
+    a.nw = nw;
+    a.divide = 1;
+    double* work = nullptr;
+    if (!(r = cuda_check(ctx, cudaMallocAsync((void**)&work, sizeof(double) * 2 * a.ld * a.k, st)))) {
+      r = cuda_check(ctx, launch_expm_ext(d, a, adjoint, nsteps, order, dX, dY, work, st));
+      cudaFreeAsync(work, st);
+    }
+    cudaFreeAsync(dw, st);
+    return r;
+  }
   double* work = nullptr;
   const long n = 2L * k * recept_size(d, nw);
   if ((r = cuda_check(ctx, cudaMallocAsync((void**)&work, sizeof(double) * 2 * n, st)))) return r;

@@ -96,8 +96,9 @@ extern "C" int hymor_expm_apply_dev_noalloc(hymor_ctx* ctx, int k, double dt, in
   double* work = nullptr;
   int r = scratch_for_ctx_device(ctx, &work);
   if (r) return r;
-  // launch_expm uses work[0, 3n): v, and the two alternating Taylor terms; every Taylor
-  // step is launched directly (graph_ok false), also with the shock-position blocks
+  // launch_expm uses work[0, 3n): v, and the two alternating Taylor terms. With the shock-
+  // position blocks the steps run in one cooperative launch (the kernel of the allocating
+  // entry point), else every Taylor step is launched directly (graph_ok false)
   launch_expm(d, k, dt, nsteps, order, dX, dY, transpose, work, ctx_stream(ctx), false);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return ctx_fail(ctx, HYMOR_ERR_CUDA, cudaGetErrorString(e));
