@@ -715,6 +715,7 @@ int hymor_ctx_create(const hymor_config* cfg, const hymor_mesh* mesh, hymor_ctx*
   if (cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess || d.sms < 1)
     return bail(fail(ctx, HYMOR_ERR_CUDA, "multiprocessor count"));
   d.coef = nullptr;
+  d.coef_nz = nullptr;
   d.jwork = nullptr;
   d.sj = ShockJac{};
   d.up_cols = nullptr;

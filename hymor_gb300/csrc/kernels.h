@@ -51,6 +51,9 @@ struct DevCtx {
                      // screened CFL reduction's FP32 maxima and block counters
   // Jacobian
   double* coef;    // N * 144 stencil blocks (or null)
+  // which cells have entries (or null): the matvecs' masks (N), then per input variable whether
+  // the cell's own blocks have a non-zero entry (4 x N)
+  unsigned char* coef_nz;
   float2* coef_ff; // float-float copy of coef for the propagator (or null)
   int coef_version, coef_ff_version;  // writes of coef, and the write coef_ff was split from
   // the cooperative Taylor propagator in float-float (1, the default) or FP64 (0)

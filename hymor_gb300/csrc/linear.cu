@@ -138,6 +138,7 @@ struct ScatArgs {
   const double* Fp[4];
   const double* Fb[4];
   double* coef;
+  unsigned char* nz;    // 4 x N, byte var N + m: cell m has a non-zero entry of that variable
   Wrap w;
   double eps, inv_eps;  // inv_eps: the rounded reciprocal of eps, 0 to divide
   long N;
@@ -180,6 +181,7 @@ __global__ void __launch_bounds__(256) k_scatter(ScatArgs a) {
   for (long m = blockIdx.x * (long)blockDim.x + threadIdx.x; m < N; m += (long)gridDim.x * blockDim.x) {
     const int j = (int)((unsigned)m / nchi_u), i = (int)((unsigned)m - (unsigned)j * nchi_u);
     double fb[4];
+    unsigned long long any = 0;
 #pragma unroll
     for (int vo = 0; vo < 4; ++vo) fb[vo] = a.Fb[vo][m];
 #pragma unroll
@@ -192,9 +194,13 @@ __global__ void __launch_bounds__(256) k_scatter(ScatArgs a) {
         const long o = off + (long)(3 * (nj % 3u) + ni % 3u) * a.lane + m;  // the input cell's colour
         const int q = (b + 1) * 3 + (aa + 1);
 #pragma unroll
-        for (int vo = 0; vo < 4; ++vo)
-          a.coef[((long)(q * 4 + vo) * 4 + var) * N + m] = div_eps(a.Fp[vo][o] - fb[vo], a.eps, a.inv_eps);
+        for (int vo = 0; vo < 4; ++vo) {
+          const double d = div_eps(a.Fp[vo][o] - fb[vo], a.eps, a.inv_eps);
+          any |= (unsigned long long)__double_as_longlong(d) << 1;
+          a.coef[((long)(q * 4 + vo) * 4 + var) * N + m] = d;
+        }
       }
+    a.nz[var * N + m] = any != 0;
   }
 }
 
@@ -202,6 +208,7 @@ __global__ void __launch_bounds__(256) k_scatter(ScatArgs a) {
 // acc_j += c_acc * y_j. Vectors: 4N each, column-major batch.
 struct MvArgs {
   const double* coef;
+  const unsigned char* nz;
   const double* X;
   double* Y;
   double* acc;
@@ -219,6 +226,25 @@ struct MvArgs {
   long ld;  // vector stride (4N, or 4N + Nchi with the shock unknowns)
   int k, transpose;
 };
+
+// Cells without entries: at and above the shocked rows the residual is masked, so a quarter to
+// four fifths of the cells of a shock-fitted flow have all-zero blocks, which need not be read
+// nor multiplied. nz[m] (written with the blocks): kMaskRow when cell m's own blocks have a
+// non-zero entry (its outputs), kMaskCol when a block that takes cell m as its input does (the
+// transpose's outputs). A skipped output is zero, except that a zero times an infinity or NaN
+// is NaN: it takes a NaN where an input of its neighbours is not finite. Only the matvecs whose
+// time is the blocks' read or their FP64 products test the mask, with a quarter of the cells
+// empty: the FP64 batch (800 x 400, 64 vectors: 4.88 -> 3.64 ms; one vector 82.9 -> 66.2 us),
+// and one float-float vector on a large grid (1200 x 400, 200 matvecs: 19.6 -> 16.5 ms). The
+// thread-per-output ones and the float-float batches wait for the latency of their loads, which
+// the test lengthens (100 x 80: one vector 840 -> 927 us, 64 vectors 7.6 -> 9.1 ms).
+constexpr unsigned kMaskRow = 1, kMaskCol = 2;
+__device__ __forceinline__ unsigned poison(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7ff00000u) == 0x7ff00000u;
+}
+__device__ __forceinline__ double poisoned(double y, unsigned bad) {
+  return bad ? __longlong_as_double(0x7ff8000000000000LL) : y;
+}
 
 // ST: the blocks exceed L2 and are read with streaming (evict-first) loads, which keep the
 // vectors that every neighbour re-reads in L2; blocks that fit stay cached from one matvec
@@ -328,6 +354,18 @@ __device__ __forceinline__ void matvec_multi(const MvArgs& a) {
       for (int v = 0; v < kVecChunk; ++v)
 #pragma unroll
         for (int c = 0; c < 4; ++c) y[v][c] = 0;
+      unsigned bad = 0;  // bit v: a non-finite input of vector v met a zero block
+      if (!(a.nz[m] & (a.transpose ? kMaskCol : kMaskRow))) {
+        for (int b = -1; b <= 1; ++b)
+          for (int aa = -1; aa <= 1; ++aa) {
+            const long n = a.transpose ? a.w.nbr(i, j, -aa, -b) : a.w.nbr(i, j, aa, b);
+            if (n < 0) continue;
+            for (int v = 0; v < nv; ++v) {
+              const double* x = a.X + (long)(v0 + v) * n4 + n;
+              bad |= (poison(x[0]) | poison(x[N]) | poison(x[2 * N]) | poison(x[3 * N])) << v;
+            }
+          }
+      } else
 #pragma unroll
       for (int b = -1; b <= 1; ++b)
 #pragma unroll
@@ -368,7 +406,7 @@ __device__ __forceinline__ void matvec_multi(const MvArgs& a) {
         const double sc = a.vscale ? a.vscale[v0 + v] : a.scale;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          const double val = sc * y[v][c];
+          const double val = sc * poisoned(y[v][c], bad & (1u << v));
           yo[c * N + m] = val;
           if (a.acc) {
             double* ac = a.acc + (long)(v0 + v) * n4;
@@ -453,6 +491,7 @@ __global__ void __launch_bounds__(kMvThreads, 2) k_expm_coop(MvArgs base, int ns
 // relative level than this rounding; the Jacobian is a finite-difference one (~1e-8).
 struct MvFf {
   const float2* coef;
+  const unsigned char* nz;
   const float2* X;
   float2* Y;
   float2* acc;             // the running sum, or null
@@ -477,6 +516,22 @@ template <bool ST>
 __device__ __forceinline__ ff ldff_coef(const float2* p, long i) {
   const float2 v = ST ? __ldcs(p + i) : p[i];
   return ff{v.x, v.y};
+}
+
+// the sum of the inputs of cell (i, j)'s neighbours times zero: 0, or NaN where one is not
+// finite (a cell without entries)
+__device__ __forceinline__ float ff_poison_window(const MvFf& a, const float2* x, int i, int j) {
+  float s = 0.0f;
+  for (int q = 0; q < 9; ++q) {
+    const long n = a.transpose ? a.w.nbr(i, j, 1 - q % 3, 1 - q / 3) : a.w.nbr(i, j, q % 3 - 1, q / 3 - 1);
+    if (n < 0) continue;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 v = x[e * a.N + n];
+      s = __fmaf_rn(v.x, 0.0f, __fmaf_rn(v.y, 0.0f, s));
+    }
+  }
+  return s;
 }
 
 // one output of a term: val = scale y into Y, and the running sum
@@ -551,6 +606,16 @@ __device__ __forceinline__ void matvec_multi_ff(const MvFf& a) {
     for (int v = 0; v < KV; ++v)
 #pragma unroll
       for (int c = 0; c < 4; ++c) y[v][c] = ff{0.0f, 0.0f};
+    if (KV == 1 && !(a.nz[m] & (a.transpose ? kMaskCol : kMaskRow))) {
+#pragma unroll
+      for (int v = 0; v < KV; ++v)
+        if (v < nv) {
+          const float z = ff_poison_window(a, a.X + (long)(v0 + v) * n4, i, j);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) mvff_out(a, v0 + v, (long)(v0 + v) * n4 + c * N + m, ff{z, 0.0f});
+        }
+      continue;
+    }
     // one neighbour block at a time for a single vector (its 16 pairs in registers), all
     // nine unrolled for a chunk
 #pragma unroll(KV == 1 ? 1 : 3)
@@ -696,11 +761,27 @@ __global__ void k_copy(const double* __restrict__ s, double* __restrict__ d, lon
 }
 
 // per-cell block layout <-> plane layout
-__global__ void k_blocks_to_planes(const double* blk, double* pl, long N) {
+// (nz, zeroed: byte (input variable) N + m set where cell m has a non-zero entry of it)
+__global__ void k_blocks_to_planes(const double* blk, double* pl, unsigned char* nz, long N) {
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < N * 144; t += (long)gridDim.x * blockDim.x) {
     const long m = t / 144;
     const int e = (int)(t % 144);
-    pl[(long)e * N + m] = blk[t];
+    const double c = blk[t];
+    pl[(long)e * N + m] = c;
+    if (((unsigned long long)__double_as_longlong(c) << 1) != 0) nz[(e & 3) * N + m] = 1;
+  }
+}
+// the masks of the matvecs (kMaskRow, kMaskCol) from the 4 x N bytes of the input variables
+__global__ void k_masks(unsigned char* mask, const unsigned char* nz, Wrap w, long N) {
+  for (long m = blockIdx.x * (long)blockDim.x + threadIdx.x; m < N; m += (long)gridDim.x * blockDim.x) {
+    const int j = (int)((unsigned)m / (unsigned)w.nchi), i = (int)((unsigned)m - (unsigned)j * (unsigned)w.nchi);
+    auto any = [&](long c) { return nz[c] | nz[N + c] | nz[2 * N + c] | nz[3 * N + c]; };
+    unsigned r = any(m) ? kMaskRow : 0;
+    for (int q = 0; q < 9; ++q) {
+      const long n = w.nbr(i, j, 1 - q % 3, 1 - q / 3);
+      if (n >= 0 && any(n)) r |= kMaskCol;
+    }
+    mask[m] = (unsigned char)r;
   }
 }
 __global__ void k_planes_to_blocks(const double* pl, double* blk, long N) {
@@ -1124,9 +1205,10 @@ int grid_for(long n, int threads) {
 // receptivity rows, accumulation) that each wait for the last.
 //
 // So that a term needs a single pass, every output is formed whole by one owner: a thread per
-// (cell, component, vector) for the stencil outputs, as matvec_one, and a warp for each output
-// with a long row: the cells (i, sc_i - 1) that A12 and B write (their 36 stencil products and
-// the row's products shared over the lanes), the shock speeds, and the adjoint's tails. The
+// (cell, component, vector) for the stencil outputs, as matvec_one, and a warp for the outputs
+// with long rows, their stencil products and the rows' products shared over the lanes: a
+// column's cell (i, sc_i - 1) that A12 writes with its shock speed, each component of that cell
+// where B writes it, and the adjoint's tails. The
 // warps take the long rows first. What bounds it: the FP64 pipe (144 FMA per cell and vector,
 // 4.6 us at 160 x 97) and the latency of one pass and a barrier per term; 8 warps per SM keep
 // that pipe busy (a dependent FP64 instruction waits about as long as one issues) and leave
@@ -1168,7 +1250,33 @@ __device__ __forceinline__ void ext_out(const ExtArgs& a, const ExtTerm& t, long
   }
 }
 
-// the lane's share of the stencil row of output component c of cell m = (i, j)
+// The warp's sums of four values: lanes 0, 8, 16, 24 end with those of s[0], s[1], s[2], s[3]
+// (two values folded per lane and step while there are several: 6 additions for the four, FP64
+// ones, instead of 20).
+__device__ __forceinline__ double warp_sum4(const double (&s)[4], int lane) {
+  const bool hi = lane & 16, hi2 = lane & 8;
+  const double a = (hi ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[2], 16);
+  const double b = (hi ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, hi ? s[1] : s[3], 16);
+  double r = (hi2 ? b : a) + __shfl_xor_sync(0xffffffffu, hi2 ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+  return r;
+}
+
+// the lane's share of the four stencil rows of cell m = (i, j)
+__device__ __forceinline__ void ext_stencil_lane4(const ExtArgs& a, const double* x, long m, int i, int j, int lane,
+                                                  double (&s)[4]) {
+#pragma unroll 1
+  for (int e = lane; e < 36; e += 32) {
+    const int q = e >> 2, v = e & 3;
+    const long n = a.wr.nbr(i, j, q % 3 - 1, q / 3 - 1);
+    if (n < 0) continue;
+    const double xv = x[v * a.N + n];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) s[c] = fma(a.coef[(long)(q * 16 + c * 4 + v) * a.N + m], xv, s[c]);
+  }
+}
+// the lane's share of the stencil row of component c
 __device__ __forceinline__ double ext_stencil_lane(const ExtArgs& a, const double* x, int c, long m, int i, int j,
                                                    int lane, double s) {
   for (int e = lane; e < 36; e += 32) {
@@ -1179,8 +1287,8 @@ __device__ __forceinline__ double ext_stencil_lane(const ExtArgs& a, const doubl
   return s;
 }
 
-// the lane's share of Σ_d Σ_vin b[d * db + vin] Σ_k u_k,vin(n + d): a row of B on the freestream
-// blocks u of x (b at its column's first entry)
+// the lane's share of Σ_d Σ_vin b[d * db + vin] Σ_k u_k,vin(m + d - 1): a row of B (b: its first
+// entry) on the freestream blocks u of x
 __device__ __forceinline__ double ext_upstream_lane(const ExtArgs& a, const double* x, const double* b, int db, int m,
                                                     int lane, double s) {
   const int p4 = 4 * a.nchi;
@@ -1200,15 +1308,17 @@ __device__ __forceinline__ void ext_pass(const ExtArgs& a, const ExtTerm& t) {
   const long N = a.N;
   const unsigned N_u = (unsigned)N, nchi_u = (unsigned)nchi;
   const bool rec = a.w != nullptr;
-  // the warps' items: rows of the shock speeds, rows of A12 (forward), rows of B (forward),
+  // the warps' items: columns of the shock unknowns (the speeds, forward without B also the
+  // cells (i, sc_i - 1); the adjoint's tail rows), with B the rows of those cells (A12's, then
+  // B's: a row each, because B's 12 products per frequency make them the longest items),
   // freestream entries (by 32; the adjoint: a warp per entry of a block, lanes over the
   // frequencies), stencil outputs (by 32)
-  const int r_spd = a.shock ? a.k * nchi : 0;
-  const int r_a12 = !T && a.shock ? a.k * p4 : 0;
+  const int r_sh = a.shock ? a.k * nchi : 0;
+  const int r_a12 = !T && rec && a.shock ? a.k * p4 : 0;
   const int r_b = !T && rec ? a.k * p4 : 0;
   const int per_free = T ? p4 : (a.nw * p4 + 31) / 32;
   const int r_free = rec ? a.k * per_free : 0;
-  const int b0 = r_spd, b1 = b0 + r_a12, b2 = b1 + r_b, b3 = b2 + r_free;
+  const int b0 = r_sh, b1 = b0 + r_a12, b2 = b1 + r_b, b3 = b2 + r_free;
   const unsigned outs = 4u * N_u;
   const int items = b3 + (int)((outs * (unsigned)a.k + 31) / 32);
   for (int it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < items; it += warps) {
@@ -1248,32 +1358,51 @@ __device__ __forceinline__ void ext_pass(const ExtArgs& a, const ExtTerm& t) {
         if (d == 0 || d == 1) y = fma(a.sj.a21[i * 8 + d * 4 + comp], x[4 * N + i], y);
       }
       ext_out(a, t, vec * a.ld + w, y);
-    } else if (it < b0) {
+    } else if (T && it < b0) {  // A12^T q + A22^T r
       const int vec = it / nchi, i = it - vec * nchi;
       const double* x = t.X + vec * a.ld;
-      const double* xr = x + 4 * N;
-      double s;
-      if (!T) {  // A22 r + A21 q (+ B's speed rows)
-        s = lane_dot(a.sj.a22 + (long)i * nchi, xr, nchi, lane);
-        if (lane < 8)
-          s = fma(a.sj.a21[i * 8 + lane], x[(lane & 3) * N + i + (long)(a.sj.rows[i] - 2 - (lane >> 2)) * nchi], s);
-        if (rec) s = ext_upstream_lane(a, x, a.bs + i * 12, 4, i, lane, s);
-      } else {  // A12^T q + A22^T r
-        s = lane_dot(a.sj.a22t + (long)i * nchi, xr, nchi, lane);
-        const double* row = a.sj.a12t + (long)i * p4;
+      double s = lane_dot(a.sj.a22t + (long)i * nchi, x + 4 * N, nchi, lane);
+      const double* row = a.sj.a12t + (long)i * p4;
 #pragma unroll 2
-        for (int p = lane; p < nchi; p += 32) {
-          const double* xp = x + p + (long)(a.sj.rows[p] - 2) * nchi;
+      for (int p = lane; p < nchi; p += 32) {
+        const double* xp = x + p + (long)(a.sj.rows[p] - 2) * nchi;
 #pragma unroll
-          for (int v = 0; v < 4; ++v) s = fma(row[v * nchi + p], xp[v * N], s);
-        }
+        for (int v = 0; v < 4; ++v) s = fma(row[v * nchi + p], xp[v * N], s);
       }
       s = warp_sum(s);
       if (lane == 0) ext_out(a, t, vec * a.ld + 4 * N + i, s);
+    } else if (it < b0) {
+      // column i: the speed A21 q + A22 r (+ B's), and without B the cell (i, sc_i - 1), whose
+      // stencil rows A12 r joins
+      const int vec = it / nchi, i = it - vec * nchi, j = a.sj.rows[i] - 2;
+      const long m = i + (long)j * nchi;
+      const double* x = t.X + vec * a.ld;
+      const double* xr = x + 4 * N;
+      double spd = 0;
+      if (lane < 8) spd = a.sj.a21[i * 8 + lane] * x[(lane & 3) * N + m - (long)(lane >> 2) * nchi];
+      if (rec) {
+        spd += lane_dot(a.sj.a22 + (long)i * nchi, xr, nchi, lane);
+        spd = ext_upstream_lane(a, x, a.bs + i * 12, 4, i, lane, spd);
+      } else {
+        double s[4] = {0, 0, 0, 0};
+#pragma unroll 1
+        for (int p = lane; p < nchi; p += 32) {
+          const double rp = xr[p];
+          spd = fma(a.sj.a22[(long)i * nchi + p], rp, spd);
+#pragma unroll
+          for (int v = 0; v < 4; ++v) s[v] = fma(a.sj.a12[((long)v * nchi + i) * nchi + p], rp, s[v]);
+        }
+        ext_stencil_lane4(a, x, m, i, j, lane, s);
+        const double y = warp_sum4(s, lane);
+        if ((lane & 7) == 0) ext_out(a, t, vec * a.ld + (lane >> 3) * N + m, y);
+      }
+      spd = warp_sum(spd);
+      if (lane == 0) ext_out(a, t, vec * a.ld + 4 * N + i, spd);
     } else if (it < b2) {
-      const bool sh = it < b1;  // a row of A12 (with B's when both write the cell), or of B alone
+      // a row of A12 (with B's when both write the cell), or of B alone
+      const bool sh = it < b1;
       const int r = it - (sh ? b0 : b1), vec = r / p4, e = r - vec * p4, v = e / nchi, i = e - v * nchi;
-      const bool both = a.shock && rec && a.sj.rows[i] == a.brows[i];
+      const bool both = a.shock && a.sj.rows[i] == a.brows[i];
       if (!sh && both) continue;
       const int j = (sh ? a.sj.rows[i] : a.brows[i]) - 2;
       const long m = i + (long)j * nchi;
@@ -1386,6 +1515,7 @@ void launch_matvec(const DevCtx& d, int k, const double* X, double* Y, int trans
   a.c_prev = 0;
   a.vscale = nullptr;
   a.coef = d.coef;
+  a.nz = d.coef_nz;
   a.X = X;
   a.Y = Y;
   a.acc = nullptr;
@@ -1503,6 +1633,7 @@ static void launch_expm_body(const DevCtx& d, int k, double dt, int nsteps, int 
   a.c_prev = 0;
   a.vscale = nullptr;
   a.coef = d.coef;
+  a.nz = d.coef_nz;
   a.w = make_wrap(d.cfg);
   a.N = d.N;
   a.ld = n / k;
@@ -1773,6 +1904,7 @@ void launch_jacobian_assemble(DevCtx& d, cudaStream_t st, JacLanes& L, const int
   ScatArgs sa;
   for (int v = 0; v < 4; ++v) sa.Fb[v] = Fb[v];
   sa.coef = d.coef;
+  sa.nz = d.coef_nz + N;
   sa.w = make_wrap(c);
   sa.eps = c.perturbation_magnitude;
   sa.inv_eps = div_eps_reciprocal(sa.eps);
@@ -1798,6 +1930,7 @@ void launch_jacobian_assemble(DevCtx& d, cudaStream_t st, JacLanes& L, const int
     k_scatter<<<dim3(grid_for(N, 256), 1, n / 9), 256, 0, ls>>>(sl);
   });
   lanes_join(L, st);
+  k_masks<<<grid_for(N, 256), 256, 0, st>>>(d.coef_nz, d.coef_nz + N, make_wrap(c), N);
   if (shock_blocks) launch_shock_assemble(d, Fb, L, hrows, st);
 }
 
@@ -1932,11 +2065,16 @@ int ensure_linear(hymor_ctx* ctx) {
     if (cudaMalloc(&p, sizeof(double) * 144 * d.N) != cudaSuccess)
       return ctx_fail(ctx, HYMOR_ERR_CUDA, "Jacobian allocation failed");
     ctx_allocs(ctx).push_back(p);
-    d.coef = static_cast<double*>(p);
+    double* coef = static_cast<double*>(p);
+    if (cudaMalloc(&p, 5 * d.N) != cudaSuccess)
+      return ctx_fail(ctx, HYMOR_ERR_CUDA, "Jacobian row mask allocation failed");
+    ctx_allocs(ctx).push_back(p);
+    d.coef_nz = static_cast<unsigned char*>(p);
     if (cudaMalloc(&p, sizeof(double) * 8 * d.N) != cudaSuccess)
       return ctx_fail(ctx, HYMOR_ERR_CUDA, "Jacobian workspace allocation failed");
     ctx_allocs(ctx).push_back(p);
     d.jwork = static_cast<double*>(p);
+    d.coef = coef;
   }
   return 0;
 }
@@ -2098,6 +2236,7 @@ int expm_cooperative(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
   base.c_prev = 0;
   base.vscale = nullptr;
   base.coef = d.coef;
+  base.nz = d.coef_nz;
   base.w = make_wrap(d.cfg);
   base.N = d.N;
   base.ld = 4 * d.N;
@@ -2120,6 +2259,7 @@ int expm_cooperative(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
   if (ffp) {
     MvFf bf;
     bf.coef = d.coef_ff;
+    bf.nz = base.nz;
     bf.X = nullptr;
     bf.Y = nullptr;
     bf.acc = nullptr;
@@ -2287,7 +2427,9 @@ int hymor_jacobian_set(hymor_ctx* ctx, const double* coef) {
   double* tmp = nullptr;
   if ((r = cuda_check(ctx, cudaMallocAsync((void**)&tmp, sizeof(double) * 144 * d.N, st)))) return r;
   r = cuda_check(ctx, cudaMemcpyAsync(tmp, coef, sizeof(double) * 144 * d.N, cudaMemcpyHostToDevice, st));
-  k_blocks_to_planes<<<grid_for(d.N * 144, 256), 256, 0, st>>>(tmp, d.coef, d.N);
+  cudaMemsetAsync(d.coef_nz + d.N, 0, 4 * d.N, st);
+  k_blocks_to_planes<<<grid_for(d.N * 144, 256), 256, 0, st>>>(tmp, d.coef, d.coef_nz + d.N, d.N);
+  k_masks<<<grid_for(d.N, 256), 256, 0, st>>>(d.coef_nz, d.coef_nz + d.N, make_wrap(d.cfg), d.N);
   ++d.coef_version;
   cudaFreeAsync(tmp, st);
   if (r) return r;
