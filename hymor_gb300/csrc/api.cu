@@ -417,12 +417,6 @@ int check_err_words(hymor_ctx* ctx, const unsigned* h) {
   return 0;
 }
 
-int read_err(hymor_ctx* ctx) {
-  unsigned h[kErrCount];
-  CU(cudaMemcpyAsync(h, ctx->d.err, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
-  CU(cudaStreamSynchronize(ctx->stream));
-  return check_err_words(ctx, h);
-}
 
 int set_device(hymor_ctx* ctx) {
   CU(cudaSetDevice(ctx->device));
@@ -435,7 +429,19 @@ int set_device(hymor_ctx* ctx) {
 constexpr size_t kScalPitch = 32;
 size_t state_pitch(size_t n) { return (n + 31) & ~size_t(31); }
 size_t header_doubles(size_t n) { return 4 * state_pitch(n) + kScalPitch + (n + 1) / 2; }
-size_t stage_bytes(int n) { return header_doubles(n) * sizeof(double) + kErrCount * sizeof(unsigned); }
+size_t stage_bytes(int n) {  // a multiple of 256: hymor_residual's staged flux follows
+  return (header_doubles(n) * sizeof(double) + kErrCount * sizeof(unsigned) + 255) & ~size_t(255);
+}
+// a residual's flux up to this size goes through the staging buffer when the caller's memory is
+// pageable (2 MB: a host copy of ~0.1 ms)
+constexpr size_t kFluxStage = 2u << 20;
+
+int read_err(hymor_ctx* ctx) {  // through the staging buffer, as the state's download
+  unsigned* h = reinterpret_cast<unsigned*>(ctx->stage + header_doubles(ctx->d.nchi) * sizeof(double));
+  CU(cudaMemcpyAsync(h, ctx->d.err, kErrCount * sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+  CU(cudaStreamSynchronize(ctx->stream));
+  return check_err_words(ctx, h);
+}
 
 void drop_step_graph(hymor_ctx* ctx);
 
@@ -525,7 +531,7 @@ int enqueue_download(hymor_ctx* ctx, double* q, bool with_err) {
   cudaStream_t st = ctx->stream;
   if (q) CU(cudaMemcpy2DAsync(q, G * 8, d.S.rho, Gp * 8, G * 8, 4, cudaMemcpyDeviceToHost, st));
   // the error words follow the header on the device as in the staging buffer: one copy
-  CU(cudaMemcpyAsync(ctx->stage, d.Sp.x, with_err ? stage_bytes(n) : header_doubles(n) * 8,
+  CU(cudaMemcpyAsync(ctx->stage, d.Sp.x, header_doubles(n) * 8 + (with_err ? kErrCount * sizeof(unsigned) : 0),
                      cudaMemcpyDeviceToHost, st));
   return 0;
 }
@@ -693,7 +699,12 @@ int hymor_ctx_create(const hymor_config* cfg, const hymor_mesh* mesh, hymor_ctx*
       (r = dalloc(ctx, &d.aY, d.G)))
     return bail(r);
   for (int v = 0; v < 4; ++v)
-    if ((r = dalloc(ctx, &d.F[v], d.N)) || (r = dalloc(ctx, &d.SF[v], d.N))) return bail(r);
+    if ((r = dalloc(ctx, &d.F[v], d.N))) return bail(r);
+  {  // the stored flux in one block, as the host has it, so that it moves in one copy
+    double* b = nullptr;
+    if ((r = dalloc(ctx, &b, 4 * (size_t)d.N))) return bail(r);
+    for (int v = 0; v < 4; ++v) d.SF[v] = b + v * d.N;
+  }
   {  // shock points of S, the scalars, the cell indices and the error words in one block,
      // laid out like the pinned staging buffer, so that they move in one copy
     const size_t np = state_pitch(d.nchi);
@@ -761,7 +772,8 @@ int hymor_ctx_create(const hymor_config* cfg, const hymor_mesh* mesh, hymor_ctx*
         cudaEventCreateWithFlags(&ctx->cfl_fork, cudaEventDisableTiming) != cudaSuccess)
       return bail(fail(ctx, HYMOR_ERR_CUDA, "event"));
   }
-  if (cudaMallocHost(&ctx->stage, stage_bytes(d.nchi)) != cudaSuccess)
+  const size_t flux_bytes = 4 * (size_t)d.N * sizeof(double);
+  if (cudaMallocHost(&ctx->stage, stage_bytes(d.nchi) + (flux_bytes <= kFluxStage ? flux_bytes : 0)) != cudaSuccess)
     return bail(fail(ctx, HYMOR_ERR_CUDA, "pinned staging allocation failed"));
   cudaEventCreate(&ctx->t0);
   cudaEventCreate(&ctx->t1);
@@ -854,8 +866,7 @@ int hymor_residual(hymor_ctx* ctx, double* flux) {
   TRY(set_device(ctx));
   DevCtx& d = ctx->d;
   cudaStream_t st = ctx->stream;
-  launch_update_thermo(d, 3, 0, 0, st);
-  launch_sound_cmax(d, true, st);
+  launch_thermo_sound(d, st);
   ctx->a_stale = false;
   d.up_cols = d.res_up;  // rho_0_upstream_p of the reference's Dict, when set
   launch_shock_bc(d, true, false, false, 0, 0, 1, st);
@@ -864,10 +875,21 @@ int hymor_residual(hymor_ctx* ctx, double* flux) {
   launch_flux(d, true, SF, st);
   stored_flux_written(ctx);
   CU(cudaGetLastError());
-  if (flux)
-    for (int v = 0; v < 4; ++v)
-      CU(cudaMemcpyAsync(flux + v * d.N, d.SF[v], d.N * 8, cudaMemcpyDeviceToHost, st));
-  return read_err(ctx);
+  if (!flux) return read_err(ctx);
+  // The four planes in one copy, straight into page-locked memory, or through the pinned staging
+  // buffer and one host copy (a copy into pageable memory waits for the stream and goes through
+  // the driver's own staging each time: 180 x 60, four planes, 27 us more than page-locked ones);
+  // a large flux goes straight to pageable memory, where the driver's staging overlaps.
+  const size_t bytes = 4 * (size_t)d.N * sizeof(double);
+  cudaPointerAttributes at;
+  const bool pinned = cudaPointerGetAttributes(&at, flux) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
+  if (!pinned) cudaGetLastError();
+  const bool staged = !pinned && bytes <= kFluxStage;
+  double* to = staged ? reinterpret_cast<double*>(ctx->stage + stage_bytes(d.nchi)) : flux;
+  CU(cudaMemcpyAsync(to, d.SF[0], bytes, cudaMemcpyDeviceToHost, st));
+  const int r = read_err(ctx);
+  if (staged) std::memcpy(flux, to, bytes);
+  return r;
 }
 
 int hymor_set_upstream(hymor_ctx* ctx, const double* cols) {
@@ -891,8 +913,7 @@ int hymor_set_upstream(hymor_ctx* ctx, const double* cols) {
 int hymor_set_flux(hymor_ctx* ctx, const double* flux) {
   if (!ctx || !flux) return HYMOR_ERR_INVALID;
   TRY(set_device(ctx));
-  for (int v = 0; v < 4; ++v)
-    CU(cudaMemcpyAsync(ctx->d.SF[v], flux + v * ctx->d.N, ctx->d.N * 8, cudaMemcpyHostToDevice, ctx->stream));
+  CU(cudaMemcpyAsync(ctx->d.SF[0], flux, 4 * ctx->d.N * 8, cudaMemcpyHostToDevice, ctx->stream));
   stored_flux_written(ctx);
   CU(cudaStreamSynchronize(ctx->stream));
   return 0;

@@ -434,11 +434,12 @@ __device__ __forceinline__ Cons lane_cons(const Cons& q, long off) {
 // Per-row bands of A = R + lam Q^T Q, right-hand sides Q^T y and interval reciprocals,
 // one thread per row (the rows are independent), after copying the shock points of S
 // into the stage array at stage 1.
+template <bool LANES>
 __global__ void __launch_bounds__(128) k_spline_rows(SplineArgs A) {
   const int n = A.n;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const long off = blockIdx.z * A.lane;
+  const long off = LANES ? blockIdx.z * A.lane : 0;
   const ShockPts pts = lane_pts(A.pts, off);
   double* xs = A.ws + off;
   double* yx = xs + n;
@@ -698,13 +699,14 @@ constexpr int kSplineArrays = 14;
 // every warp of the SM; the serial parts use one or two warps
 constexpr int kSplineThreads = 1024;
 
+template <bool LANES>
 __global__ void __launch_bounds__(kSplineThreads) k_spline_fit(SplineArgs A) {
   __shared__ float red[33 * 4];
   extern __shared__ float4 shf4[];
   float* shf = reinterpret_cast<float*>(shf4);
   const int n = A.n, m = n - 2, tid = threadIdx.x, nt = blockDim.x;
   const int mp = spline_stride(n);
-  double* const ws = A.ws + blockIdx.z * A.lane;
+  double* const ws = A.ws + (LANES ? blockIdx.z * A.lane : 0);
   double* xs = ws;
   double* yx = xs + n;
   double* yy = yx + n;
@@ -901,6 +903,7 @@ struct ColShared {
   int sc[kColCols];
 };
 
+template <bool LANES>
 __global__ void __launch_bounds__(kColThreads) k_shock_columns(ColArgs A) {
   __shared__ ColShared sh;
   const hymor_config& c = A.cfg;
@@ -908,8 +911,8 @@ __global__ void __launch_bounds__(kColThreads) k_shock_columns(ColArgs A) {
   const int lane = threadIdx.x % kColCols, w = threadIdx.x / kColCols;
   const int i = blockIdx.x * kColCols + lane;
   const bool act = i < nchi;
-  const long off = blockIdx.z * A.lane;
-  const double* xs = A.ws + blockIdx.z * A.ws_lane;
+  const long off = LANES ? blockIdx.z * A.lane : 0;
+  const double* xs = A.ws + (LANES ? blockIdx.z * A.ws_lane : 0);
   const double* cxs = xs + 3 * nchi;
   const double* cys = xs + 4 * nchi;
   const double* gxs = xs + 5 * nchi;
@@ -1116,6 +1119,7 @@ struct BcArgs {
 };
 
 // point t of the two edges of one phase (0: chi edges, 1: eta edges)
+template <bool LANES>
 __device__ __forceinline__ void bc_edge_point(const BcArgs& A, int phase, int t) {
   const hymor_config& c = A.cfg;
   const int nchi = c.nchi, neta = c.neta, NI = nchi + 2, NJ = neta + 2;
@@ -1125,7 +1129,7 @@ __device__ __forceinline__ void bc_edge_point(const BcArgs& A, int phase, int t)
   const int bc = edge == 0 ? c.bc_chi0 : edge == 1 ? c.bc_chi1 : edge == 2 ? c.bc_eta0 : c.bc_eta1;
   if (bc == HYMOR_BC_SHOCK) return;
   EdgeCtx e{edge, bc, NI, NJ, nchi, neta};
-  const long off = blockIdx.z * A.lane;
+  const long off = LANES ? blockIdx.z * A.lane : 0;
   const Cons q = lane_cons(A.q, off);
   edge_bc_point(c, e, A.m, q, A.p + off, A.T + off, A.a_bc + off, k, len);
   if (bc == HYMOR_BC_SYMMETRY) {
@@ -1140,6 +1144,7 @@ __device__ __forceinline__ void bc_edge_point(const BcArgs& A, int phase, int t)
 
 // One boundary phase, one thread per edge point: the chi edges, then (second launch) the
 // eta edges, whose corners read the chi ghosts.
+template <bool LANES>
 __global__ void __launch_bounds__(256) k_bc_edges(BcArgs A) {
   const int len = A.phase == 0 ? A.cfg.neta + 2 : A.cfg.nchi + 2;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1147,7 +1152,25 @@ __global__ void __launch_bounds__(256) k_bc_edges(BcArgs A) {
     A.pS.x[0] = A.pS.x[1];
     if (!A.on_S) A.pts.x[0] = A.pts.x[1];
   }
-  if (t < 2 * len) bc_edge_point(A, A.phase, t);
+  if (t < 2 * len) bc_edge_point<LANES>(A, A.phase, t);
+}
+
+// Both phases in one launch, for grids whose phases have at most kBcOneBlock points: one block
+// takes the chi edges, meets at its barrier and takes the eta edges. A launch and its dependency
+// cost 3-4 us of the chain that the residual waits for (180 x 60; the RK step of 100 x 80: 214 ->
+// 212 us), but a phase of several passes of one block loses that again (334 x 137: 0.98 times the
+// speed; 800 x 400: the chain 5-9 us longer).
+constexpr int kBcOneBlock = 512;
+template <bool LANES>
+__global__ void __launch_bounds__(kBcOneBlock) k_bc_edges_one(BcArgs A) {
+  const int l0 = 2 * (A.cfg.neta + 2), l1 = 2 * (A.cfg.nchi + 2);
+  if (A.fix_pts && threadIdx.x == 0 && A.cfg.nchi >= 2) {
+    A.pS.x[0] = A.pS.x[1];
+    if (!A.on_S) A.pts.x[0] = A.pts.x[1];
+  }
+  for (int t = threadIdx.x; t < l0; t += blockDim.x) bc_edge_point<LANES>(A, 0, t);
+  __syncthreads();
+  for (int t = threadIdx.x; t < l1; t += blockDim.x) bc_edge_point<LANES>(A, 1, t);
 }
 
 // ---------------------------------------------------------------------------
@@ -1841,6 +1864,29 @@ __device__ __forceinline__ double cell_c2(const SoundArgs& A, long k, int i, int
   return A.gamma * p * ir;
 }
 
+// UPDATE_THERMODYNAMIC_PROPERTIES and UPDATE_SOUND_SPEED of S in one pass (k_update_thermo mode 3
+// and k_sound_cmax mode 1 without its maximum): both form p from the same four values, and a
+// launch on a small grid costs as much as its work (180 x 60: 5.2 + 5.8 us in two kernels).
+__global__ void __launch_bounds__(256) k_thermo_sound(UpdArgs a, SoundArgs A) {
+  const int NI = a.nchi + 2, NJ = a.neta + 2;
+  const long G = (long)NI * NJ;
+  for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < G; k += (long)gridDim.x * blockDim.x) {
+    const int i = (int)((unsigned)k % (unsigned)NI), j = (int)((unsigned)k / (unsigned)NI);
+    const double r = a.S.rho[k], u = a.S.ru[k], v = a.S.rv[k], e = a.S.rE[k];
+    const double ir = frcp(r);
+    const double eint = fma(-0.5, fma(u, u, v * v) * ir, e);
+    const double p = eint * a.gm1;
+    a.p[k] = p;
+    a.T[k] = eint * ir;
+    A.aS[k] = sqrt(j == 0 && A.isothermal_eta0 ? cell_c2(A, k, i, j) : A.gamma * p * ir);
+    const bool nb = ((a.nrcbc & 1) && i == 1) || ((a.nrcbc & 2) && i == NI - 2) || ((a.nrcbc & 4) && j == 1) ||
+                    ((a.nrcbc & 8) && j == NJ - 2);
+    if (nb) a.aY[k] = sqrt((a.gm1 + 1) * p / r);
+    if (i >= 1 && i <= a.nchi && j >= 1 && j <= a.neta && !(positive(r) && positive(p)))
+      atomicOr(&a.err[kErrFlags], kBitNumeric);
+  }
+}
+
 __global__ void __launch_bounds__(256) k_sound_cmax(SoundArgs A) {
   const int NI = A.nchi + 2, NJ = A.neta + 2;
   const long G = (long)NI * NJ;
@@ -2347,7 +2393,7 @@ int grid_for(long n, int threads) {
 // ===========================================================================
 // launchers
 
-void launch_update_thermo(const DevCtx& d, int mode, double cY, double cS, cudaStream_t st) {
+static UpdArgs upd_args(const DevCtx& d, int mode, double cY, double cS) {
   UpdArgs a;
   a.S = d.S;
   a.Y = d.Y;
@@ -2368,7 +2414,11 @@ void launch_update_thermo(const DevCtx& d, int mode, double cY, double cS, cudaS
   a.aY = d.aY;
   a.nrcbc = (d.cfg.bc_chi0 == HYMOR_BC_OUTFLOW_NRCBC) | ((d.cfg.bc_chi1 == HYMOR_BC_OUTFLOW_NRCBC) << 1) |
             ((d.cfg.bc_eta0 == HYMOR_BC_OUTFLOW_NRCBC) << 2) | ((d.cfg.bc_eta1 == HYMOR_BC_OUTFLOW_NRCBC) << 3);
-  k_update_thermo<<<grid_for(d.G, 256), 256, 0, st>>>(a);
+  return a;
+}
+
+void launch_update_thermo(const DevCtx& d, int mode, double cY, double cS, cudaStream_t st) {
+  k_update_thermo<<<grid_for(d.G, 256), 256, 0, st>>>(upd_args(d, mode, cY, cS));
 }
 
 void launch_spline(const DevCtx& d, bool on_S, bool copy_pts, cudaStream_t st) {
@@ -2382,8 +2432,10 @@ void launch_spline(const DevCtx& d, bool on_S, bool copy_pts, cudaStream_t st) {
   sa.n = d.nchi;
   sa.copy_pts = copy_pts;
   sa.lane = d.lane_stride;
-  k_spline_rows<<<dim3((d.nchi + 127) / 128, 1, d.lanes), 128, 0, st>>>(sa);
-  k_spline_fit<<<dim3(1, 1, d.lanes), kSplineThreads, sizeof(float) * kSplineArrays * spline_stride(d.nchi), st>>>(sa);
+  // (the single-lane kernels without the lane offsets: the RK step's serial chain waits for them)
+  const bool ln = d.lanes > 1;
+  (ln ? k_spline_rows<true> : k_spline_rows<false>)<<<dim3((d.nchi + 127) / 128, 1, d.lanes), 128, 0, st>>>(sa);
+  (ln ? k_spline_fit<true> : k_spline_fit<false>)<<<dim3(1, 1, d.lanes), kSplineThreads, sizeof(float) * kSplineArrays * spline_stride(d.nchi), st>>>(sa);
 }
 
 void launch_columns_bc(const DevCtx& d, bool on_S, bool move, double cY, double cS, int a_mode, bool do_shock,
@@ -2432,7 +2484,7 @@ void launch_columns_bc(const DevCtx& d, bool on_S, bool move, double cY, double 
     ca.two_igm1 = 2 / (c.gamma - 1);
     ca.lane = d.lane_stride;
     ca.ws_lane = d.spl_shared ? 0 : d.lane_stride;
-    k_shock_columns<<<dim3((d.nchi + kColCols - 1) / kColCols, 1, d.lanes), kColThreads, 0, st>>>(ca);
+    (d.lanes > 1 ? k_shock_columns<true> : k_shock_columns<false>)<<<dim3((d.nchi + kColCols - 1) / kColCols, 1, d.lanes), kColThreads, 0, st>>>(ca);
   }
   const bool fix = shock && move && c.bc_chi0 == HYMOR_BC_SYMMETRY;
   if (do_bc || fix) {
@@ -2454,11 +2506,15 @@ void launch_columns_bc(const DevCtx& d, bool on_S, bool move, double cY, double 
     }
     ba.lane = d.lane_stride;
     ba.phase = 0;
-    k_bc_edges<<<dim3((2 * d.NJ + 255) / 256, 1, d.lanes), 256, 0, st>>>(ba);
+    if (do_bc && 2 * std::max(d.NI, d.NJ) <= kBcOneBlock) {
+      (d.lanes > 1 ? k_bc_edges_one<true> : k_bc_edges_one<false>)<<<dim3(1, 1, d.lanes), 2 * std::max(d.NI, d.NJ) <= 256 ? 256 : kBcOneBlock, 0, st>>>(ba);
+      return;
+    }
+    (d.lanes > 1 ? k_bc_edges<true> : k_bc_edges<false>)<<<dim3((2 * d.NJ + 255) / 256, 1, d.lanes), 256, 0, st>>>(ba);
     if (do_bc) {
       ba.phase = 1;
       ba.fix_pts = 0;
-      k_bc_edges<<<dim3((2 * d.NI + 255) / 256, 1, d.lanes), 256, 0, st>>>(ba);
+      (d.lanes > 1 ? k_bc_edges<true> : k_bc_edges<false>)<<<dim3((2 * d.NI + 255) / 256, 1, d.lanes), 256, 0, st>>>(ba);
     }
   }
 }
@@ -2605,7 +2661,11 @@ void launch_flux_class(const DevCtx& d, bool on_S, double* const out[4], int til
   a.err = d.err;
   a.lane = d.lane_stride;
   // the split tiling's classes: half-height tiles, halo by thread loads
-  const bool half = flux_split(d) && tile_class >= 0 && d.tiles;
+  // and a whole grid of few tiles: an FP64 tile takes as long as its warps' FP64 instructions on
+  // one SM, so half the warps on twice the SMs finish sooner while SMs are idle (180 x 60,
+  // the residual without its copy to the host, with k_thermo_sound and k_bc_edges_one: 48 -> 36 us)
+  const bool few = tile_class < 0 && !ffv && d.lanes == 1 && flux_tiles(d) <= d.sms;
+  const bool half = (flux_split(d) && tile_class >= 0 && d.tiles) || few;
   const int rows = half ? TY / 2 : flux_rows(d);
   const bool tma = d.tma && !half;
   FluxMaps tm;
@@ -2684,8 +2744,9 @@ void flux_kernel_setup() {
   flux_setup_variant<true, 16, true>();
   flux_setup_variant<false, TY / 2, false>();
   flux_setup_variant<true, TY / 2, false>();
-  cudaFuncSetAttribute(k_spline_fit, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(float) * kSplineArrays * spline_stride(4096));
+  for (auto* fit : {k_spline_fit<false>, k_spline_fit<true>})
+    cudaFuncSetAttribute(fit, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sizeof(float) * kSplineArrays * spline_stride(4096));
 }
 
 void launch_flow_cells(const DevCtx& d, cudaStream_t st) {
@@ -2702,7 +2763,7 @@ void launch_flow_cells(const DevCtx& d, cudaStream_t st) {
   k_flow_cells<<<(d.nchi * 32 + 63) / 64, 64, 0, st>>>(A);
 }
 
-void launch_sound_cmax(const DevCtx& d, bool recompute, cudaStream_t st, bool max_only) {
+static SoundArgs sound_args(const DevCtx& d, int mode) {
   SoundArgs A;
   A.S = d.S;
   A.aS = d.aS;
@@ -2711,11 +2772,19 @@ void launch_sound_cmax(const DevCtx& d, bool recompute, cudaStream_t st, bool ma
   A.gamma = d.cfg.gamma;
   A.nchi = d.nchi;
   A.neta = d.neta;
-  A.mode = recompute ? (max_only ? 2 : 1) : 0;
+  A.mode = mode;
   A.nrcbc = (d.cfg.bc_chi0 == HYMOR_BC_OUTFLOW_NRCBC) | ((d.cfg.bc_chi1 == HYMOR_BC_OUTFLOW_NRCBC) << 1) |
             ((d.cfg.bc_eta0 == HYMOR_BC_OUTFLOW_NRCBC) << 2) | ((d.cfg.bc_eta1 == HYMOR_BC_OUTFLOW_NRCBC) << 3);
   A.isothermal_eta0 = d.cfg.bc_eta0 == HYMOR_BC_NO_SLIP_ISOTHERMAL;
-  k_sound_cmax<<<grid_for(d.G, 256), 256, 0, st>>>(A);
+  return A;
+}
+
+void launch_sound_cmax(const DevCtx& d, bool recompute, cudaStream_t st, bool max_only) {
+  k_sound_cmax<<<grid_for(d.G, 256), 256, 0, st>>>(sound_args(d, recompute ? (max_only ? 2 : 1) : 0));
+}
+
+void launch_thermo_sound(const DevCtx& d, cudaStream_t st) {
+  k_thermo_sound<<<grid_for(d.G, 256), 256, 0, st>>>(upd_args(d, 3, 0, 0), sound_args(d, 1));
 }
 
 void launch_cfl(const DevCtx& d, cudaStream_t st) {

@@ -138,6 +138,8 @@ void launch_flow_cells(const DevCtx& d, cudaStream_t st);
 // Sound speed of S (recompute) and max|a| into scal[kCmax]; recompute=false only reduces aS.
 // max_only (with recompute): the max, and a only on the lines outflow_NRCBC reads.
 void launch_sound_cmax(const DevCtx& d, bool recompute, cudaStream_t st, bool max_only = false);
+// Thermodynamic state of S (launch_update_thermo mode 3) and its sound speed in one pass.
+void launch_thermo_sound(const DevCtx& d, cudaStream_t st);
 // CFL maxima and dt (scal[kDt]).
 void launch_cfl(const DevCtx& d, cudaStream_t st);
 void launch_cfl_screened(const DevCtx& d, cudaStream_t st);

@@ -2318,12 +2318,10 @@ int hymor_linearize(hymor_ctx* ctx) {
   // LINEARIZE_L.jl:43-56: flow cells and shock BC, thermo, sound speed, boundary conditions
   if (d.cfg.shock_enabled) {
     launch_flow_cells(d, st);
-    launch_update_thermo(d, 3, 0, 0, st);
-    launch_sound_cmax(d, true, st);
+    launch_thermo_sound(d, st);
     launch_shock_bc_flags(d, true, false, true, false, 1, st);
   }
-  launch_update_thermo(d, 3, 0, 0, st);
-  launch_sound_cmax(d, true, st);
+  launch_thermo_sound(d, st);
   launch_shock_bc_flags(d, true, false, false, true, 1, st);
   std::vector<int> rows;
   if (shock_blocks) {
