@@ -502,6 +502,7 @@ struct MvFf {
   Wrap w;
   long N, ld;
   int k, transpose;
+  int chunk;  // vectors per item of matvec_tile_ff
 };
 
 __device__ __forceinline__ ff ldff(const float2* p, long i) {
@@ -583,44 +584,32 @@ __device__ __forceinline__ void matvec_one_ff(const MvFf& a) {
   }
 }
 
-// (cell, chunk of KV vectors) items, as matvec_multi (KV = kVecChunk; KV = 1 for a single
-// vector on a large grid, where the smaller register set raises the occupancy of this
-// HBM-bound case: the 144 block entries are read once per cell and vector)
-template <int KV, bool ST>
-__device__ __forceinline__ void matvec_multi_ff(const MvFf& a) {
+// One vector on a large grid: a cell per thread and vector, one neighbour block at a time (its
+// 16 pairs in registers). The 144 block entries are read once per cell and vector, so this case
+// is bound by HBM, and the small register set raises the occupancy that keeps its loads in
+// flight.
+template <bool ST>
+__device__ __forceinline__ void matvec_cell_ff(const MvFf& a) {
   const long N = a.N;
-  const long n4 = a.ld;
-  const int chunks = (a.k + KV - 1) / KV;
-  const long items = N * chunks;
   const unsigned N_u = (unsigned)N, nchi_u = (unsigned)a.w.nchi;
-  for (long w = blockIdx.x * (long)blockDim.x + threadIdx.x; w < items; w += (long)gridDim.x * blockDim.x) {
-    const unsigned wu = (unsigned)w;
-    const unsigned ch = wu / N_u;
-    const unsigned m = wu - ch * N_u;
+  for (long w = blockIdx.x * (long)blockDim.x + threadIdx.x; w < N * a.k; w += (long)gridDim.x * blockDim.x) {
+    const unsigned wu = (unsigned)w, vec = wu / N_u, m = wu - vec * N_u;
     const unsigned j_u = m / nchi_u;
     const int i = (int)(m - j_u * nchi_u), j = (int)j_u;
-    const int v0 = (int)ch * KV;
-    const int nv = min(KV, a.k - v0);
-    ff y[KV][4];
+    const float2* x = a.X + (long)vec * a.ld;
+    const long o = (long)vec * a.ld + m;
+    if (!(a.nz[m] & (a.transpose ? kMaskCol : kMaskRow))) {
+      const float z = ff_poison_window(a, x, i, j);
 #pragma unroll
-    for (int v = 0; v < KV; ++v)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) y[v][c] = ff{0.0f, 0.0f};
-    if (KV == 1 && !(a.nz[m] & (a.transpose ? kMaskCol : kMaskRow))) {
-#pragma unroll
-      for (int v = 0; v < KV; ++v)
-        if (v < nv) {
-          const float z = ff_poison_window(a, a.X + (long)(v0 + v) * n4, i, j);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) mvff_out(a, v0 + v, (long)(v0 + v) * n4 + c * N + m, ff{z, 0.0f});
-        }
+      for (int c = 0; c < 4; ++c) mvff_out(a, (int)vec, o + c * N, ff{z, 0.0f});
       continue;
     }
-    // one neighbour block at a time for a single vector (its 16 pairs in registers), all
-    // nine unrolled for a chunk
-#pragma unroll(KV == 1 ? 1 : 3)
+    ff y[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) y[c] = ff{0.0f, 0.0f};
+#pragma unroll 1
     for (int b = -1; b <= 1; ++b)
-#pragma unroll(KV == 1 ? 1 : 3)
+#pragma unroll 1
       for (int aa = -1; aa <= 1; ++aa) {
         const long n = a.transpose ? a.w.nbr(i, j, -aa, -b) : a.w.nbr(i, j, aa, b);
         if (n < 0) continue;
@@ -629,89 +618,128 @@ __device__ __forceinline__ void matvec_multi_ff(const MvFf& a) {
         ff B[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) B[e] = ldff_coef<ST>(a.coef, (long)(q * 16 + e) * N + cell);
-        // unrolled over the chunk with a predicate, so that the pairs of y stay in registers
+        const ff xs[4] = {ldff(x, n), ldff(x, N + n), ldff(x, 2 * N + n), ldff(x, 3 * N + n)};
 #pragma unroll
-        for (int v = 0; v < KV; ++v) {
-          if (v >= nv) continue;
-          const float2* x = a.X + (long)(v0 + v) * n4;
-          const ff xs[4] = {ldff(x, n), ldff(x, N + n), ldff(x, 2 * N + n), ldff(x, 3 * N + n)};
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            // row c of the block, or column c for the transpose
-            const ff bs[4] = {B[a.transpose ? c : c * 4], B[a.transpose ? 4 + c : c * 4 + 1],
-                              B[a.transpose ? 8 + c : c * 4 + 2], B[a.transpose ? 12 + c : c * 4 + 3]};
-            y[v][c] = ff_dot4(bs, xs, y[v][c]);
-          }
+        for (int c = 0; c < 4; ++c) {
+          // row c of the block, or column c for the transpose
+          const ff bs[4] = {B[a.transpose ? c : c * 4], B[a.transpose ? 4 + c : c * 4 + 1],
+                            B[a.transpose ? 8 + c : c * 4 + 2], B[a.transpose ? 12 + c : c * 4 + 3]};
+          y[c] = ff_dot4(bs, xs, y[c]);
         }
       }
 #pragma unroll
-    for (int v = 0; v < KV; ++v)
-      if (v < nv)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) mvff_out(a, v0 + v, (long)(v0 + v) * n4 + c * N + m, y[v][c]);
+    for (int c = 0; c < 4; ++c) mvff_out(a, (int)vec, o + c * N, y[c]);
   }
 }
 
-// (cell, output component, chunk of KV vectors) items: 4 block entries per neighbour in
-// registers instead of 16, for the occupancy that keeps the FP32 pipe busy with a batch
-// (the four threads of a cell read its inputs four times, from L1)
+// A batch of vectors: a block takes a tile of 32 x kFfRows cells and a chunk of up to kVecChunk
+// vectors, stages the vectors' tile and halo in shared memory, and a thread forms the outputs of
+// its cell for the chunk (four components each). What bounds it is the FP32 pipe (~1950
+// instructions per cell and vector, 16 independent chains per thread) and the latency of the 16
+// pairs of a neighbour block, which four blocks of four warps on an SM, each at its own place,
+// hide in part (FP32 pipe 36 %, issue slots 46 % busy by ncu). Before, a thread per component
+// read the inputs from global memory for every neighbour: 38 x 4 loads of L2 per cell and vector.
+// 600 x 300, 8 vectors, adjoint, us per matvec of the batch: 279 before; 178 in tiles of 32 x 8
+// cells; 159 in tiles of 32 x 4 with the cells without entries left out (187 with the pairs by
+// cp.async through a double buffer, 181 with an L2 prefetch of them, 174 with two components of
+// eight vectors per thread and the next pairs in registers). The chunk index runs fastest, so
+// that the blocks of a tile's chunks read its pairs at about the same time.
+constexpr int kFfRows = 4;
+constexpr int kFfHx = 34, kFfHalo = kFfHx * (kFfRows + 2), kFfThreads = 32 * kFfRows;
+template <int KV>
+constexpr int ff_tile_smem() { return KV * 4 * kFfHalo * (int)sizeof(float2); }
+long ff_tiles(const Wrap& w) { return (long)((w.nchi + 31) / 32) * ((w.neta + kFfRows - 1) / kFfRows); }
+
 template <int KV, bool ST>
-__device__ __forceinline__ void matvec_comp_ff(const MvFf& a) {
+__device__ __forceinline__ void matvec_tile_ff(const MvFf& a, float2* xs) {
   const long N = a.N;
-  const long n4 = a.ld;
-  const int chunks = (a.k + KV - 1) / KV;
-  const long items = 4 * N * chunks;
-  const unsigned N_u = (unsigned)N, nchi_u = (unsigned)a.w.nchi;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < items; t += (long)gridDim.x * blockDim.x) {
-    const unsigned tu = (unsigned)t;
-    const unsigned r = tu / N_u;
-    const unsigned m = tu - r * N_u;
-    const int comp = (int)(r & 3u);
-    const int v0 = (int)(r >> 2) * KV;
-    const int nv = min(KV, a.k - v0);
-    const unsigned j_u = m / nchi_u;
-    const int i = (int)(m - j_u * nchi_u), j = (int)j_u;
-    ff y[KV];
+  const int nchi = a.w.nchi, neta = a.w.neta;
+  const int kv = a.chunk, chunks = (a.k + kv - 1) / kv, tx = (nchi + 31) / 32;
+  const int items = tx * ((neta + kFfRows - 1) / kFfRows) * chunks;
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  // block slot q of (aa, b): input cell (i + aa, j + b), or of the transpose the output cell
+  // (i - aa, j - b), which owns the block
+  const int sg = a.transpose ? -1 : 1;
+  const long sc = a.transpose ? N : 4 * N, se = a.transpose ? 4 * N : N;
+  for (int it = blockIdx.x; it < items; it += gridDim.x) {
+    const int tile = it / chunks, v0 = (it - tile * chunks) * kv, nv = min(kv, a.k - v0);
+    const int i0 = (tile % tx) * 32, j0 = (tile / tx) * kFfRows;
+    const int i = i0 + lane, j = j0 + row;
+    const long m = i + (long)j * nchi;
+    const bool in = i < nchi && j < neta;
+    const bool act = in && (a.nz[m] & (a.transpose ? kMaskCol : kMaskRow));
+    // cells past the grid's edge wrap where it is periodic; the others are never used
+    for (int h = threadIdx.x; h < kFfHalo; h += kFfThreads) {
+      int ii = i0 - 1 + h % kFfHx, jj = j0 - 1 + h / kFfHx;
+      if (a.w.per_chi) ii = ii < 0 ? ii + nchi : (ii >= nchi ? ii - nchi : ii);
+      if (a.w.per_eta) jj = jj < 0 ? jj + neta : (jj >= neta ? jj - neta : jj);
+      if (ii < 0 || ii >= nchi || jj < 0 || jj >= neta) continue;
+      const float2* x = a.X + (long)v0 * a.ld + ii + (long)jj * nchi;
 #pragma unroll
-    for (int v = 0; v < KV; ++v) y[v] = ff{0.0f, 0.0f};
+      for (int v = 0; v < KV; ++v)
+        if (v < nv)
 #pragma unroll
-    for (int q = 0; q < 9; ++q) {
-      const int b = q / 3 - 1, aa = q % 3 - 1;
-      const long n = a.transpose ? a.w.nbr(i, j, -aa, -b) : a.w.nbr(i, j, aa, b);
-      if (n < 0) continue;
-      const long cell = a.transpose ? n : m;
-      ff B[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int plane = a.transpose ? q * 16 + e * 4 + comp : q * 16 + comp * 4 + e;
-        B[e] = ldff_coef<ST>(a.coef, (long)plane * N + cell);
-      }
-#pragma unroll
-      for (int v = 0; v < KV; ++v) {
-        if (v >= nv) continue;
-        const float2* x = a.X + (long)(v0 + v) * n4;
-        const ff xs[4] = {ldff(x, n), ldff(x, N + n), ldff(x, 2 * N + n), ldff(x, 3 * N + n)};
-        y[v] = ff_dot4(B, xs, y[v]);
-      }
+          for (int e = 0; e < 4; ++e) xs[(v * 4 + e) * kFfHalo + h] = x[v * a.ld + e * N];
     }
+    __syncthreads();
+    if (in) {
+      ff y[KV][4];
 #pragma unroll
-    for (int v = 0; v < KV; ++v)
-      if (v < nv) mvff_out(a, v0 + v, (long)(v0 + v) * n4 + comp * N + m, y[v]);
+      for (int v = 0; v < KV; ++v)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) y[v][c] = ff{0.0f, 0.0f};
+#pragma unroll 1
+      for (int q = 0; q < 9; ++q) {
+        const int da = sg * (q % 3 - 1), db = sg * (q / 3 - 1);
+        const float2* xq = xs + (lane + 1 + da) + (row + 1 + db) * kFfHx;
+        const long n = a.w.nbr(i, j, da, db);
+        if (n < 0) continue;
+        if (act) {
+          const float2* p = a.coef + (long)(q * 16) * N + (a.transpose ? n : m);
+          ff B[16];
+#pragma unroll
+          for (int c = 0; c < 4; ++c)  // row c of the block, or column c for the transpose
+#pragma unroll
+            for (int e = 0; e < 4; ++e) B[c * 4 + e] = ldff_coef<ST>(p, c * sc + e * se);
+#pragma unroll
+          for (int v = 0; v < KV; ++v) {
+            if (v >= nv) continue;
+            const ff xv[4] = {ldff(xq, (v * 4) * kFfHalo), ldff(xq, (v * 4 + 1) * kFfHalo),
+                              ldff(xq, (v * 4 + 2) * kFfHalo), ldff(xq, (v * 4 + 3) * kFfHalo)};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) y[v][c] = ff_dot4(B + c * 4, xv, y[v][c]);
+          }
+        } else {  // a cell without entries: zero, or NaN where an input is not finite
+#pragma unroll
+          for (int v = 0; v < KV; ++v)
+            if (v < nv)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float2 t = xq[(v * 4 + e) * kFfHalo];
+                y[v][0].h = __fmaf_rn(t.x, 0.0f, __fmaf_rn(t.y, 0.0f, y[v][0].h));
+              }
+        }
+      }
+#pragma unroll
+      for (int v = 0; v < KV; ++v)
+        if (v < nv)
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            mvff_out(a, v0 + v, (long)(v0 + v) * a.ld + c * N + m, act ? y[v][c] : y[v][0]);
+    }
+    __syncthreads();  // the next item's inputs take the shared memory
   }
 }
 
 // The cooperative propagation in float-float (degree >= 2, the late-sum order of
 // k_expm_coop): the input vectors are split into the running sum, and the sum is joined
-// into the FP64 output after the last step. MODE 0: matvec_comp_ff<kVecChunk> (a batch on a
-// large grid), 1: matvec_one_ff (few cells x vectors), 2: matvec_multi_ff<1> (one vector on
-// a large grid), 3: matvec_multi_ff<kVecChunk> (a batch on a small grid). Measured on the
-// 800 x 400 Jacobian: 68 us per vector-matvec for one vector (MODE 2; 111 in FP64) and for
-// 8 (MODE 0; 83 with MODE 3, 91 in FP64); 64 vectors on the 100 x 80 one: 18.5 ms for 250
-// matvecs with MODE 3, 24 with MODE 0, 40 in FP64.
+// into the FP64 output after the last step. MODE 0: matvec_tile_ff (a batch), 1: matvec_one_ff
+// (few cells x vectors: ff_one), 2: matvec_cell_ff (one vector).
 template <int MODE, bool ST>
-__global__ void __launch_bounds__(kMvThreads, MODE == 1 || MODE == 3 ? 2 : 3) k_expm_coop_ff(MvFf base, int nsteps, int order, const double* xin,
+__global__ void __launch_bounds__(MODE == 0 ? kFfThreads : kMvThreads, MODE == 0 ? 4 : (MODE == 2 ? 3 : 2)) k_expm_coop_ff(MvFf base, int nsteps, int order, const double* xin,
                                                                 double* yout, float2* t1, float2* t2, float2* vout,
                                                                 const int* vsteps) {
+  extern __shared__ float2 ff_tile[];
   cg::grid_group grid = cg::this_grid();
   const long nall = base.ld * (long)base.k;
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < nall; q += (long)gridDim.x * blockDim.x)
@@ -738,9 +766,8 @@ __global__ void __launch_bounds__(kMvThreads, MODE == 1 || MODE == 3 ? 2 : 3) k_
       a.c_prev = c_prev;
       a.c_acc = ff_from_double(1.0 / (double)fact);
       if (MODE == 1) matvec_one_ff<ST>(a);
-      else if (MODE == 2) matvec_multi_ff<1, ST>(a);
-      else if (MODE == 3) matvec_multi_ff<kVecChunk, ST>(a);
-      else matvec_comp_ff<kVecChunk, ST>(a);
+      else if (MODE == 2) matvec_cell_ff<ST>(a);
+      else matvec_tile_ff<kVecChunk, ST>(a, ff_tile);
       grid.sync();
       src = a.Y;
       prev = j == 1 ? a.Y : nullptr;
@@ -2104,8 +2131,8 @@ struct KrylovScratch {
 struct LinearState {
   ExpmCache expm;
   KrylovScratch kry;
-  int coop_blocks[12] = {};  // co-resident blocks per SM of k_expm_coop<false>, <true>,
-                             // k_expm_coop_ff<0>, <1>, <2>, <3>, each with ordinary and
+  int coop_blocks[10] = {};  // co-resident blocks per SM of k_expm_coop<false>, <true>,
+                             // k_expm_coop_ff<0>, <1>, <2>, each with ordinary and
                              // streaming block loads
   JacLanes lanes;               // workspaces of the linearisations' perturbed residuals
 };
@@ -2168,9 +2195,15 @@ int ensure_lanes(hymor_ctx* ctx, JacLanes** out) {
   return 0;
 }
 
-// grids from this many cells take the thread-per-component float-float batch
-constexpr long kFfCompCells = 65536;
-
+// Cells x vectors below which the float-float propagation gives every output a thread: there it
+// is bound by the latency of a pass, above by the loads and products, which a cell per thread
+// (one vector) and the tiles (a batch) make once for four outputs. A propagation of one context
+// alone, thread per output against the other, ms: one vector, 250 matvecs, 100 x 80 1.40 / 2.82,
+// 200 x 150 2.81 / 3.09, 300 x 200 8.12 / 4.83, 400 x 300 13.8 / 6.6; 150 matvecs of 100 x 80
+// with 4 vectors 1.72 / 2.81, 8 vectors 3.06 / 3.09, 16 vectors 5.10 / 3.79, of 200 x 100 with 2
+// vectors 2.41 / 2.08, of 300 x 200 with 2 vectors 8.29 / 3.26.
+constexpr long kFfOneCells = 40000;
+bool ff_one(long N, int k) { return N * k < kFfOneCells; }
 
 // hdts, hsteps (host, k entries, hsteps non-increasing), or null: vector c is propagated
 // hsteps[c] steps of hdts[c] instead of nsteps of dt.
@@ -2210,25 +2243,25 @@ int expm_cooperative(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
   }
   int* blocks_per_sm = linear_state(ctx).coop_blocks;
   const bool one = mv_one(d.N, k, d.sms);
-  // float-float: thread per output on few cells x vectors, one cell per thread for one vector,
-  // a thread per output component for a batch on a large grid, a chunk per thread on a small
-  const int ffmode = one ? 1 : (k == 1 ? 2 : (d.N >= kFfCompCells ? 0 : 3));
+  // float-float: thread per output on few cells x vectors, else a cell per thread for one vector
+  // and tiles for a batch
+  const int ffmode = ff_one(d.N, k) ? 1 : (k == 1 ? 2 : 0);
   const int kind = ffp ? 2 + ffmode : (one ? 1 : 0);
   const int kst = 2 * kind + coef_stream(d);
-  const void* kerns[12] = {(const void*)k_expm_coop<false, false>,  (const void*)k_expm_coop<false, true>,
+  const void* kerns[10] = {(const void*)k_expm_coop<false, false>,  (const void*)k_expm_coop<false, true>,
                            (const void*)k_expm_coop<true, false>,   (const void*)k_expm_coop<true, true>,
                            (const void*)k_expm_coop_ff<0, false>,   (const void*)k_expm_coop_ff<0, true>,
                            (const void*)k_expm_coop_ff<1, false>,   (const void*)k_expm_coop_ff<1, true>,
-                           (const void*)k_expm_coop_ff<2, false>,   (const void*)k_expm_coop_ff<2, true>,
-                           (const void*)k_expm_coop_ff<3, false>,   (const void*)k_expm_coop_ff<3, true>};
+                           (const void*)k_expm_coop_ff<2, false>,   (const void*)k_expm_coop_ff<2, true>};
   const void* kern = kerns[kst];
   if (!blocks_per_sm[kst] &&
-      (r = cuda_check(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm[kst], kern, kMvThreads, 0))))
+      (r = cuda_check(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm[kst], kern, kind == 2 ? kFfThreads : kMvThreads,
+                                                                        kind == 2 ? ff_tile_smem<kVecChunk>() : 0))))
     return r;
-  // the batched float-float path takes a thread per output component
-  const long items = mv_items(d.N, k, d.sms) * (kind == 2 ? 4 : 1);
-  const int th = mv_threads(items, d.sms);
-  const long want = (items + th - 1) / th;
+  const long items = kind == 4 ? d.N : (kind == 3 ? 4 * d.N * k : mv_items(d.N, k, d.sms));
+  const int th = kind == 2 ? kFfThreads : mv_threads(items, d.sms);
+  const int nch = (k + kVecChunk - 1) / kVecChunk, chunk = (k + nch - 1) / nch;
+  const long want = kind == 2 ? ff_tiles(make_wrap(d.cfg)) * ((k + chunk - 1) / chunk) : (items + th - 1) / th;
   // co-resident: blocks of th <= 256 threads need no more than a 256-thread block
   const int grid = (int)std::min<long>(want, (long)blocks_per_sm[kst] * d.sms);
   MvArgs base;
@@ -2273,11 +2306,13 @@ int expm_cooperative(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
     bf.ld = base.ld;
     bf.k = k;
     bf.transpose = transpose;
+    bf.chunk = chunk;
     float2* f1 = reinterpret_cast<float2*>(t1);
     float2* f2 = reinterpret_cast<float2*>(t2);
     float2* fo = reinterpret_cast<float2*>(vout);
     void* fargs[] = {&bf, &nsteps, &order, &dX, &dY, &f1, &f2, &fo, &vsteps};
-    return cuda_check(ctx, cudaLaunchCooperativeKernel(kern, grid, th, fargs, 0, st));
+    return cuda_check(ctx, cudaLaunchCooperativeKernel(kern, grid, th, fargs,
+                                                       kind == 2 ? ff_tile_smem<kVecChunk>() : 0, st));
   }
   if ((r = cuda_check(ctx, cudaMemcpyAsync(v, dX, sizeof(double) * n, cudaMemcpyDeviceToDevice, st)))) return r;
   if ((r = cuda_check(ctx, cudaMemcpyAsync(vout, dX, sizeof(double) * n, cudaMemcpyDeviceToDevice, st)))) return r;
