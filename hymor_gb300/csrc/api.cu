@@ -727,6 +727,10 @@ int hymor_ctx_create(const hymor_config* cfg, const hymor_mesh* mesh, hymor_ctx*
     return bail(fail(ctx, HYMOR_ERR_CUDA, "multiprocessor count"));
   d.coef = nullptr;
   d.coef_nz = nullptr;
+  for (int t = 0; t < 2; ++t) {
+    d.fx_part[t] = nullptr;
+    d.fx_ex[t] = nullptr;
+  }
   d.jwork = nullptr;
   d.sj = ShockJac{};
   d.up_cols = nullptr;

@@ -55,6 +55,11 @@ struct DevCtx {
   // the cell's own blocks have a non-zero entry (4 x N)
   unsigned char* coef_nz;
   float2* coef_ff; // float-float copy of coef for the propagator (or null)
+  // integer parts and exponents of the blocks for the fixed-point matvec, forward and transposed
+  // (or null), and the write of the blocks they were made from
+  int2* fx_part[2];
+  short* fx_ex[2];
+  int fx_version[2];
   int coef_version, coef_ff_version;  // writes of coef, and the write coef_ff was split from
   // the cooperative Taylor propagator in float-float (1, the default) or FP64 (0)
   int expm_ff;
@@ -151,7 +156,7 @@ void launch_classical_stage(const DevCtx& d, double cY, cudaStream_t st);
 
 // ---- linear.cu ----
 void launch_matvec(const DevCtx& d, int k, const double* X, double* Y, int transpose, double scale,
-                   cudaStream_t st, long ld = 0);
+                   cudaStream_t st, long ld = 0, bool fx = false);
 // graph_ok: with the shock blocks, the Taylor steps may be captured once into a CUDA graph
 // and replayed (false: every step is launched directly, nothing is instantiated).
 void launch_expm(const DevCtx& d, int k, double dt, int nsteps, int order, const double* X,

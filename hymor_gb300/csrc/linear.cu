@@ -15,6 +15,7 @@
 #include <algorithm>
 
 #include "ff.cuh"
+#include "fx.cuh"
 #include "kernels.h"
 
 namespace cg = cooperative_groups;
@@ -416,6 +417,219 @@ __device__ __forceinline__ void matvec_multi(const MvArgs& a) {
           }
         }
       }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The batched FP64 matvec in fixed point (fx.cuh). A is kept as integer parts for the direction
+// applied, made once per write of the blocks: entry (input component e, slot q, output row r) of
+// output cell m at plane ((e 9 + q) 4 + r), against the power of two shared by the nine slots of
+// (r, e), whose exponents are 16 planes of 16 bits. A block of 256 threads stages a tile of 32 x
+// 4 cells of up to kFxVecs vectors, each component against the largest exponent of its tile and
+// halo, and a thread forms two rows of its cell: per component the nine slots' products exactly
+// in 64-bit integers, then the four components' sums aligned to the largest and added.
+//
+// Accuracy: the parts and the dropped low product leave ~2^-57 of (largest |a| of a row's nine
+// slots) x (largest |x| of the tile), against 2^-52 to 2^-51 of the sum of |a x| of the FP64
+// chain. Where that sum (formed beside it from 12 leading bits of the factors, a lower bound) is
+// below 2^-5 of that product, the row is formed in FP64 instead: so it is for single small
+// entries (L e_i stays exact: an entry above the line has all its 53 bits within the 58), for
+// tiles with an infinity or a NaN, and for exponents beyond +-900.
+//
+// What bounds it: the integer multiply pipe, 432 wide multiply-adds per cell and vector (FP64:
+// 144 multiply-adds at a fifteenth of that rate, 0.98 of the pipe by ncu), 51 % busy beside the
+// shifts of the alignment and the parts (42 %) and the FP64 rows (11 %). 800 x 400, 64 vectors:
+// 3.64 -> 2.29 ms. Error against sums in 113 bits, relative in the 2-norm, random rows of
+// magnitudes 1e-4 .. 2 and component scales 1e-2 .. 1e2: 5.3e-17 (the FP64 chain: 2.1e-16).
+constexpr int kFxVecs = 4, kFxRows = 4;
+constexpr int kFxHx = 34, kFxHalo = kFxHx * (kFxRows + 2);
+constexpr unsigned kFxLeast = 1u << 19;  // 2^-5 of a full-scale product of the 12-bit leads
+
+struct FxArgs {
+  const int2* part;
+  const short* ex;  // 16 x N, plane r 4 + e
+  MvArgs mv;        // the FP64 blocks, vectors and sizes
+};
+
+template <bool T>
+__global__ void __launch_bounds__(256) k_fx_build(const double* coef, int2* part, short* ex, Wrap w, long N) {
+  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < 16 * N; t += (long)gridDim.x * blockDim.x) {
+    const long m = t % N;
+    const int re = (int)(t / N), r = re >> 2, e = re & 3;
+    const int j = (int)((unsigned)m / (unsigned)w.nchi), i = (int)((unsigned)m - (unsigned)j * (unsigned)w.nchi);
+    double a[9];
+    int f = 0;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+      const int da = q % 3 - 1, db = q / 3 - 1;
+      const long n = T ? w.nbr(i, j, -da, -db) : w.nbr(i, j, da, db);
+      a[q] = n < 0 ? 0.0 : (T ? coef[(long)(q * 16 + e * 4 + r) * N + n] : coef[(long)(q * 16 + re) * N + m]);
+      f = max(f, fx_field(a[q]));
+    }
+    const int E = fx_exponent(f);
+    ex[t] = (short)E;
+#pragma unroll
+    for (int q = 0; q < 9; ++q)
+      part[(long)((e * 9 + q) * 4 + r) * N + m] = E == kFxZero || E == kFxBad ? make_int2(0, 0) : fx_split(a[q], E);
+  }
+}
+
+// row r of cell m on the vector x, in FP64 (matvec_multi's chain)
+__device__ __noinline__ double fx_row_f64(const MvArgs& a, const double* x, long m, int i, int j, int r) {
+  const long N = a.N;
+  double y = 0;
+#pragma unroll 3
+  for (int q = 0; q < 9; ++q) {
+    const int da = q % 3 - 1, db = q / 3 - 1;
+    const long n = a.transpose ? a.w.nbr(i, j, -da, -db) : a.w.nbr(i, j, da, db);
+    if (n < 0) continue;
+    const double* c = a.transpose ? a.coef + (long)(q * 16 + r) * N + n : a.coef + (long)(q * 16 + r * 4) * N + m;
+    const long ce = a.transpose ? 4 * N : N;
+    y = fma(c[0], x[n], fma(c[ce], x[N + n], fma(c[2 * ce], x[2 * N + n], fma(c[3 * ce], x[3 * N + n], y))));
+  }
+  return y;
+}
+
+__global__ void __launch_bounds__(256, 2) k_matvec_fx(FxArgs A) {
+  __shared__ int2 xs[kFxVecs * 4 * kFxHalo];
+  __shared__ int smax[kFxVecs * 4];
+  const MvArgs& a = A.mv;
+  const long N = a.N;
+  const int nchi = a.w.nchi, neta = a.w.neta, tx = (nchi + 31) / 32, chunks = (a.k + kFxVecs - 1) / kFxVecs;
+  const int lane = threadIdx.x & 31, row = (threadIdx.x >> 5) % kFxRows, r0 = (threadIdx.x >> 7) * 2;
+  // the chunk runs fastest: the blocks of a tile's chunks read its parts at about the same time
+  const int tile = blockIdx.x / chunks, v0 = (blockIdx.x - tile * chunks) * kFxVecs, nv = min(kFxVecs, a.k - v0);
+  const int i0 = (tile % tx) * 32, j0 = (tile / tx) * kFxRows;
+  const int i = i0 + lane, j = j0 + row;
+  const long m = i + (long)j * nchi;
+  const bool in = i < nchi && j < neta;
+  if (threadIdx.x < kFxVecs * 4) smax[threadIdx.x] = 0;
+  __syncthreads();
+  // a halo cell per thread: its values, the tile's largest exponent of each, then the parts
+  // (cells past the grid's edge wrap where it is periodic; the others' parts meet zero entries)
+  double xv[kFxVecs * 4];
+  const int h = threadIdx.x;
+  if (h < (kFxHalo + 31) / 32 * 32) {
+    int ii = i0 - 1 + h % kFxHx, jj = j0 - 1 + h / kFxHx;
+    if (a.w.per_chi) ii = ii < 0 ? ii + nchi : (ii >= nchi ? ii - nchi : ii);
+    if (a.w.per_eta) jj = jj < 0 ? jj + neta : (jj >= neta ? jj - neta : jj);
+    const bool ok = h < kFxHalo && ii >= 0 && ii < nchi && jj >= 0 && jj < neta;
+    const double* x = a.X + (long)v0 * a.ld + (ok ? ii + (long)jj * nchi : 0);
+    int mine = 0;
+#pragma unroll
+    for (int c = 0; c < kFxVecs * 4; ++c) {
+      xv[c] = ok && (c >> 2) < nv ? x[(c >> 2) * a.ld + (c & 3) * N] : 0.0;
+      const int f = __reduce_max_sync(0xffffffffu, fx_field(xv[c]));
+      if (lane == c) mine = f;
+    }
+    if (lane < kFxVecs * 4) atomicMax(&smax[lane], mine);
+  }
+  __syncthreads();
+  if (h < kFxHalo) {
+#pragma unroll
+    for (int c = 0; c < kFxVecs * 4; ++c) {
+      const int E = fx_exponent(smax[c]);
+      xs[c * kFxHalo + h] = E == kFxZero || E == kFxBad ? make_int2(0, 0) : fx_split(xv[c], E);
+    }
+  }
+  __syncthreads();
+  if (!in) return;
+  const int sg = a.transpose ? -1 : 1;
+  const int2* x0 = xs + (lane + 1) + (row + 1) * kFxHx;
+  long long T[2][kFxVecs];
+  unsigned S[2][kFxVecs];
+  int top[2][kFxVecs];  // the largest exponent of the four components' products
+  bool f64[2] = {false, false};
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int v = 0; v < kFxVecs; ++v) {
+      T[r][v] = 0;
+      S[r][v] = 0;
+      top[r][v] = -0x7fffffff;
+    }
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int ea = A.ex[((r0 + r) * 4 + e) * N + m];
+      if (ea == kFxBad) f64[r] = true;
+      if (ea == kFxZero) continue;
+#pragma unroll
+      for (int v = 0; v < kFxVecs; ++v) {
+        const int ev = fx_exponent(smax[v * 4 + e]);
+        if (ev != kFxZero) top[r][v] = max(top[r][v], ea + ev);
+      }
+    }
+  // (a cell without entries has nothing to sum: its outputs are zero, or FP64's NaN)
+  const int ne = a.nz[m] & (a.transpose ? kMaskCol : kMaskRow) ? 4 : 0;
+#pragma unroll 1
+  for (int e = 0; e < ne; ++e) {
+    long long hh[2][kFxVecs], cr[2][kFxVecs];
+    unsigned se[2][kFxVecs];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int v = 0; v < kFxVecs; ++v) {
+        hh[r][v] = cr[r][v] = 0;
+        se[r][v] = 0;
+      }
+#pragma unroll 1
+    for (int b = 0; b < 3; ++b)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const int2* p = A.part + (long)((e * 9 + b * 3 + c) * 4 + r0) * N + m;
+        const int2 p0 = p[0], p1 = p[N];
+        // the leads' sum over the cell and its four face neighbours: a lower bound
+        const bool face = c == 1 || b == 1;
+        const unsigned l0 = (unsigned)abs(p0.x) >> 17, l1 = (unsigned)abs(p1.x) >> 17;
+        const int2* xq = x0 + e * kFxHalo + sg * (c - 1) + sg * (b - 1) * kFxHx;
+#pragma unroll
+        for (int v = 0; v < kFxVecs; ++v) {
+          const int2 x = xq[v * 4 * kFxHalo];
+          hh[0][v] += (long long)p0.x * x.x;
+          hh[1][v] += (long long)p1.x * x.x;
+          cr[0][v] += (long long)p0.x * x.y;
+          cr[1][v] += (long long)p1.x * x.y;
+          cr[0][v] += (long long)p0.y * x.x;
+          cr[1][v] += (long long)p1.y * x.x;
+          if (face) {
+            const unsigned lx = (unsigned)abs(x.x) >> 17;
+            se[0][v] += l0 * lx;
+            se[1][v] += l1 * lx;
+          }
+        }
+      }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int ea = A.ex[((r0 + r) * 4 + e) * N + m];
+#pragma unroll
+      for (int v = 0; v < kFxVecs; ++v) {
+        const long long W = hh[r][v] + ((cr[r][v] + (1ll << (kFxLow - 1))) >> kFxLow);
+        const int sh = top[r][v] - ea - fx_exponent(smax[v * 4 + e]) + 1;  // >= 1 where W != 0
+        if (W != 0 && sh < 63) T[r][v] += (W + (1ll << (sh - 1))) >> sh;
+        if (se[r][v] && sh <= 32) S[r][v] += se[r][v] >> (sh - 1);
+      }
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < kFxVecs; ++v) {
+    if (v >= nv) continue;
+    bool bad = false;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) bad |= fx_exponent(smax[v * 4 + e]) == kFxBad;
+    const double sc = a.vscale ? a.vscale[v0 + v] : a.scale;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      double y = 0.0;
+      bool ok = !bad && !f64[r];
+      if (ok && top[r][v] != -0x7fffffff) {
+        y = fx_to_double(T[r][v], top[r][v] - kFxBits + 1, ok);
+        ok = ok && S[r][v] >= kFxLeast;
+      }
+      if (!ok) y = fx_row_f64(a, a.X + (long)(v0 + v) * a.ld, m, i, j, r0 + r);
+      a.Y[(long)(v0 + v) * a.ld + (r0 + r) * N + m] = sc == 1.0 ? y : sc * y;
     }
   }
 }
@@ -1534,8 +1748,26 @@ void launch_k_matvec(const DevCtx& d, int k, const MvArgs& a, int grid, int th, 
   else k_matvec<false, false><<<grid, th, 0, st>>>(a);
 }
 
+// Batches that take the fixed-point matvec: those where even the first one after a write of the
+// blocks, which makes their parts (~0.35 ns a cell and their storage, against ~66 ps saved per
+// cell and vector), is no slower than in FP64. Repeated, smaller ones would gain too (300 x 200,
+// 16 vectors: 173 -> 125 us), but their first took 75 us longer.
+static bool fx_takes(const DevCtx& d, int k) {
+  return k >= 8 && (long)(k - 6) * d.N >= 1000000 && !mv_one(d.N, k, d.sms);
+}
+
+// the integer parts of the blocks for one direction, made again after each write of the blocks
+static void launch_fx_build(DevCtx& d, int transpose, cudaStream_t st) {
+  if (d.fx_version[transpose] == d.coef_version) return;
+  (transpose ? k_fx_build<true> : k_fx_build<false>)<<<grid_for(16 * d.N, 256), 256, 0, st>>>(
+      d.coef, d.fx_part[transpose], d.fx_ex[transpose], make_wrap(d.cfg), d.N);
+  d.fx_version[transpose] = d.coef_version;
+}
+
+// fx: the fixed-point parts are current for this direction (the entry points that may allocate
+// make them: fx_ready)
 void launch_matvec(const DevCtx& d, int k, const double* X, double* Y, int transpose, double scale,
-                   cudaStream_t st, long ld) {
+                   cudaStream_t st, long ld, bool fx) {
   if (ld <= 0) ld = op_size(d);
   MvArgs a;
   a.acc_prev = nullptr;
@@ -1555,7 +1787,13 @@ void launch_matvec(const DevCtx& d, int k, const double* X, double* Y, int trans
   a.transpose = transpose;
   const long items = mv_items(d.N, k, d.sms);
   const int th = mv_threads(items, d.sms);
-  launch_k_matvec(d, k, a, grid_for(items, th), th, st);
+  if (fx && fx_takes(d, k)) {
+    FxArgs f{d.fx_part[transpose != 0], d.fx_ex[transpose != 0], a};
+    const long tiles = (long)((d.nchi + 31) / 32) * ((d.neta + kFxRows - 1) / kFxRows);
+    k_matvec_fx<<<(unsigned)(tiles * ((k + kFxVecs - 1) / kFxVecs)), 256, 0, st>>>(f);
+  } else {
+    launch_k_matvec(d, k, a, grid_for(items, th), th, st);
+  }
   if (d.sj.on) launch_shock_mv(d, k, X, Y, transpose, scale, st, ld);
 }
 
@@ -2469,11 +2707,34 @@ int hymor_jacobian_set(hymor_ctx* ctx, const double* coef) {
   return cuda_check(ctx, cudaStreamSynchronize(st));
 }
 
+// Whether the fixed-point matvec takes k vectors, with its parts made (their storage on first
+// use; without the memory for it the FP64 matvec serves).
+static bool fx_ready(hymor_ctx* ctx, int k, int transpose) {
+  DevCtx& d = ctx_dev(ctx);
+  const int t = transpose != 0;
+  if (!fx_takes(d, k)) return false;
+  if (!d.fx_part[t]) {
+    void *p = nullptr, *e = nullptr;
+    if (cudaMalloc(&p, sizeof(int2) * 144 * d.N) != cudaSuccess || cudaMalloc(&e, sizeof(short) * 16 * d.N) != cudaSuccess) {
+      if (p) cudaFree(p);
+      cudaGetLastError();
+      return false;
+    }
+    ctx_allocs(ctx).push_back(p);
+    ctx_allocs(ctx).push_back(e);
+    d.fx_part[t] = static_cast<int2*>(p);
+    d.fx_ex[t] = static_cast<short*>(e);
+    d.fx_version[t] = d.coef_version - 1;
+  }
+  launch_fx_build(d, t, ctx_stream(ctx));
+  return true;
+}
+
 int hymor_matvec_dev(hymor_ctx* ctx, int k, const double* dX, double* dY, int transpose) {
   if (!ctx || k < 1 || !dX || !dY) return HYMOR_ERR_INVALID;
   DevCtx& d = ctx_dev(ctx);
   if (!d.coef) return ctx_fail(ctx, HYMOR_ERR_NOT_READY, "no Jacobian: call hymor_linearize or hymor_jacobian_set");
-  launch_matvec(d, k, dX, dY, transpose, 1.0, ctx_stream(ctx));
+  launch_matvec(d, k, dX, dY, transpose, 1.0, ctx_stream(ctx), 0, fx_ready(ctx, k, transpose));
   return cuda_check(ctx, cudaGetLastError());
 }
 
@@ -2488,7 +2749,7 @@ int hymor_matvec(hymor_ctx* ctx, int k, const double* X, double* Y, int transpos
   if ((r = cuda_check(ctx, cudaMallocAsync((void**)&dx, bytes, st)))) return r;
   if ((r = cuda_check(ctx, cudaMallocAsync((void**)&dy, bytes, st)))) return r;
   cudaMemcpyAsync(dx, X, bytes, cudaMemcpyHostToDevice, st);
-  launch_matvec(d, k, dx, dy, transpose, 1.0, st);
+  launch_matvec(d, k, dx, dy, transpose, 1.0, st, 0, fx_ready(ctx, k, transpose));
   cudaMemcpyAsync(Y, dy, bytes, cudaMemcpyDeviceToHost, st);
   cudaFreeAsync(dx, st);
   cudaFreeAsync(dy, st);
@@ -2510,12 +2771,13 @@ int hymor_bench_matvec(hymor_ctx* ctx, int k, const double* dX, double* dY, int 
     return r;
   }
   const long n4 = op_size(d);
+  const bool fx = !per_vector && fx_ready(ctx, k, transpose);
   cudaEventRecord(e0, st);
   for (int rep = 0; rep < reps; ++rep) {
     if (per_vector) {
       for (int v = 0; v < k; ++v) launch_matvec(d, 1, dX + v * n4, dY + v * n4, transpose, 1.0, st);
     } else {
-      launch_matvec(d, k, dX, dY, transpose, 1.0, st);
+      launch_matvec(d, k, dX, dY, transpose, 1.0, st, 0, fx);
     }
   }
   cudaEventRecord(e1, st);

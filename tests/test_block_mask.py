@@ -39,8 +39,10 @@ def _operator(nchi, neta, seed=1):
     return cs, sol, L, co
 
 
-def test_batched_matvec(require_gpu):
-    nchi, neta, k = 83, 59, 41            # past the thread-per-output path, an odd last chunk
+@pytest.mark.parametrize("nchi,neta", [(83, 59), (230, 131)])
+def test_batched_matvec(require_gpu, nchi, neta):
+    """Past the thread-per-output path with an odd last chunk: in FP64, and in fixed point."""
+    k = 41
     cs, sol, L, co = _operator(nchi, neta)
     orc = O.Oracle(cs)
     X = np.random.Generator(np.random.PCG64(2)).standard_normal((L.n, k))
@@ -54,7 +56,7 @@ def test_batched_matvec(require_gpu):
             one = A @ np.ascontiguousarray(X[:, vec])
             assert np.array_equal(np.isnan(Y[:, vec]), np.isnan(one)) and np.isnan(one).any()
             ok = np.isfinite(one)
-            assert np.array_equal(Y[ok, vec], one[ok])
+            assert rel_err(Y[ok, vec], one[ok]) < 1e-14
         for vec in (1, 39):
             ref = orc.matvec(co, X[:, vec], transpose=A is not L)
             assert rel_err(Y[:, vec], ref) < 1e-13
