@@ -645,13 +645,30 @@ __device__ __forceinline__ void matvec_cells(const MvArgs& a) {
 template <bool ONE, bool ST>
 __global__ void __launch_bounds__(kMvThreads) k_matvec(MvArgs a) { matvec_cells<ONE, ST>(a); }
 
+// The Taylor coefficients 1 / j! of a propagation, formed on the host: a warp's
+// FP64 division takes the sub-partition's FP64 pipe for ~800 cycles, and in every warp once per
+// matvec it cost a small grid's matvec ~0.3 us (100 x 80, one vector: 523 -> 487 us for 250).
+constexpr int kMaxOrder = 20;
+struct Taylor {
+  double c[kMaxOrder + 1];
+};
+Taylor taylor_coefficients(int order) {
+  Taylor t{};
+  long fact = 1;
+  for (int j = 1; j <= order && j <= kMaxOrder; ++j) {
+    fact *= j;
+    t.c[j] = 1.0 / (double)fact;
+  }
+  return t;
+}
+
 // The whole Taylor propagation in one cooperative launch: the blocks are co-resident
 // (cudaLaunchCooperativeKernel) and meet at a grid barrier after every matvec, instead of
 // one kernel per matvec. Same per-cell arithmetic, in the same order, as launch_expm.
 // vsteps (k entries, non-increasing, or null): vector c takes vsteps[c] steps, so that at
 // step s only the first #{c : vsteps[c] > s} vectors advance (a contiguous prefix).
 template <bool ONE, bool ST>
-__global__ void __launch_bounds__(kMvThreads, 2) k_expm_coop(MvArgs base, int nsteps, int order, double* v,
+__global__ void __launch_bounds__(kMvThreads, 2) k_expm_coop(MvArgs base, Taylor tc, int nsteps, int order, double* v,
                                                              double* t1, double* t2, double* vout,
                                                              const int* vsteps) {
   cg::grid_group grid = cg::this_grid();
@@ -669,16 +686,14 @@ __global__ void __launch_bounds__(kMvThreads, 2) k_expm_coop(MvArgs base, int ns
     const double* src = late ? vout : v;
     const double* prev = nullptr;
     double c_prev = 0;
-    long fact = 1;
     for (int j = 1; j <= order; ++j) {
-      fact *= j;
       MvArgs a = base;
       a.X = src;
       a.Y = (j % 2) ? t1 : t2;
       a.acc = (late && j == 1) ? nullptr : vout;
       a.acc_prev = prev;
       a.c_prev = c_prev;
-      a.c_acc = 1.0 / (double)fact;
+      a.c_acc = tc.c[j];
       matvec_cells<ONE, ST>(a);
       grid.sync();
       src = a.Y;
@@ -950,7 +965,7 @@ __device__ __forceinline__ void matvec_tile_ff(const MvFf& a, float2* xs) {
 // into the FP64 output after the last step. MODE 0: matvec_tile_ff (a batch), 1: matvec_one_ff
 // (few cells x vectors: ff_one), 2: matvec_cell_ff (one vector).
 template <int MODE, bool ST>
-__global__ void __launch_bounds__(MODE == 0 ? kFfThreads : kMvThreads, MODE == 0 ? 4 : (MODE == 2 ? 3 : 2)) k_expm_coop_ff(MvFf base, int nsteps, int order, const double* xin,
+__global__ void __launch_bounds__(MODE == 0 ? kFfThreads : kMvThreads, MODE == 0 ? 4 : (MODE == 2 ? 3 : 2)) k_expm_coop_ff(MvFf base, Taylor tc, int nsteps, int order, const double* xin,
                                                                 double* yout, float2* t1, float2* t2, float2* vout,
                                                                 const int* vsteps) {
   extern __shared__ float2 ff_tile[];
@@ -969,16 +984,14 @@ __global__ void __launch_bounds__(MODE == 0 ? kFfThreads : kMvThreads, MODE == 0
     const float2* src = vout;
     const float2* prev = nullptr;
     ff c_prev{0.0f, 0.0f};
-    long fact = 1;
     for (int j = 1; j <= order; ++j) {
-      fact *= j;
       MvFf a = base;
       a.X = src;
       a.Y = (j % 2) ? t1 : t2;
       a.acc = j == 1 ? nullptr : vout;
       a.acc_prev = prev;
       a.c_prev = c_prev;
-      a.c_acc = ff_from_double(1.0 / (double)fact);
+      a.c_acc = ff_from_double(tc.c[j]);
       if (MODE == 1) matvec_one_ff<ST>(a);
       else if (MODE == 2) matvec_cell_ff<ST>(a);
       else matvec_tile_ff<kVecChunk, ST>(a, ff_tile);
@@ -990,6 +1003,207 @@ __global__ void __launch_bounds__(MODE == 0 ? kFfThreads : kMvThreads, MODE == 0
   }
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < nall; q += (long)gridDim.x * blockDim.x)
     yout[q] = ff_to_double(ldff(vout, q));
+}
+
+// ---------------------------------------------------------------------------
+// The float-float propagation of a small grid, resident on chip: a block owns a tile of cells for
+// the whole propagation, with the tile's blocks, the terms and the running sums in shared memory
+// (one thread per cell and component); from one matvec to the next only the ring of halo values
+// goes through global memory, and a block waits for its neighbours' terms only, not for the
+// grid. The same pairs as k_expm_coop_ff.
+//
+// What bounds it: the latency of a term, i.e. 36 float-float products in a chain of nine blocks,
+// the write of the term, the flag, and the neighbours' read of it. With a thread per output, the
+// blocks from L2 and a grid barrier (1.15 us by itself) per matvec, 100 x 80 took 5.6 us per
+// matvec alone and 3.4 with three contexts at once; so it takes 4.9 and 2.0 (100 x 80, 4 vectors:
+// 11.3 -> 6.7 with three at once; 60 x 40, 12 vectors: 11.3 -> 8.4; 160 x 120: 6.9 -> 5.6).
+//
+// Terms are published in sequence, into two buffers in turn: a block writes term s + 2 over term
+// s only after its neighbours have published term s + 1, for which they have read term s. The
+// waits are bounded (kResPolls): a block that gives up sets kBitTimeout and stops, and so do its
+// neighbours in turn; the blocks are co-resident (a cooperative launch).
+constexpr int kResPolls = 1 << 20;
+constexpr int kResFlag = 8;  // flags are 32 bytes apart
+
+struct ResTile {
+  int tw, th, tx, ty;  // tile size in cells, tiles
+  unsigned* flag;      // tx ty flags: the number of terms published
+  unsigned* err;
+};
+
+long res_smem(const ResTile& t, int k) {
+  const long items = 4L * t.tw * t.th, halo = (long)(t.tw + 2) * (t.th + 2);
+  return (long)sizeof(float2) * (36 * items + 8L * k * halo + 2L * k * items);
+}
+// the tiling of at most `blocks` tiles with the fewest cells per tile (then the smallest halo)
+ResTile res_tiling(const Wrap& w, int blocks) {
+  ResTile best{0, 0, 0, 0, nullptr, nullptr};
+  for (int tw = 4; tw <= 64; ++tw) {
+    const int tx = (w.nchi + tw - 1) / tw;
+    if (tx > blocks) continue;
+    const int rows = blocks / tx, th = std::max(2, (w.neta + rows - 1) / rows), ty = (w.neta + th - 1) / th;
+    const long c = (long)tw * th, b = (long)best.tw * best.th;
+    if (!best.tw || c < b || (c == b && tw + th < best.tw + best.th)) best = ResTile{tw, th, tx, ty, nullptr, nullptr};
+  }
+  return best;
+}
+
+__global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor tc, int nsteps, int order, const double* xin,
+                                                      double* yout, float2* g0, float2* g1, const int* vsteps) {
+  extern __shared__ float2 ff_tile[];
+  const long N = a.N;
+  const int nchi = a.w.nchi, neta = a.w.neta;
+  const int cells = rt.tw * rt.th, items = 4 * cells, hw = rt.tw + 2, halo = hw * (rt.th + 2);
+  const int kall = a.k;
+  float2* const cA = ff_tile;                                   // (36, items)
+  float2* const xs = cA + 36 * items;                           // (2, k, 4, halo)
+  float2* const sum = xs + (long)8 * kall * halo;               // (k, items)
+  float2* const old = sum + (long)kall * items;                 // (k, items): the first term, added late
+  const int tile = blockIdx.x, tX = tile % rt.tx, tY = tile / rt.tx;
+  const int i0 = tX * rt.tw, j0 = tY * rt.th, w = min(rt.tw, nchi - i0), hgt = min(rt.th, neta - j0);
+  const int t = threadIdx.x, nt = blockDim.x;
+  const int comp = t / cells, cell = t - comp * cells, ly = cell / rt.tw, lx = cell - ly * rt.tw;
+  const int i = i0 + lx, j = j0 + ly;
+  const long m = i + (long)j * nchi;
+  const bool in = t < items && lx < w && ly < hgt;
+  const bool edge = in && (lx == 0 || ly == 0 || lx == w - 1 || ly == hgt - 1);
+  const int sg = a.transpose ? -1 : 1;
+  unsigned ok = 0;  // bit q: the neighbour exists
+  if (in) {
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+      const long n = a.w.nbr(i, j, sg * (q % 3 - 1), sg * (q / 3 - 1));
+      if (n < 0) continue;
+      ok |= 1u << q;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        // row comp of the block (columns e), or column comp of it for the transpose
+        const int plane = a.transpose ? q * 16 + e * 4 + comp : q * 16 + comp * 4 + e;
+        cA[(q * 4 + e) * items + t] = a.coef[(long)plane * N + (a.transpose ? n : m)];
+      }
+    }
+  }
+  const int own = comp * halo + (lx + 1) + (ly + 1) * hw;
+  // the neighbouring tiles: lanes 0 .. 8 of the first warp
+  int nb = -1;
+  if (t < 9 && t != 4) {
+    int bx = tX + t % 3 - 1, by = tY + t / 3 - 1;
+    if (a.w.per_chi) bx = bx < 0 ? rt.tx - 1 : (bx >= rt.tx ? 0 : bx);
+    if (a.w.per_eta) by = by < 0 ? rt.ty - 1 : (by >= rt.ty ? 0 : by);
+    if (bx >= 0 && bx < rt.tx && by >= 0 && by < rt.ty && bx + by * rt.tx != tile) nb = bx + by * rt.tx;
+  }
+  unsigned seq = 0;  // terms published
+  // the edge values of the term just written to buffer seq & 1 are on their way: publish it, wait
+  // for the neighbours' and fetch the ring; false when a wait gave up
+  auto exchange = [&](int ka) -> bool {
+    __syncthreads();
+    const int pb = seq & 1;
+    ++seq;
+    bool good = true;
+    if (t == 0) {
+      __threadfence();
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(rt.flag + (long)tile * kResFlag), "r"(seq) : "memory");
+    }
+    if (nb >= 0) {
+      good = false;
+      for (int p = 0; p < kResPolls && !good; ++p) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(rt.flag + (long)nb * kResFlag) : "memory");
+        good = v >= seq;
+      }
+    }
+    if (!__syncthreads_and(good)) {
+      if (t == 0) atomicOr(rt.err, kBitTimeout);
+      return false;
+    }
+    const float2* g = pb ? g1 : g0;
+    float2* x = xs + (long)pb * kall * 4 * halo;
+    const int ring = 2 * (w + 2) + 2 * hgt;
+    for (int r = t; r < ring * 4; r += nt) {
+      const int e = r / ring, c = r - e * ring;
+      int hx, hy;
+      if (c < 2 * (w + 2)) {
+        hy = c < w + 2 ? 0 : hgt + 1;
+        hx = c < w + 2 ? c : c - (w + 2);
+      } else {
+        const int c2 = c - 2 * (w + 2);
+        hy = 1 + (c2 >> 1);
+        hx = c2 & 1 ? w + 1 : 0;
+      }
+      int ii = i0 - 1 + hx, jj = j0 - 1 + hy;
+      if (a.w.per_chi) ii = ii < 0 ? ii + nchi : (ii >= nchi ? ii - nchi : ii);
+      if (a.w.per_eta) jj = jj < 0 ? jj + neta : (jj >= neta ? jj - neta : jj);
+      if (ii < 0 || ii >= nchi || jj < 0 || jj >= neta) continue;
+      for (int v = 0; v < ka; ++v)
+        x[(v * 4 + e) * halo + hx + hy * hw] = __ldcg(g + v * a.ld + e * N + ii + (long)jj * nchi);
+    }
+    __syncthreads();
+    return true;
+  };
+  // a value of the next term: into the tile's shared copy and, on the tile's edge, the buffer
+  auto put = [&](int v, ff val) {
+    const int pb = seq & 1;
+    xs[((long)pb * kall + v) * 4 * halo + own] = make_float2(val.h, val.l);
+    if (edge) stff(pb ? g1 : g0, v * a.ld + comp * N + m, val);
+  };
+  if (in)
+    for (int v = 0; v < kall; ++v) {
+      const ff x = ff_from_double_checked(xin[v * a.ld + comp * N + m]);
+      stff(sum, v * items + t, x);
+      put(v, x);
+    }
+  // (a propagation that gave up leaves NaN beside its error bit)
+  auto fail = [&]() {
+    if (in)
+      for (int v = 0; v < kall; ++v) yout[v * a.ld + comp * N + m] = __longlong_as_double(0x7ff8000000000000LL);
+  };
+  if (!exchange(kall)) return fail();
+  int ka = kall;
+  for (int s = 0; s < nsteps; ++s) {
+    if (vsteps) {
+      ka = 0;
+      while (ka < kall && vsteps[ka] > s) ++ka;
+    }
+    ff c1{0.0f, 0.0f};
+    for (int jt = 1; jt <= order; ++jt) {
+      const ff c = ff_from_double(tc.c[jt]);
+      const bool last = jt == order;
+      if (in)
+        for (int v = 0; v < ka; ++v) {
+          const float2* x = xs + ((long)((seq - 1) & 1) * kall + v) * 4 * halo + (lx + 1) + (ly + 1) * hw;
+          ff y{0.0f, 0.0f};
+#pragma unroll
+          for (int q = 0; q < 9; ++q) {
+            if (!(ok >> q & 1)) continue;
+            const float2* xq = x + sg * (q % 3 - 1) + sg * (q / 3 - 1) * hw;
+            ff B[4], X[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              B[e] = ldff(cA, (q * 4 + e) * items + t);
+              X[e] = ldff(xq, e * halo);
+            }
+            y = ff_dot4(B, X, y);
+          }
+          // mvff_out's term and running sum
+          const ff val = ff_mul(ff_from_double(a.vscale ? a.vscale[v] : a.scale), y);
+          if (jt == 1) {
+            stff(old, v * items + t, val);
+          } else {
+            ff r = ldff(sum, v * items + t);
+            if (jt == 2) r = ff_add(r, ff_mul(ldff(old, v * items + t), c1));
+            r = ff_add(r, ff_mul(val, c));
+            stff(sum, v * items + t, r);
+            if (last) put(v, r);
+          }
+          if (!last) put(v, val);
+        }
+      c1 = c;
+      if (last && s + 1 == nsteps) break;
+      if (!exchange(ka)) return fail();
+    }
+  }
+  if (in)
+    for (int v = 0; v < kall; ++v) yout[v * a.ld + comp * N + m] = ff_to_double(ldff(sum, v * items + t));
 }
 
 __global__ void k_coef_to_ff(const double* __restrict__ c, float2* __restrict__ f, long n) {
@@ -2369,6 +2583,7 @@ struct KrylovScratch {
 struct LinearState {
   ExpmCache expm;
   KrylovScratch kry;
+  bool res_ready = false;  // k_expm_res_ff's shared memory is set
   int coop_blocks[10] = {};  // co-resident blocks per SM of k_expm_coop<false>, <true>,
                              // k_expm_coop_ff<0>, <1>, <2>, each with ordinary and
                              // streaming block loads
@@ -2441,6 +2656,7 @@ int ensure_lanes(hymor_ctx* ctx, JacLanes** out) {
 // with 4 vectors 1.72 / 2.81, 8 vectors 3.06 / 3.09, 16 vectors 5.10 / 3.79, of 200 x 100 with 2
 // vectors 2.41 / 2.08, of 300 x 200 with 2 vectors 8.29 / 3.26.
 constexpr long kFfOneCells = 40000;
+constexpr long kResSmem = 220 * 1024;  // shared memory of the resident propagation
 bool ff_one(long N, int k) { return N * k < kFfOneCells; }
 
 // hdts, hsteps (host, k entries, hsteps non-increasing), or null: vector c is propagated
@@ -2452,15 +2668,16 @@ int expm_cooperative(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
   ExpmCache& c = expm_cache(ctx);
   const long n = 4 * d.N * (long)k;
   int r;
-  if (4 * n + 2 * k > c.cap) {
+  const long flags = (long)kResFlag / 2 * d.sms;  // doubles: the resident propagation's flags
+  if (4 * n + 2 * k + flags > c.cap) {
     if ((r = cuda_check(ctx, cudaStreamSynchronize(st)))) return r;
     if (c.buf) cudaFree(c.buf);
     c.buf = nullptr;
     c.cap = 0;
     void* p = nullptr;
-    if ((r = cuda_check(ctx, cudaMalloc(&p, sizeof(double) * (4 * n + 2 * k))))) return r;
+    if ((r = cuda_check(ctx, cudaMalloc(&p, sizeof(double) * (4 * n + 2 * k + flags))))) return r;
     c.buf = static_cast<double*>(p);
-    c.cap = 4 * n + 2 * k;
+    c.cap = 4 * n + 2 * k + flags;
   }
   double* v = c.buf;
   double* t1 = c.buf + n;
@@ -2527,6 +2744,7 @@ int expm_cooperative(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
     base.vscale = vscale;
     nsteps = hsteps[0];
   }
+  Taylor tc = taylor_coefficients(order);
   if (ffp) {
     MvFf bf;
     bf.coef = d.coef_ff;
@@ -2548,13 +2766,27 @@ int expm_cooperative(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
     float2* f1 = reinterpret_cast<float2*>(t1);
     float2* f2 = reinterpret_cast<float2*>(t2);
     float2* fo = reinterpret_cast<float2*>(vout);
-    void* fargs[] = {&bf, &nsteps, &order, &dX, &dY, &f1, &f2, &fo, &vsteps};
+    ResTile rt = ffmode == 1 ? res_tiling(base.w, d.sms) : ResTile{};
+    if (ffmode == 1 && 4 * rt.tw * rt.th <= 1024 && res_smem(rt, k) <= kResSmem) {
+      bool& ready = linear_state(ctx).res_ready;
+      if (!ready && (r = cuda_check(ctx, cudaFuncSetAttribute(k_expm_res_ff, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                              (int)kResSmem))))
+        return r;
+      ready = true;
+      rt.flag = reinterpret_cast<unsigned*>(c.buf + 4 * n + 2 * k);
+      rt.err = d.err;
+      if ((r = cuda_check(ctx, cudaMemsetAsync(rt.flag, 0, sizeof(double) * flags, st)))) return r;
+      void* rargs[] = {&bf, &rt, &tc, &nsteps, &order, &dX, &dY, &f1, &f2, &vsteps};
+      return cuda_check(ctx, cudaLaunchCooperativeKernel((const void*)k_expm_res_ff, rt.tx * rt.ty,
+                                                         (4 * rt.tw * rt.th + 31) / 32 * 32, rargs, res_smem(rt, k), st));
+    }
+    void* fargs[] = {&bf, &tc, &nsteps, &order, &dX, &dY, &f1, &f2, &fo, &vsteps};
     return cuda_check(ctx, cudaLaunchCooperativeKernel(kern, grid, th, fargs,
                                                        kind == 2 ? ff_tile_smem<kVecChunk>() : 0, st));
   }
   if ((r = cuda_check(ctx, cudaMemcpyAsync(v, dX, sizeof(double) * n, cudaMemcpyDeviceToDevice, st)))) return r;
   if ((r = cuda_check(ctx, cudaMemcpyAsync(vout, dX, sizeof(double) * n, cudaMemcpyDeviceToDevice, st)))) return r;
-  void* args[] = {&base, &nsteps, &order, &v, &t1, &t2, &vout, &vsteps};
+  void* args[] = {&base, &tc, &nsteps, &order, &v, &t1, &t2, &vout, &vsteps};
   if ((r = cuda_check(ctx, cudaLaunchCooperativeKernel(kern, grid, th, args, 0, st))))
     return r;
   return cuda_check(ctx, cudaMemcpyAsync(dY, vout, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
