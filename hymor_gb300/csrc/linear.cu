@@ -1012,22 +1012,28 @@ __global__ void __launch_bounds__(MODE == 0 ? kFfThreads : kMvThreads, MODE == 0
 // goes through global memory, and a block waits for its neighbours' terms only, not for the
 // grid. The same pairs as k_expm_coop_ff.
 //
-// What bounds it: the latency of a term, i.e. 36 float-float products in a chain of nine blocks,
-// the write of the term, the flag, and the neighbours' read of it. With a thread per output, the
-// blocks from L2 and a grid barrier (1.15 us by itself) per matvec, 100 x 80 took 5.6 us per
-// matvec alone and 3.4 with three contexts at once; so it takes 4.9 and 2.0 (100 x 80, 4 vectors:
-// 11.3 -> 6.7 with three at once; 60 x 40, 12 vectors: 11.3 -> 8.4; 160 x 120: 6.9 -> 5.6).
+// The values of a tile's edge are published with their term's number beside each half, {h, s, l,
+// s} in 16 bytes, and a reader of the ring polls the value itself until both halves carry its
+// term's number: no flag, no fence, and one block barrier per matvec. Two buffers take the terms
+// in turn: a block writes term s + 2 over term s only after it has read term s + 1 of all its
+// neighbours, which they form after they have read term s. The waits are bounded (kResPolls): a
+// block that gives up sets kBitTimeout, leaves NaN and stops, and so do its neighbours in turn;
+// the blocks are co-resident (a cooperative launch).
 //
-// Terms are published in sequence, into two buffers in turn: a block writes term s + 2 over term
-// s only after its neighbours have published term s + 1, for which they have read term s. The
-// waits are bounded (kResPolls): a block that gives up sets kBitTimeout and stops, and so do its
-// neighbours in turn; the blocks are co-resident (a cooperative launch).
+// What bounds it: the latency of a term, i.e. 36 float-float products in a chain of nine blocks
+// (~3 instructions in four cycles with two warps per sub-partition), the write of a value and its
+// neighbours' read. 100 x 80, one vector, us per matvec alone and with three contexts at once: a
+// thread per output with the blocks from L2 and a grid barrier (1.15 us by itself) 5.6 and 3.4;
+// resident with a flag per tile behind a fence 4.9 and 2.0; so 3.8 and 1.5. Several vectors are
+// shared by groups of threads, so that neither their chains nor their polls follow one another in
+// one thread: 60 x 40, twelve vectors, us for the propagation 1660 with the blocks from L2, 1500
+// in one group, 762 so.
 constexpr int kResPolls = 1 << 20;
-constexpr int kResFlag = 8;  // flags are 32 bytes apart
+constexpr int kResThreads = 512;  // of a block with several groups: two blocks' registers per SM
 
 struct ResTile {
   int tw, th, tx, ty;  // tile size in cells, tiles
-  unsigned* flag;      // tx ty flags: the number of terms published
+  int groups;          // of threads, a thread per cell and component each, that share the vectors
   unsigned* err;
 };
 
@@ -1036,20 +1042,21 @@ long res_smem(const ResTile& t, int k) {
   return (long)sizeof(float2) * (36 * items + 8L * k * halo + 2L * k * items);
 }
 // the tiling of at most `blocks` tiles with the fewest cells per tile (then the smallest halo)
-ResTile res_tiling(const Wrap& w, int blocks) {
-  ResTile best{0, 0, 0, 0, nullptr, nullptr};
+ResTile res_tiling(const Wrap& w, int blocks, int k) {
+  ResTile best{0, 0, 0, 0, 1, nullptr};
   for (int tw = 4; tw <= 64; ++tw) {
     const int tx = (w.nchi + tw - 1) / tw;
     if (tx > blocks) continue;
     const int rows = blocks / tx, th = std::max(2, (w.neta + rows - 1) / rows), ty = (w.neta + th - 1) / th;
     const long c = (long)tw * th, b = (long)best.tw * best.th;
-    if (!best.tw || c < b || (c == b && tw + th < best.tw + best.th)) best = ResTile{tw, th, tx, ty, nullptr, nullptr};
+    if (!best.tw || c < b || (c == b && tw + th < best.tw + best.th)) best = ResTile{tw, th, tx, ty, 1, nullptr};
   }
+  best.groups = std::max(1, std::min(k, kResThreads / (4 * best.tw * best.th)));
   return best;
 }
 
 __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor tc, int nsteps, int order, const double* xin,
-                                                      double* yout, float2* g0, float2* g1, const int* vsteps) {
+                                                      double* yout, uint4* g0, uint4* g1, const int* vsteps) {
   extern __shared__ float2 ff_tile[];
   const long N = a.N;
   const int nchi = a.w.nchi, neta = a.w.neta;
@@ -1061,11 +1068,11 @@ __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor
   float2* const old = sum + (long)kall * items;                 // (k, items): the first term, added late
   const int tile = blockIdx.x, tX = tile % rt.tx, tY = tile / rt.tx;
   const int i0 = tX * rt.tw, j0 = tY * rt.th, w = min(rt.tw, nchi - i0), hgt = min(rt.th, neta - j0);
-  const int t = threadIdx.x, nt = blockDim.x;
+  const int tid = threadIdx.x, nt = blockDim.x, vg = tid / items, t = tid - vg * items;  // vectors vg, vg + groups, ...
   const int comp = t / cells, cell = t - comp * cells, ly = cell / rt.tw, lx = cell - ly * rt.tw;
   const int i = i0 + lx, j = j0 + ly;
   const long m = i + (long)j * nchi;
-  const bool in = t < items && lx < w && ly < hgt;
+  const bool in = vg < rt.groups && lx < w && ly < hgt;
   const bool edge = in && (lx == 0 || ly == 0 || lx == w - 1 || ly == hgt - 1);
   const int sg = a.transpose ? -1 : 1;
   unsigned ok = 0;  // bit q: the neighbour exists
@@ -1075,6 +1082,7 @@ __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor
       const long n = a.w.nbr(i, j, sg * (q % 3 - 1), sg * (q / 3 - 1));
       if (n < 0) continue;
       ok |= 1u << q;
+      if (vg > 0) continue;  // the first group brings the blocks for all
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         // row comp of the block (columns e), or column comp of it for the transpose
@@ -1084,43 +1092,15 @@ __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor
     }
   }
   const int own = comp * halo + (lx + 1) + (ly + 1) * hw;
-  // the neighbouring tiles: lanes 0 .. 8 of the first warp
-  int nb = -1;
-  if (t < 9 && t != 4) {
-    int bx = tX + t % 3 - 1, by = tY + t / 3 - 1;
-    if (a.w.per_chi) bx = bx < 0 ? rt.tx - 1 : (bx >= rt.tx ? 0 : bx);
-    if (a.w.per_eta) by = by < 0 ? rt.ty - 1 : (by >= rt.ty ? 0 : by);
-    if (bx >= 0 && bx < rt.tx && by >= 0 && by < rt.ty && bx + by * rt.tx != tile) nb = bx + by * rt.tx;
-  }
-  unsigned seq = 0;  // terms published
-  // the edge values of the term just written to buffer seq & 1 are on their way: publish it, wait
-  // for the neighbours' and fetch the ring; false when a wait gave up
+  unsigned seq = 1;  // the number of the term being formed; its buffer is seq & 1
+  // the ring of the term just published; false when a wait gave up
+  const int ring = 2 * (w + 2) + 2 * hgt;
   auto exchange = [&](int ka) -> bool {
-    __syncthreads();
-    const int pb = seq & 1;
-    ++seq;
+    const uint4* g = seq & 1 ? g1 : g0;
+    float2* x = xs + (long)(seq & 1) * kall * 4 * halo;
     bool good = true;
-    if (t == 0) {
-      __threadfence();
-      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(rt.flag + (long)tile * kResFlag), "r"(seq) : "memory");
-    }
-    if (nb >= 0) {
-      good = false;
-      for (int p = 0; p < kResPolls && !good; ++p) {
-        unsigned v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(rt.flag + (long)nb * kResFlag) : "memory");
-        good = v >= seq;
-      }
-    }
-    if (!__syncthreads_and(good)) {
-      if (t == 0) atomicOr(rt.err, kBitTimeout);
-      return false;
-    }
-    const float2* g = pb ? g1 : g0;
-    float2* x = xs + (long)pb * kall * 4 * halo;
-    const int ring = 2 * (w + 2) + 2 * hgt;
-    for (int r = t; r < ring * 4; r += nt) {
-      const int e = r / ring, c = r - e * ring;
+    for (int r = tid; r < ring * 4 * ka; r += nt) {  // the vectors spread over the threads too: a poll is a wait
+      const int ve = r / ring, v = ve >> 2, e = ve & 3, c = r - ve * ring;
       int hx, hy;
       if (c < 2 * (w + 2)) {
         hy = c < w + 2 ? 0 : hgt + 1;
@@ -1131,23 +1111,39 @@ __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor
         hx = c2 & 1 ? w + 1 : 0;
       }
       int ii = i0 - 1 + hx, jj = j0 - 1 + hy;
-      if (a.w.per_chi) ii = ii < 0 ? ii + nchi : (ii >= nchi ? ii - nchi : ii);
-      if (a.w.per_eta) jj = jj < 0 ? jj + neta : (jj >= neta ? jj - neta : jj);
-      if (ii < 0 || ii >= nchi || jj < 0 || jj >= neta) continue;
-      for (int v = 0; v < ka; ++v)
-        x[(v * 4 + e) * halo + hx + hy * hw] = __ldcg(g + v * a.ld + e * N + ii + (long)jj * nchi);
+      const bool wi = ii < 0 || ii >= nchi, wj = jj < 0 || jj >= neta;
+      if ((wi && !a.w.per_chi) || (wj && !a.w.per_eta) || (wi && wj)) continue;  // no such input (Wrap::nbr)
+      if (wi) ii = ii < 0 ? ii + nchi : ii - nchi;
+      if (wj) jj = jj < 0 ? jj + neta : jj - neta;
+      const uint4* p = g + v * a.ld + e * N + ii + (long)jj * nchi;
+      uint4 u;
+      int polls = 0;
+      do {
+        asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w)
+                     : "l"(p)
+                     : "memory");
+      } while ((u.y != seq || u.w != seq) && ++polls < kResPolls && good);
+      good = good && u.y == seq && u.w == seq;
+      x[((long)v * 4 + e) * halo + hx + hy * hw] = make_float2(__uint_as_float(u.x), __uint_as_float(u.z));
     }
-    __syncthreads();
+    if (!__syncthreads_and(good)) {
+      if (tid == 0) atomicOr(rt.err, kBitTimeout);
+      return false;
+    }
+    ++seq;
     return true;
   };
-  // a value of the next term: into the tile's shared copy and, on the tile's edge, the buffer
+  // a value of the term: into the tile's shared copy and, on the tile's edge, published
   auto put = [&](int v, ff val) {
-    const int pb = seq & 1;
-    xs[((long)pb * kall + v) * 4 * halo + own] = make_float2(val.h, val.l);
-    if (edge) stff(pb ? g1 : g0, v * a.ld + comp * N + m, val);
+    xs[((long)(seq & 1) * kall + v) * 4 * halo + own] = make_float2(val.h, val.l);
+    if (edge)
+      asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"((seq & 1 ? g1 : g0) + v * a.ld + comp * N + m),
+                   "r"(__float_as_uint(val.h)), "r"(seq), "r"(__float_as_uint(val.l)), "r"(seq)
+                   : "memory");
   };
   if (in)
-    for (int v = 0; v < kall; ++v) {
+    for (int v = vg; v < kall; v += rt.groups) {
       const ff x = ff_from_double_checked(xin[v * a.ld + comp * N + m]);
       stff(sum, v * items + t, x);
       put(v, x);
@@ -1155,7 +1151,7 @@ __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor
   // (a propagation that gave up leaves NaN beside its error bit)
   auto fail = [&]() {
     if (in)
-      for (int v = 0; v < kall; ++v) yout[v * a.ld + comp * N + m] = __longlong_as_double(0x7ff8000000000000LL);
+      for (int v = vg; v < kall; v += rt.groups) yout[v * a.ld + comp * N + m] = __longlong_as_double(0x7ff8000000000000LL);
   };
   if (!exchange(kall)) return fail();
   int ka = kall;
@@ -1169,7 +1165,7 @@ __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor
       const ff c = ff_from_double(tc.c[jt]);
       const bool last = jt == order;
       if (in)
-        for (int v = 0; v < ka; ++v) {
+        for (int v = vg; v < ka; v += rt.groups) {
           const float2* x = xs + ((long)((seq - 1) & 1) * kall + v) * 4 * halo + (lx + 1) + (ly + 1) * hw;
           ff y{0.0f, 0.0f};
 #pragma unroll
@@ -1203,7 +1199,7 @@ __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor
     }
   }
   if (in)
-    for (int v = 0; v < kall; ++v) yout[v * a.ld + comp * N + m] = ff_to_double(ldff(sum, v * items + t));
+    for (int v = vg; v < kall; v += rt.groups) yout[v * a.ld + comp * N + m] = ff_to_double(ldff(sum, v * items + t));
 }
 
 __global__ void k_coef_to_ff(const double* __restrict__ c, float2* __restrict__ f, long n) {
@@ -2668,16 +2664,15 @@ int expm_cooperative(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
   ExpmCache& c = expm_cache(ctx);
   const long n = 4 * d.N * (long)k;
   int r;
-  const long flags = (long)kResFlag / 2 * d.sms;  // doubles: the resident propagation's flags
-  if (4 * n + 2 * k + flags > c.cap) {
+  if (4 * n + 2 * k > c.cap) {
     if ((r = cuda_check(ctx, cudaStreamSynchronize(st)))) return r;
     if (c.buf) cudaFree(c.buf);
     c.buf = nullptr;
     c.cap = 0;
     void* p = nullptr;
-    if ((r = cuda_check(ctx, cudaMalloc(&p, sizeof(double) * (4 * n + 2 * k + flags))))) return r;
+    if ((r = cuda_check(ctx, cudaMalloc(&p, sizeof(double) * (4 * n + 2 * k))))) return r;
     c.buf = static_cast<double*>(p);
-    c.cap = 4 * n + 2 * k + flags;
+    c.cap = 4 * n + 2 * k;
   }
   double* v = c.buf;
   double* t1 = c.buf + n;
@@ -2766,19 +2761,21 @@ int expm_cooperative(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
     float2* f1 = reinterpret_cast<float2*>(t1);
     float2* f2 = reinterpret_cast<float2*>(t2);
     float2* fo = reinterpret_cast<float2*>(vout);
-    ResTile rt = ffmode == 1 ? res_tiling(base.w, d.sms) : ResTile{};
+    ResTile rt = ffmode == 1 ? res_tiling(base.w, d.sms, k) : ResTile{};
     if (ffmode == 1 && 4 * rt.tw * rt.th <= 1024 && res_smem(rt, k) <= kResSmem) {
       bool& ready = linear_state(ctx).res_ready;
       if (!ready && (r = cuda_check(ctx, cudaFuncSetAttribute(k_expm_res_ff, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                               (int)kResSmem))))
         return r;
       ready = true;
-      rt.flag = reinterpret_cast<unsigned*>(c.buf + 4 * n + 2 * k);
       rt.err = d.err;
-      if ((r = cuda_check(ctx, cudaMemsetAsync(rt.flag, 0, sizeof(double) * flags, st)))) return r;
-      void* rargs[] = {&bf, &rt, &tc, &nsteps, &order, &dX, &dY, &f1, &f2, &vsteps};
+      // two buffers of 16 bytes per value: the four vectors of the other paths (v .. vout); no
+      // term has number 0
+      if ((r = cuda_check(ctx, cudaMemsetAsync(v, 0, sizeof(double) * 4 * n, st)))) return r;
+      uint4 *g0 = reinterpret_cast<uint4*>(v), *g1 = reinterpret_cast<uint4*>(t2);
+      void* rargs[] = {&bf, &rt, &tc, &nsteps, &order, &dX, &dY, &g0, &g1, &vsteps};
       return cuda_check(ctx, cudaLaunchCooperativeKernel((const void*)k_expm_res_ff, rt.tx * rt.ty,
-                                                         (4 * rt.tw * rt.th + 31) / 32 * 32, rargs, res_smem(rt, k), st));
+                                                         (4 * rt.tw * rt.th * rt.groups + 31) / 32 * 32, rargs, res_smem(rt, k), st));
     }
     void* fargs[] = {&bf, &tc, &nsteps, &order, &dX, &dY, &f1, &f2, &fo, &vsteps};
     return cuda_check(ctx, cudaLaunchCooperativeKernel(kern, grid, th, fargs,
