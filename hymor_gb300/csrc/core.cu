@@ -400,7 +400,7 @@ __device__ void edge_bc_point(const hymor_config& c, const EdgeCtx& e, const Dev
 //   k_bc_edges       the two boundary phases (chi edges, then eta edges, whose corners
 //                    read the chi ghosts), one launch each, one thread per edge point
 // Spline workspace (units of n = Nchi doubles): 0 knots, 1-2 ordinates x/y, 3-4
-// second derivatives x/y, 5-6 fitted values x/y, 7-11 per-row d0 d1 d2 rhs_x rhs_y,
+// second derivatives x/y, 5-6 unused, 7-11 per-row d0 d1 d2 rhs_x rhs_y,
 // 12-14 FP64 Cholesky factors of the fallback solve, 15 interval reciprocals
 // 1/(x[k+1] - x[k]).
 
@@ -460,21 +460,21 @@ __global__ void __launch_bounds__(128) k_spline_rows(SplineArgs A) {
     pts.x[i] = A.pS.x[i]; pts.y[i] = A.pS.y[i];
     pts.chi[i] = A.pS.chi[i]; pts.eta[i] = A.pS.eta[i];
   }
-  if (i + 1 < n) ih[i] = 1.0 / (X(i + 1) - X(i));
+  if (i + 1 < n) ih[i] = exact_rcp(X(i + 1) - X(i));
   const int m = n - 2;
   const int jj = i;
   if (jj < m) {
     const int j = jj + 1;
     const double hm = X(j) - X(j - 1), h0 = X(j + 1) - X(j);
-    const double qm = 1.0 / hm, qp = 1.0 / h0, q0 = -qm - qp;
-    d0[jj] = (hm + h0) / 3 + lam * (qm * qm + q0 * q0 + qp * qp);
+    const double qm = exact_rcp(hm), qp = exact_rcp(h0), q0 = -qm - qp;
+    d0[jj] = exact_third(hm + h0) + lam * (qm * qm + q0 * q0 + qp * qp);
     double e1 = 0, e2 = 0;
     if (jj + 1 < m) {
       const double h1 = X(j + 2) - X(j + 1);
-      const double qm1 = 1.0 / h0, qp1 = 1.0 / h1, q01 = -qm1 - qp1;
-      e1 = h0 / 6 + lam * (q0 * qm1 + qp * q01);
+      const double qm1 = qp, qp1 = exact_rcp(h1), q01 = -qm1 - qp1;
+      e1 = 0.5 * exact_third(h0) + lam * (q0 * qm1 + qp * q01);
+      if (jj + 2 < m) e2 = lam * (qp * qp1);
     }
-    if (jj + 2 < m) e2 = lam * (qp * (1.0 / (X(j + 2) - X(j + 1))));
     d1[jj] = e1;
     d2[jj] = e2;
     rx[jj] = qm * src.x[j - 1] + q0 * src.x[j] + qp * src.x[j + 1];
@@ -712,8 +712,6 @@ __global__ void __launch_bounds__(kSplineThreads) k_spline_fit(SplineArgs A) {
   double* yy = yx + n;
   double* cx = yy + n;
   double* cy = cx + n;
-  double* gx = cy + n;
-  double* gy = gx + n;
   const double* d0 = ws + 7 * n;
   const double* d1 = d0 + n;
   const double* d2 = d1 + n;
@@ -735,18 +733,14 @@ __global__ void __launch_bounds__(kSplineThreads) k_spline_fit(SplineArgs A) {
   float* ey = ex + mp;
   const double lam = A.lam;
   for (int i = tid; i < n; i += nt) { cx[i] = 0; cy[i] = 0; }
-  if (m <= 0) {
-    __syncthreads();
-    for (int i = tid; i < n; i += nt) { gx[i] = yx[i]; gy[i] = yy[i]; }
-    return;
-  }
+  if (m <= 0) return;
   const double* ih = ws + 15 * n;
   float qloc = 0.f, yloc = 0.f;  // max 2 (1/h_{k-1} + 1/h_k) and max |y| over this thread's rows
   for (int j = tid; j < m; j += nt) {
-    fd0[j] = (float)d0[j]; fd1[j] = (float)d1[j]; fd2[j] = (float)d2[j];
-    qloc = fmaxf(qloc, 2.f * ((float)ih[j] + (float)ih[j + 1]));
+    fd0[j] = ff_narrow(d0[j]); fd1[j] = ff_narrow(d1[j]); fd2[j] = ff_narrow(d2[j]);
+    qloc = fmaxf(qloc, 2.f * (ff_narrow(ih[j]) + ff_narrow(ih[j + 1])));
   }
-  for (int i = tid; i < n; i += nt) yloc = fmaxf(yloc, fmaxf(fabsf((float)yx[i]), fabsf((float)yy[i])));
+  for (int i = tid; i < n; i += nt) yloc = fmaxf(yloc, fmaxf(fabsf(ff_narrow(yx[i])), fabsf(ff_narrow(yy[i]))));
   __syncthreads();
   float* pa = fl1;  // pivots a_j = l0_j^2
   float* pt = fl2;  // t_j = l0_j l1_j
@@ -771,8 +765,8 @@ __global__ void __launch_bounds__(kSplineThreads) k_spline_fit(SplineArgs A) {
     fb[j] = j >= 2 ? fd2[j - 2] * rsqrtf(pa[j - 2]) * il : 0.f;  // l2_{j-2} / l0_j
     fp[j] = pt[j] * il * il;                                     // l1_j / l0_j
     fq[j] = fd2[j] * il * il;                                    // l2_j / l0_j
-    wx[j] = (float)rx[j] * il;
-    wy[j] = (float)ry[j] * il;
+    wx[j] = ff_narrow(rx[j]) * il;
+    wy[j] = ff_narrow(ry[j]) * il;
   }
   __syncthreads();
   // fd0/fd1 are free now: forward-sweep scratch
@@ -787,10 +781,10 @@ __global__ void __launch_bounds__(kSplineThreads) k_spline_fit(SplineArgs A) {
     // x += e (FP64), then the FP64 residual of the next pass
     float mx[4] = {0.f, 0.f, qloc, yloc};  // |e|, |gamma|, |Q| bound, |y|
     for (int j = tid; j < m; j += nt) {
-      const double vx = cx[j + 1] + (double)ex[j], vy = cy[j + 1] + (double)ey[j];
+      const double vx = cx[j + 1] + ff_widen(ex[j]), vy = cy[j + 1] + ff_widen(ey[j]);
       cx[j + 1] = vx; cy[j + 1] = vy;
       mx[0] = fmaxf(mx[0], fmaxf(fabsf(ex[j]), fabsf(ey[j])));
-      mx[1] = fmaxf(mx[1], fmaxf(fabsf((float)vx), fabsf((float)vy)));
+      mx[1] = fmaxf(mx[1], fmaxf(fabsf(ff_narrow(vx)), fabsf(ff_narrow(vy))));
     }
     block_max_f32<4>(mx, red);
     const float emax = mx[0], xmax = mx[1];
@@ -809,8 +803,8 @@ __global__ void __launch_bounds__(kSplineThreads) k_spline_fit(SplineArgs A) {
       if (j >= 2) { ax = fma(d2[j - 2], cx[j - 1], ax); ay = fma(d2[j - 2], cy[j - 1], ay); }
       if (j + 1 < m) { ax = fma(d1[j], cx[j + 2], ax); ay = fma(d1[j], cy[j + 2], ay); }
       if (j + 2 < m) { ax = fma(d2[j], cx[j + 3], ax); ay = fma(d2[j], cy[j + 3], ay); }
-      wx[j] = (float)(rx[j] - ax) * fil[j];
-      wy[j] = (float)(ry[j] - ay) * fil[j];
+      wx[j] = ff_narrow(rx[j] - ax) * fil[j];
+      wy[j] = ff_narrow(ry[j] - ay) * fil[j];
     }
     __syncthreads();
   }
@@ -818,11 +812,6 @@ __global__ void __launch_bounds__(kSplineThreads) k_spline_fit(SplineArgs A) {
     if (tid == 0)
       chol_solve_f64(m, d0, d1, d2, rx, ry, ws + 12 * n, ws + 13 * n, ws + 14 * n, cx, cy);
     __syncthreads();
-  }
-  // fitted values g = y - lam Q gamma
-  for (int i = tid; i < n; i += nt) {
-    gx[i] = spline_g(n, ih, yx, cx, lam, i);
-    gy[i] = spline_g(n, ih, yy, cy, lam, i);
   }
 }
 
@@ -838,6 +827,7 @@ struct ColArgs {
   unsigned* err;
   DevMesh m;
   double cY, cS;
+  double lam;                             // of the spline fit
   const double* up_cols;                  // per-column upstream state (4 x Nchi) or null
   int move, on_S;
   int disturbed;                          // any freestream disturbance amplitude non-zero
@@ -848,21 +838,29 @@ struct ColArgs {
   long lane, ws_lane;  // offsets of the next lane's buffers and spline workspace (grid z)
 };
 
-// value and slope of the fitted spline at t (Linear() extrapolation outside the knots)
-__device__ void spline_at(int n, const double* xs, const double* g, const double* gam, const double* ih, double t,
-                          int guess, double& val, double& der) {
+// value and slope of the fitted spline at t (Linear() extrapolation outside the knots); the
+// fitted values of the two knots it needs are formed here, by every column's threads, not by the
+// one block of the fit
+__device__ void spline_at(int n, const double* xs, const double* ys, const double* gam, const double* ih, double lam,
+                          double t, int guess, double& val, double& der) {
+  double g0, g1;  // of knots k, k + 1
+  auto fitted = [&](int k) {
+    g0 = spline_g(n, ih, ys, gam, lam, k);
+    g1 = spline_g(n, ih, ys, gam, lam, k + 1);
+  };
   auto in_der = [&](int k, double tt) {
     const double h = xs[k + 1] - xs[k], a = xs[k + 1] - tt, b = tt - xs[k];
-    return (g[k + 1] - g[k]) * ih[k] + ((h * h - 3 * a * a) * gam[k] + (3 * b * b - h * h) * gam[k + 1]) * (ih[k] * (1.0 / 6));
+    return (g1 - g0) * ih[k] + ((h * h - 3 * a * a) * gam[k] + (3 * b * b - h * h) * gam[k + 1]) * (ih[k] * (1.0 / 6));
   };
-  if (t < xs[0]) { der = in_der(0, xs[0]); val = g[0] + der * (t - xs[0]); return; }
-  if (t > xs[n - 1]) { der = in_der(n - 2, xs[n - 1]); val = g[n - 1] + der * (t - xs[n - 1]); return; }
+  if (t < xs[0]) { fitted(0); der = in_der(0, xs[0]); val = g0 + der * (t - xs[0]); return; }
+  if (t > xs[n - 1]) { fitted(n - 2); der = in_der(n - 2, xs[n - 1]); val = g1 + der * (t - xs[n - 1]); return; }
   // the knots stay close to the mesh abscissae, so walk from the column's own interval
   int k = guess < 0 ? 0 : (guess > n - 2 ? n - 2 : guess);
   while (k > 0 && xs[k] > t) --k;
   while (k < n - 2 && xs[k + 1] <= t) ++k;
+  fitted(k);
   const double h = xs[k + 1] - xs[k], a = xs[k + 1] - t, b = t - xs[k];
-  val = (a * g[k] + b * g[k + 1]) * ih[k] + ((a * a * a - h * h * a) * gam[k] + (b * b * b - h * h * b) * gam[k + 1]) * (ih[k] * (1.0 / 6));
+  val = (a * g0 + b * g1) * ih[k] + ((a * a * a - h * h * a) * gam[k] + (b * b * b - h * h * b) * gam[k + 1]) * (ih[k] * (1.0 / 6));
   der = in_der(k, t);
 }
 
@@ -915,8 +913,8 @@ __global__ void __launch_bounds__(kColThreads) k_shock_columns(ColArgs A) {
   const double* xs = A.ws + (LANES ? blockIdx.z * A.ws_lane : 0);
   const double* cxs = xs + 3 * nchi;
   const double* cys = xs + 4 * nchi;
-  const double* gxs = xs + 5 * nchi;
-  const double* gys = xs + 6 * nchi;
+  const double* yxs = xs + nchi;
+  const double* yys = xs + 2 * nchi;
   const double* ih = xs + 15 * nchi;
   const ShockPts pts = lane_pts(A.pts, off);
   const Cons q = lane_cons(A.tgt, off);
@@ -926,7 +924,7 @@ __global__ void __launch_bounds__(kColThreads) k_shock_columns(ColArgs A) {
   // and its slope at the column's abscissa
   if (act && w < 2) {
     double v, dv;
-    spline_at(nchi, xs, w == 0 ? gxs : gys, w == 0 ? cxs : cys, ih, A.m.chi1[i], i - 1, v, dv);
+    spline_at(nchi, xs, w == 0 ? yxs : yys, w == 0 ? cxs : cys, ih, A.lam, A.m.chi1[i], i - 1, v, dv);
     (w == 0 ? sh.xv : sh.yv)[lane] = v;
     (w == 0 ? sh.xd : sh.yd)[lane] = dv;
   } else if (act) {
@@ -2477,6 +2475,7 @@ void launch_columns_bc(const DevCtx& d, bool on_S, bool move, double cY, double 
     ca.pts = pts;
     ca.pS = d.Sp;
     ca.ws = d.spl;
+    ca.lam = (1 - c.spline_param) / c.spline_param;
     ca.cell_idx = d.cell_idx;
     ca.beta = d.beta;
     ca.speed_x = d.speed_x;
