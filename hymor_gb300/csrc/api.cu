@@ -433,8 +433,10 @@ size_t stage_bytes(int n) {  // a multiple of 256: hymor_residual's staged flux 
   return (header_doubles(n) * sizeof(double) + kErrCount * sizeof(unsigned) + 255) & ~size_t(255);
 }
 // a residual's flux up to this size goes through the staging buffer when the caller's memory is
-// pageable (2 MB: a host copy of ~0.1 ms)
-constexpr size_t kFluxStage = 2u << 20;
+// pageable: the host's copy out of it runs at ~25 GB/s, so that the driver's own path is the
+// faster one beyond. The residual in us, staged and straight: 30 x 20 39.4 and 44.9, 60 x 40 43
+// and 46, 90 x 40 (115 KB) 45.8 and 46.6, 120 x 60 (230 KB) 53 and 47, 500 x 120 (1.9 MB) 196 and 78
+constexpr size_t kFluxStage = 128u << 10;
 
 int read_err(hymor_ctx* ctx) {  // through the staging buffer, as the state's download
   unsigned* h = reinterpret_cast<unsigned*>(ctx->stage + header_doubles(ctx->d.nchi) * sizeof(double));
@@ -881,9 +883,7 @@ int hymor_residual(hymor_ctx* ctx, double* flux) {
   CU(cudaGetLastError());
   if (!flux) return read_err(ctx);
   // The four planes in one copy, straight into page-locked memory, or through the pinned staging
-  // buffer and one host copy (a copy into pageable memory waits for the stream and goes through
-  // the driver's own staging each time: 180 x 60, four planes, 27 us more than page-locked ones);
-  // a large flux goes straight to pageable memory, where the driver's staging overlaps.
+  // buffer and one host copy, or (above kFluxStage) straight into pageable memory.
   const size_t bytes = 4 * (size_t)d.N * sizeof(double);
   cudaPointerAttributes at;
   const bool pinned = cudaPointerGetAttributes(&at, flux) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;

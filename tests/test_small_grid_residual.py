@@ -1,6 +1,6 @@
 """The residual's small-grid paths: both boundary phases in one block (up to 512 points a phase),
-half-height tiles while there are no more tiles than SMs, and its flux through the staging
-buffer, straight into page-locked memory, or straight into pageable memory (above 2 MB)."""
+half-height tiles while there are no more of them than SMs, and its flux through the staging
+buffer, straight into page-locked memory, or straight into pageable memory (above 128 KB)."""
 import numpy as np
 import pytest
 import torch
