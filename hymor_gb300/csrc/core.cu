@@ -50,8 +50,14 @@ struct TileGeo {
   static constexpr int PS = TMA ? (HP * (TYV + 2) + 15) / 16 * 16 : NH;  // halo plane stride
   static constexpr int NCOR = CX * (TYV + 1);      // corners
   static constexpr int NBTF = TX * (TYV + 1);      // bt faces
-  static constexpr int THREADS = 32 * TYV;
 };
+// Threads of a tile's block: a warp per tile row, or (WIDE) a warp per row of lr faces and one
+// per row of bt faces. On a grid of few tiles the time of a tile is what the step waits for, and
+// with a warp per tile row that is three faces one after another (one lr, two of the 5 x 31 bt
+// faces); WIDE evaluates all of them at once, in registers (72 at most) that a full SM of tiles
+// does not have. kWideTiles is the line.
+template <int TYV, bool WIDE>
+constexpr int flux_threads() { return WIDE ? 32 * (2 * TYV + 1) : 32 * TYV; }
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
   return static_cast<unsigned>(__cvta_generic_to_shared(p));
@@ -1348,10 +1354,11 @@ __device__ __forceinline__ void face_flux_ff(const FluxArgs& a, const double* s_
 }
 
 // Returns false when a TMA wait gave up (the block then stops).
-template <bool AXI, bool SUTH, int TYV, bool FFV, bool TMA>
+template <bool AXI, bool SUTH, int TYV, bool FFV, bool TMA, bool WIDE>
 __device__ __forceinline__ bool flux_tile(const FluxArgs& a, const FluxMaps& tm, int bx, int by, double* sm,
                                           uint64_t* bar, unsigned& phase) {
   using G = TileGeo<TYV, TMA>;
+  constexpr int NT = flux_threads<TYV, WIDE>();
   // halo planes; with TMA the first six are the staged copies of the ghosted planes
   double* s_r = sm;
   double* s_ru = s_r + G::PS;
@@ -1412,7 +1419,7 @@ __device__ __forceinline__ bool flux_tile(const FluxArgs& a, const FluxMaps& tm,
     for (int o = 16; o > 0; o >>= 1) sc = max(sc, __shfl_xor_sync(0xffffffffu, sc, o));
     if (j0 + 1 >= sc) {
       const int ci = i0 + lane, cj = j0 + warp;
-      if (lane < TX && ci < nchi && cj < neta) {
+      if (lane < TX && (!WIDE || warp < TYV) && ci < nchi && cj < neta) {
         const long c = off + (long)ci + (long)cj * nchi;
         a.o0[c] = 0; a.o1[c] = 0; a.o2[c] = 0; a.o3[c] = 0;
       }
@@ -1447,7 +1454,7 @@ __device__ __forceinline__ bool flux_tile(const FluxArgs& a, const FluxMaps& tm,
     }
   }
   // (1) halo cells: ghosted (i0 + hx, j0 + hy)
-  for (int h0 = tid; h0 < G::NH; h0 += G::THREADS) {
+  for (int h0 = tid; h0 < G::NH; h0 += NT) {
     const int hx = h0 % HX, hy = h0 / HX;
     const int h = hid(hx, hy);
     const int gi = i0 + hx, gj = j0 + hy;
@@ -1476,7 +1483,7 @@ __device__ __forceinline__ bool flux_tile(const FluxArgs& a, const FluxMaps& tm,
   }
   __syncthreads();
   // (2) corner averages (VISCOUS_FLUX.jl:67-70, 184-185)
-  for (int cidx = tid; cidx < G::NCOR; cidx += G::THREADS) {
+  for (int cidx = tid; cidx < G::NCOR; cidx += NT) {
     const int cx = cidx % CX, cy = cidx / CX;
     if (i0 + cx <= nchi && j0 + cy <= neta) {
       const int h00 = hid(cx, cy), h10 = h00 + 1, h01 = h00 + G::HP, h11 = h01 + 1;
@@ -1499,7 +1506,8 @@ __device__ __forceinline__ bool flux_tile(const FluxArgs& a, const FluxMaps& tm,
   {
     const int fx = lane, fy = warp;
     const int gi = i0 + fx, gj = j0 + fy;  // face (gi, gj) 0-based: between ghosted (gi, gj+1), (gi+1, gj+1)
-    if (FFV && gi <= nchi && gj < neta) {
+    if (WIDE && warp >= TYV) {  // a warp of the bt faces
+    } else if (FFV && gi <= nchi && gj < neta) {
       const long f = (long)gi + (long)gj * (nchi + 1);
       const int L = hid(fx, fy + 1);
       face_flux_ff<true, AXI, SUTH>(a, s_r, s_ru, s_rv, s_rE, s_p, fu, fv, fT, fuc, fvc, fTc, L, L + 1,
@@ -1567,7 +1575,8 @@ __device__ __forceinline__ bool flux_tile(const FluxArgs& a, const FluxMaps& tm,
   for (int k = 0; k < 4; ++k) dl[k] = fl[k] - __shfl_down_sync(0xffffffffu, fl[k], 1);
   const double tls = AXI ? tl + __shfl_down_sync(0xffffffffu, tl, 1) : 0.0;
   // (3b) bt faces: TX x (TYV + 1)
-  for (int b = tid; b < (TX + 1) * (TYV + 1); b += G::THREADS) {
+  constexpr int NB = (TX + 1) * (TYV + 1);
+  for (int b = !WIDE ? tid : (warp < TYV ? NB : tid - 32 * TYV); b < NB; b += NT) {
     const int fx = b & 31, fy = b >> 5;
     if (fx >= TX) continue;
     const int gi = i0 + fx, gj = j0 + fy;  // face (gi, gj): between ghosted (gi+1, gj), (gi+1, gj+1)
@@ -1634,7 +1643,7 @@ __device__ __forceinline__ bool flux_tile(const FluxArgs& a, const FluxMaps& tm,
   {
     const int cx = lane, cy = warp;
     const int ci = i0 + cx, cj = j0 + cy;
-    if (cx < TX && ci < nchi && cj < neta) {
+    if (cx < TX && (!WIDE || cy < TYV) && ci < nchi && cj < neta) {
       const long c = (long)ci + (long)cj * nchi;
       double r0 = 0, r1 = 0, r2 = 0, r3 = 0;
       const bool active = !a.mask || (cj + 1 < a.cell_idx[ci]);
@@ -1667,12 +1676,12 @@ __device__ __forceinline__ bool flux_tile(const FluxArgs& a, const FluxMaps& tm,
 // The 2-D constant-viscosity 31 x 4 kernel is held to 56 registers for nine resident blocks
 // per SM (its shared memory allows ten), so that the persistent interior grid of the split
 // tiling keeps eight beside a spare slot; the others to 64.
-template <bool AXI, bool SUTH, int TYV>
-constexpr int flux_min_blocks() { return TYV == 4 && !AXI && !SUTH ? 9 : 32 / TYV; }
+template <bool AXI, bool SUTH, int TYV, bool WIDE>
+constexpr int flux_min_blocks() { return WIDE ? 3 : TYV == 4 && !AXI && !SUTH ? 9 : 32 / TYV; }
 
 // Tile grid (no list), or a persistent grid striding over the compact tile list of a class.
-template <bool AXI, bool SUTH, int TYV, bool FFV, bool TMA>
-__global__ void __launch_bounds__(32 * TYV, flux_min_blocks<AXI, SUTH, TYV>())
+template <bool AXI, bool SUTH, int TYV, bool FFV, bool TMA, bool WIDE = false>
+__global__ void __launch_bounds__((flux_threads<TYV, WIDE>()), (flux_min_blocks<AXI, SUTH, TYV, WIDE>()))
     k_flux(FluxArgs a, const __grid_constant__ FluxMaps tm) {
   extern __shared__ double sm_raw[];
   __shared__ uint64_t bar;  // completion of the halo TMA transfers of a tile
@@ -1687,13 +1696,13 @@ __global__ void __launch_bounds__(32 * TYV, flux_min_blocks<AXI, SUTH, TYV>())
     __syncthreads();
   }
   if (!a.list) {
-    flux_tile<AXI, SUTH, TYV, FFV, TMA>(a, tm, blockIdx.x, blockIdx.y, sm, &bar, phase);
+    flux_tile<AXI, SUTH, TYV, FFV, TMA, WIDE>(a, tm, blockIdx.x, blockIdx.y, sm, &bar, phase);
     return;
   }
   const int n = *a.count;
   for (int k = blockIdx.x; k < n; k += gridDim.x) {
     const int t = a.list[k];
-    if (!flux_tile<AXI, SUTH, TYV, FFV, TMA>(a, tm, t % a.tiles_x, t / a.tiles_x, sm, &bar, phase)) return;
+    if (!flux_tile<AXI, SUTH, TYV, FFV, TMA, WIDE>(a, tm, t % a.tiles_x, t / a.tiles_x, sm, &bar, phase)) return;
     __syncthreads();  // the next tile reuses the shared arrays
   }
 }
@@ -2638,9 +2647,16 @@ void launch_band_tiles(const DevCtx& d, const int* rows, int& jlo, int& jhi, cud
 
 template <bool AXI, bool SUTH, bool FFV, int TYV, bool TMA>
 void flux_launch_rows(const FluxArgs& a, const FluxMaps& tm, int tile_class, dim3 grid, const DevCtx& d,
-                      cudaStream_t st) {
+                      cudaStream_t st, bool wide = false) {
   const size_t smem = flux_smem<AXI, SUTH, TYV, TMA>();
   grid.z = d.lanes;
+  if constexpr (TYV == TY / 2 && !TMA) {
+    if (wide) {
+      if (a.list) grid = dim3(2 * d.sms, 1);
+      k_flux<AXI, SUTH, TYV, FFV, TMA, true><<<grid, flux_threads<TYV, true>(), smem, st>>>(a, tm);
+      return;
+    }
+  }
   if (tile_class == 1 && a.list) {
     // the shock/boundary class: a persistent grid of one block per SM over its few tiles (two
     // of the half-height tiles)
@@ -2655,10 +2671,10 @@ void flux_launch_rows(const FluxArgs& a, const FluxMaps& tm, int tile_class, dim
 
 template <bool AXI, bool SUTH, bool FFV>
 void flux_launch(const FluxArgs& a, const FluxMaps& tm, int tile_class, dim3 grid, const DevCtx& d,
-                 cudaStream_t st, int rows, bool tma) {
+                 cudaStream_t st, int rows, bool tma, bool wide) {
   const bool r16 = rows == 16;
   if (rows == TY / 2) {
-    flux_launch_rows<AXI, SUTH, FFV, TY / 2, false>(a, tm, tile_class, grid, d, st);
+    flux_launch_rows<AXI, SUTH, FFV, TY / 2, false>(a, tm, tile_class, grid, d, st, wide);
   } else if (tma) {
     if (r16) flux_launch_rows<AXI, SUTH, FFV, 16, true>(a, tm, tile_class, grid, d, st);
     else flux_launch_rows<AXI, SUTH, FFV, TY, true>(a, tm, tile_class, grid, d, st);
@@ -2668,6 +2684,10 @@ void flux_launch(const FluxArgs& a, const FluxMaps& tm, int tile_class, dim3 gri
   }
 }
 
+// Half-height tiles a block of a warp per face row (flux_threads) takes, as a multiple of the
+// SMs. us for the steps of a march, WIDE and not: 100 x 80 (80 tiles) 2036 and 2110, 200 x 150
+// (266) 1104 and 1159; 300 x 200 (500) 1261 and 1231, 400 x 200 (650) 1348 and 1309.
+constexpr long kWideTiles = 2;
 void launch_flux_class(const DevCtx& d, bool on_S, double* const out[4], int tile_class, cudaStream_t st,
                        int spare, bool ffv) {
   FluxArgs a;
@@ -2686,11 +2706,14 @@ void launch_flux_class(const DevCtx& d, bool on_S, double* const out[4], int til
   a.lane = d.lane_stride;
   // the split tiling's classes: half-height tiles, halo by thread loads
   // and a whole grid of few tiles: an FP64 tile takes as long as its warps' FP64 instructions on
-  // one SM, so half the warps on twice the SMs finish sooner while SMs are idle (180 x 60,
-  // the residual without its copy to the host, with k_thermo_sound and k_bc_edges_one: 48 -> 36 us)
-  const bool few = tile_class < 0 && !ffv && d.lanes == 1 && flux_tiles(d) <= d.sms;
+  // one SM, so half the warps on twice the SMs finish sooner while every half tile has an SM of
+  // its own (180 x 60, the residual without its copy to the host, with k_thermo_sound and
+  // k_bc_edges_one: 48 -> 36 us; with WIDE blocks too, and its copy: 59.4 -> 46.3 us)
+  const long halves = (long)flux_tiles_x(d) * ((d.neta + TY / 2 - 1) / (TY / 2));
+  const bool few = tile_class < 0 && !ffv && d.lanes == 1 && halves <= d.sms;
   const bool half = (flux_split(d) && tile_class >= 0 && d.tiles) || few;
   const int rows = half ? TY / 2 : flux_rows(d);
+  const bool wide = half && d.lanes == 1 && halves <= kWideTiles * d.sms;
   const bool tma = d.tma && !half;
   FluxMaps tm;
   if (tma) {
@@ -2726,15 +2749,15 @@ void launch_flux_class(const DevCtx& d, bool on_S, double* const out[4], int til
     grid = dim3((b > spare + 1 ? b - spare : 1) * d.sms, 1);
   }
   if (ffv) {
-    if (!axi && !suth) flux_launch<false, false, true>(a, tm, tile_class, grid, d, st, rows, tma);
-    else if (axi && !suth) flux_launch<true, false, true>(a, tm, tile_class, grid, d, st, rows, tma);
-    else if (!axi && suth) flux_launch<false, true, true>(a, tm, tile_class, grid, d, st, rows, tma);
-    else flux_launch<true, true, true>(a, tm, tile_class, grid, d, st, rows, tma);
+    if (!axi && !suth) flux_launch<false, false, true>(a, tm, tile_class, grid, d, st, rows, tma, wide);
+    else if (axi && !suth) flux_launch<true, false, true>(a, tm, tile_class, grid, d, st, rows, tma, wide);
+    else if (!axi && suth) flux_launch<false, true, true>(a, tm, tile_class, grid, d, st, rows, tma, wide);
+    else flux_launch<true, true, true>(a, tm, tile_class, grid, d, st, rows, tma, wide);
   } else {
-    if (!axi && !suth) flux_launch<false, false, false>(a, tm, tile_class, grid, d, st, rows, tma);
-    else if (axi && !suth) flux_launch<true, false, false>(a, tm, tile_class, grid, d, st, rows, tma);
-    else if (!axi && suth) flux_launch<false, true, false>(a, tm, tile_class, grid, d, st, rows, tma);
-    else flux_launch<true, true, false>(a, tm, tile_class, grid, d, st, rows, tma);
+    if (!axi && !suth) flux_launch<false, false, false>(a, tm, tile_class, grid, d, st, rows, tma, wide);
+    else if (axi && !suth) flux_launch<true, false, false>(a, tm, tile_class, grid, d, st, rows, tma, wide);
+    else if (!axi && suth) flux_launch<false, true, false>(a, tm, tile_class, grid, d, st, rows, tma, wide);
+    else flux_launch<true, true, false>(a, tm, tile_class, grid, d, st, rows, tma, wide);
   }
 }
 
