@@ -2937,14 +2937,21 @@ int hymor_jacobian_set(hymor_ctx* ctx, const double* coef) {
 }
 
 // Whether the fixed-point matvec takes k vectors, with its parts made (their storage on first
-// use; without the memory for it the FP64 matvec serves).
+// use, whatever another stream of the caller captures; without the memory for it, and while the
+// context's stream is captured, the FP64 matvec serves: a replay reads the blocks of its time).
 static bool fx_ready(hymor_ctx* ctx, int k, int transpose) {
   DevCtx& d = ctx_dev(ctx);
   const int t = transpose != 0;
-  if (!fx_takes(d, k)) return false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (!fx_takes(d, k) || cudaStreamIsCapturing(ctx_stream(ctx), &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
+    return false;
   if (!d.fx_part[t]) {
     void *p = nullptr, *e = nullptr;
-    if (cudaMalloc(&p, sizeof(int2) * 144 * d.N) != cudaSuccess || cudaMalloc(&e, sizeof(short) * 16 * d.N) != cudaSuccess) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const bool ok = cudaMalloc(&p, sizeof(int2) * 144 * d.N) == cudaSuccess && cudaMalloc(&e, sizeof(short) * 16 * d.N) == cudaSuccess;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (!ok) {
       if (p) cudaFree(p);
       cudaGetLastError();
       return false;

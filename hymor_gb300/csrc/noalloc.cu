@@ -4,10 +4,10 @@
 // service that reserves its whole device-memory budget at start-up and treats any
 // allocation during a solve as a failure, or a host runtime whose own pool allocator
 // owns the device memory and must not see a second allocator take from it.
-// hymor_expm_apply_dev allocates work vectors (and, with the shock-position unknowns,
-// instantiates a CUDA graph of one Taylor step); this entry point takes its work
-// vectors from one fixed, file-scope device array and launches every Taylor step
-// directly, so the call itself allocates nothing.
+// hymor_expm_apply_dev allocates work vectors (and, with the shock-position unknowns on
+// larger grids, instantiates a CUDA graph of one Taylor step); this entry point
+// takes its work vectors from one fixed, file-scope device array and makes no graph, so
+// the call itself allocates nothing.
 //
 // Limits and sharing rules:
 //   * the array holds 3 x kNoAllocVec doubles (24 MiB) and is held by every GPU

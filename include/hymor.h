@@ -271,9 +271,9 @@ int hymor_expm_apply_multi_dev(hymor_ctx* ctx, int k, const double* dts, const i
  * For callers that cannot call cudaMalloc during a solve: a service that reserves its whole
  * device-memory budget at start-up and treats any later allocation as a failure, or a host
  * runtime whose own pool allocator owns the device memory. hymor_expm_apply_dev allocates
- * work vectors per call (and, with the shock unknowns, instantiates a CUDA graph of one
- * Taylor step); this variant takes its work vectors from one fixed 24 MiB device array that
- * every GPU loading the library holds until exit, and launches every Taylor step directly.
+ * work vectors per call (and, with the shock unknowns on larger grids, instantiates a
+ * CUDA graph of one Taylor step); this variant takes its work vectors from one fixed 24 MiB
+ * device array that every GPU loading the library holds until exit, and makes no graph.
  * Requires hymor_operator_size * k <= 1048576 (else HYMOR_ERR_INVALID, before any device
  * work). All calls share the array and it keeps the last call's contents (nothing in it
  * needs to start at zero): calls whose GPU work overlaps race, so serialise them. The first
