@@ -2141,12 +2141,17 @@ static void launch_expm_body(const DevCtx& d, int k, double dt, int nsteps, int 
 
 
 // The extended operators' propagation in one cooperative launch (k_expm_ext): from as many
-// launches as the stencil operator's, on grids whose thread-per-output pass is the better one
-// (mv_one; above it a term is long enough to hide its launches, and a batch reads the blocks
-// once for four vectors).
+// launches as the stencil operator's, up to `most` cells x vectors: its 8 warps per SM have fewer
+// loads on their way than the launches' full SMs, so that a term of many cells takes longer alone
+// (with three contexts at once it is the faster one to ~75 000). One propagation of 60 steps of
+// degree 5 alone, ms, in launches and in one: shock-position unknowns 160 x 97 4.3 and 3.0,
+// 180 x 100 4.45 and 4.37, 210 x 105 5.2 and 5.7, 300 x 150 7.8 and 8.9, 500 x 250 17.7 and 33.9;
+// one adjoint vector 243 x 111 6.5 and 6.1, 390 x 190 12.9 and 17.8; the receptivity operator
+// (three launches a term more) 200 x 160, 64 000 in real vectors, 9.6 and 9.3.
 constexpr int kExpmCoopMinLaunches = 16;
-static bool expm_ext_fits(const DevCtx& d, int k, int nsteps, int order) {
-  return (long)nsteps * (order + 1) >= kExpmCoopMinLaunches && mv_one(d.N, k, d.sms);
+constexpr long kExtShock = 20000, kExtShockAdj = 30000, kExtRecept = 64000;
+static bool expm_ext_fits(const DevCtx& d, int k, int nsteps, int order, long most) {
+  return (long)nsteps * (order + 1) >= kExpmCoopMinLaunches && mv_one(d.N, k, d.sms) && d.N * k <= most;
 }
 static ExtArgs ext_args(const DevCtx& d, int k, double dt) {
   ExtArgs a;
@@ -2177,7 +2182,7 @@ static cudaError_t launch_expm_ext(const DevCtx& d, const ExtArgs& a, int transp
 
 void launch_expm(const DevCtx& d, int k, double dt, int nsteps, int order, const double* X, double* Yout,
                  int transpose, double* work, cudaStream_t st, bool graph_ok) {
-  if (d.sj.on && expm_ext_fits(d, k, nsteps, order)) {
+  if (d.sj.on && expm_ext_fits(d, k, nsteps, order, transpose && k == 1 ? kExtShockAdj : kExtShock)) {
     launch_expm_ext(d, ext_args(d, k, dt), transpose, nsteps, order, X, Yout, work, st);
     return;
   }
@@ -3253,7 +3258,7 @@ int hymor_recept_expm_dev(hymor_ctx* ctx, int k, int nw, const double* w, double
   DevCtx& d = ctx_dev(ctx);
   cudaStream_t st = ctx_stream(ctx);
   // (k_expm_ext counts its items in 32 bits)
-  if (expm_ext_fits(d, 2 * k, nsteps, order) && 8L * k * d.nchi * nw < (1L << 30)) {
+  if (expm_ext_fits(d, 2 * k, nsteps, order, kExtRecept) && 8L * k * d.nchi * nw < (1L << 30)) {
     ExtArgs a = ext_args(d, 2 * k, dt);
     a.bq = d.bq;
     a.bs = d.bs;
