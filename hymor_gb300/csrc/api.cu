@@ -661,6 +661,20 @@ int hymor_ctx_create(const hymor_config* cfg, const hymor_mesh* mesh, hymor_ctx*
     if ((r = upload(ctx, &p5, rxb.data(), rxb.size(), "1/x bt"))) return bail(r);
     if ((r = upload(ctx, &p6, gvis.data(), gvis.size(), "viscous CFL geometry"))) return bail(r);
     m.lrg = p1; m.btg = p2; m.rvol = p3; m.rx_lr = p4; m.rx_bt = p5; m.gvis = p6;
+    m.axi = nullptr;
+    if (cfg->axisymmetric) {
+      std::vector<double> ax(2 * (size_t)d.N);
+      for (int j = 0; j < cfg->neta; ++j)
+        for (int i = 0; i < cfg->nchi; ++i) {
+          const long c = i + (long)j * cfg->nchi, g = (i + 1) + (long)(j + 1) * (cfg->nchi + 2);
+          const double y = mesh->y_ext[g], sg = y > 0 ? 1.0 : (y < 0 ? -1.0 : y);
+          ax[c] = (mesh->fb_yn_front - mesh->fb_yn_back) * mesh->fb_area[c] * sg * rvol[c];
+          ax[d.N + c] = 0.25 / mesh->x_ext[g];
+        }
+      double* p7 = nullptr;
+      if ((r = upload(ctx, &p7, ax.data(), ax.size(), "axisymmetric cell factors"))) return bail(r);
+      m.axi = p7;
+    }
     // cell centres transposed (row index fastest), for scans along a chi column
     const int NI = cfg->nchi + 2, NJ = cfg->neta + 2;
     std::vector<double> xt((size_t)NI * NJ), yt((size_t)NI * NJ);

@@ -38,6 +38,9 @@ struct DevMesh {
   const double* lrg;   // kGeoPlanes x NLR
   const double* btg;   // kGeoPlanes x NBT
   const double* rvol;  // N
+  // axisymmetric (2 N, or null): per cell the factor of its pressure in the radial momentum rate,
+  // (front - back normal) x area x sign(y) / vol, and 1 / (4 x) of its centre (the step's flux)
+  const double* axi;
   const double* rx_lr;  // axisymmetric: (2 / Re) / x_face on lr faces (NLR)
   const double* rx_bt;  // axisymmetric: (2 / Re) / x_face on bt faces (NBT)
   const double* gvis;   // kv 2 (A_xi^2 + A_eta^2) / vol^2 per cell, kv = max(4/3, gamma/Pr) / Re
