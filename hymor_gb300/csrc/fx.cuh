@@ -16,10 +16,15 @@ namespace hymor {
 constexpr int kFxBits = 58, kFxLow = 29;
 
 // A factor's shared exponent: E with |x| < 2^E for all of them, from the largest biased exponent
-// field of their doubles; kFxZero when all are zero (or subnormal), kFxBad when one is not finite
-// or E lies outside +-900 (the products' exponents then leave the double range's middle).
+// field of their doubles; kFxZero when all are zero, kFxBad when one is not finite or E lies
+// outside +-900 (the products' exponents then leave the double range's middle). A subnormal is not
+// zero, and its product with a large factor is an ordinary number: it counts as the smallest
+// normal exponent, so that factors of which it is the largest are kFxBad.
 constexpr int kFxZero = -32768, kFxBad = 32767;
-__device__ __forceinline__ int fx_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+__device__ __forceinline__ int fx_field(double x) {
+  const unsigned h = (unsigned)__double2hiint(x) << 1;
+  return max((int)(h >> 21), (int)((h | (unsigned)__double2loint(x)) != 0u));
+}
 __device__ __forceinline__ int fx_exponent(int field) {
   if (field == 0) return kFxZero;
   const int e = field - 1022;

@@ -435,7 +435,7 @@ __device__ __forceinline__ void matvec_multi(const MvArgs& a) {
 // chain. Where that sum (formed beside it from 12 leading bits of the factors, a lower bound) is
 // below 2^-5 of that product, the row is formed in FP64 instead: so it is for single small
 // entries (L e_i stays exact: an entry above the line has all its 53 bits within the 58), for
-// tiles with an infinity or a NaN, and for exponents beyond +-900.
+// tiles with an infinity or a NaN, and for exponents beyond +-900 (subnormal factors among them).
 //
 // What bounds it: the integer multiply pipe, 432 wide multiply-adds per cell and vector (FP64:
 // 144 multiply-adds at a fifteenth of that rate, 0.98 of the pipe by ncu), 51 % busy beside the
