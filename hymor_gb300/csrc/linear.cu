@@ -1012,9 +1012,12 @@ __global__ void __launch_bounds__(MODE == 0 ? kFfThreads : kMvThreads, MODE == 0
 // goes through global memory, and a block waits for its neighbours' terms only, not for the
 // grid. The same pairs as k_expm_coop_ff.
 //
-// The values of a tile's edge are published with their term's number beside each half, {h, s, l,
-// s} in 16 bytes, and a reader of the ring polls the value itself until both halves carry its
-// term's number: no flag, no fence, and one block barrier per matvec. Two buffers take the terms
+// The values of a tile's edge are published with their term's number beside each half, two 64-bit
+// words {h, s} and {l, s}, and a reader of the ring polls the value itself until both words carry
+// its term's number: no flag, no fence, and one block barrier per matvec. A half and its number
+// are one 64-bit element of the access (.v2.b64), because the memory model orders the elements of
+// a vector access in no way and keeps only each of them whole; so a number seen means its half
+// seen, and the two words need no order between them. Two buffers take the terms
 // in turn: a block writes term s + 2 over term s only after it has read term s + 1 of all its
 // neighbours, which they form after they have read term s. The waits are bounded (kResPolls): a
 // block that gives up sets kBitTimeout, leaves NaN and stops, and so do its neighbours in turn;
@@ -1055,8 +1058,15 @@ ResTile res_tiling(const Wrap& w, int blocks, int k) {
   return best;
 }
 
+// a half of a published value with its term's number
+__device__ __forceinline__ unsigned long long res_word(float x, unsigned s) {
+  return (unsigned long long)s << 32 | __float_as_uint(x);
+}
+__device__ __forceinline__ float res_half(unsigned long long w) { return __uint_as_float((unsigned)w); }
+__device__ __forceinline__ unsigned res_term(unsigned long long w) { return (unsigned)(w >> 32); }
+
 __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor tc, int nsteps, int order, const double* xin,
-                                                      double* yout, uint4* g0, uint4* g1, const int* vsteps) {
+                                                      double* yout, ulonglong2* g0, ulonglong2* g1, const int* vsteps) {
   extern __shared__ float2 ff_tile[];
   const long N = a.N;
   const int nchi = a.w.nchi, neta = a.w.neta;
@@ -1096,7 +1106,7 @@ __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor
   // the ring of the term just published; false when a wait gave up
   const int ring = 2 * (w + 2) + 2 * hgt;
   auto exchange = [&](int ka) -> bool {
-    const uint4* g = seq & 1 ? g1 : g0;
+    const ulonglong2* g = seq & 1 ? g1 : g0;
     float2* x = xs + (long)(seq & 1) * kall * 4 * halo;
     bool good = true;
     for (int r = tid; r < ring * 4 * ka; r += nt) {  // the vectors spread over the threads too: a poll is a wait
@@ -1115,17 +1125,14 @@ __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor
       if ((wi && !a.w.per_chi) || (wj && !a.w.per_eta) || (wi && wj)) continue;  // no such input (Wrap::nbr)
       if (wi) ii = ii < 0 ? ii + nchi : ii - nchi;
       if (wj) jj = jj < 0 ? jj + neta : jj - neta;
-      const uint4* p = g + v * a.ld + e * N + ii + (long)jj * nchi;
-      uint4 u;
+      const ulonglong2* p = g + v * a.ld + e * N + ii + (long)jj * nchi;
+      unsigned long long uh, ul;
       int polls = 0;
       do {
-        asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w)
-                     : "l"(p)
-                     : "memory");
-      } while ((u.y != seq || u.w != seq) && ++polls < kResPolls && good);
-      good = good && u.y == seq && u.w == seq;
-      x[((long)v * 4 + e) * halo + hx + hy * hw] = make_float2(__uint_as_float(u.x), __uint_as_float(u.z));
+        asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(uh), "=l"(ul) : "l"(p) : "memory");
+      } while ((res_term(uh) != seq || res_term(ul) != seq) && ++polls < kResPolls && good);
+      good = good && res_term(uh) == seq && res_term(ul) == seq;
+      x[((long)v * 4 + e) * halo + hx + hy * hw] = make_float2(res_half(uh), res_half(ul));
     }
     if (!__syncthreads_and(good)) {
       if (tid == 0) atomicOr(rt.err, kBitTimeout);
@@ -1138,8 +1145,8 @@ __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor
   auto put = [&](int v, ff val) {
     xs[((long)(seq & 1) * kall + v) * 4 * halo + own] = make_float2(val.h, val.l);
     if (edge)
-      asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"((seq & 1 ? g1 : g0) + v * a.ld + comp * N + m),
-                   "r"(__float_as_uint(val.h)), "r"(seq), "r"(__float_as_uint(val.l)), "r"(seq)
+      asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"((seq & 1 ? g1 : g0) + v * a.ld + comp * N + m),
+                   "l"(res_word(val.h, seq)), "l"(res_word(val.l, seq))
                    : "memory");
   };
   if (in)
@@ -2777,7 +2784,7 @@ int expm_cooperative(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
       // two buffers of 16 bytes per value: the four vectors of the other paths (v .. vout); no
       // term has number 0
       if ((r = cuda_check(ctx, cudaMemsetAsync(v, 0, sizeof(double) * 4 * n, st)))) return r;
-      uint4 *g0 = reinterpret_cast<uint4*>(v), *g1 = reinterpret_cast<uint4*>(t2);
+      ulonglong2 *g0 = reinterpret_cast<ulonglong2*>(v), *g1 = reinterpret_cast<ulonglong2*>(t2);
       void* rargs[] = {&bf, &rt, &tc, &nsteps, &order, &dX, &dY, &g0, &g1, &vsteps};
       return cuda_check(ctx, cudaLaunchCooperativeKernel((const void*)k_expm_res_ff, rt.tx * rt.ty,
                                                          (4 * rt.tw * rt.th * rt.groups + 31) / 32 * 32, rargs, res_smem(rt, k), st));
