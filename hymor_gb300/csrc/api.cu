@@ -14,6 +14,7 @@
 namespace hymor {
 void flux_kernel_setup();
 void linear_state_release(void* p);
+int ctx_check_waits(hymor_ctx* c);
 }
 
 using namespace hymor;
@@ -429,14 +430,17 @@ int set_device(hymor_ctx* ctx) {
 constexpr size_t kScalPitch = 32;
 size_t state_pitch(size_t n) { return (n + 31) & ~size_t(31); }
 size_t header_doubles(size_t n) { return 4 * state_pitch(n) + kScalPitch + (n + 1) / 2; }
-size_t stage_bytes(int n) {  // a multiple of 256: hymor_residual's staged flux follows
+// the word that a resident propagation sets when a wait gave up (DevCtx::res_gave_up)
+size_t wait_word(int n) {
   return (header_doubles(n) * sizeof(double) + kErrCount * sizeof(unsigned) + 255) & ~size_t(255);
 }
+size_t stage_bytes(int n) { return wait_word(n) + 256; }  // a multiple of 256: hymor_residual's staged flux follows
 // a residual's flux up to this size goes through the staging buffer when the caller's memory is
 // pageable: the host's copy out of it runs at ~25 GB/s, so that the driver's own path is the
 // faster one beyond. The residual in us, staged and straight: 30 x 20 39.4 and 44.9, 60 x 40 43
 // and 46, 90 x 40 (115 KB) 45.8 and 46.6, 120 x 60 (230 KB) 53 and 47, 500 x 120 (1.9 MB) 196 and 78
 constexpr size_t kFluxStage = 128u << 10;
+constexpr int kResPolls = 1 << 20;  // of a value in a resident propagation: about a second
 
 int read_err(hymor_ctx* ctx) {  // through the staging buffer, as the state's download
   unsigned* h = reinterpret_cast<unsigned*>(ctx->stage + header_doubles(ctx->d.nchi) * sizeof(double));
@@ -795,6 +799,9 @@ int hymor_ctx_create(const hymor_config* cfg, const hymor_mesh* mesh, hymor_ctx*
   const size_t flux_bytes = 4 * (size_t)d.N * sizeof(double);
   if (cudaMallocHost(&ctx->stage, stage_bytes(d.nchi) + (flux_bytes <= kFluxStage ? flux_bytes : 0)) != cudaSuccess)
     return bail(fail(ctx, HYMOR_ERR_CUDA, "pinned staging allocation failed"));
+  d.res_polls = kResPolls;
+  d.res_gave_up = reinterpret_cast<unsigned*>(ctx->stage + wait_word(d.nchi));
+  *d.res_gave_up = 0;
   cudaEventCreate(&ctx->t0);
   cudaEventCreate(&ctx->t1);
   cudaError_t e = cudaDeviceSynchronize();
@@ -1152,6 +1159,12 @@ int hymor_set_expm_arith(hymor_ctx* ctx, int mode) {
   return 0;
 }
 
+int hymor_set_wait_limit(hymor_ctx* ctx, int polls) {
+  if (!ctx || polls < 0) return HYMOR_ERR_INVALID;
+  ctx->d.res_polls = polls;
+  return 0;
+}
+
 int hymor_set_cfl_screen(hymor_ctx* ctx, int on) {
   if (!ctx || on < 0 || on > 1) return HYMOR_ERR_INVALID;
   if (ctx->d.cfl_screen != on) {
@@ -1258,6 +1271,7 @@ int hymor_profile_phases(hymor_ctx* ctx, float* ms) {
 int hymor_synchronize(hymor_ctx* ctx) {
   if (!ctx) return HYMOR_ERR_INVALID;
   CU(cudaStreamSynchronize(ctx->stream));
+  TRY(ctx_check_waits(ctx));
   return read_err(ctx);
 }
 
@@ -1285,7 +1299,7 @@ int hymor_memcpy_d2h(hymor_ctx* ctx, void* dst, const void* src, uint64_t bytes)
   if (!ctx) return HYMOR_ERR_INVALID;
   CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
-  return 0;
+  return ctx_check_waits(ctx);
 }
 
 int hymor_memcpy_d2d(hymor_ctx* ctx, void* dst, const void* src, uint64_t bytes) {
@@ -1302,6 +1316,12 @@ namespace hymor {
 DevCtx& ctx_dev(hymor_ctx* c) { return c->d; }
 cudaStream_t ctx_stream(hymor_ctx* c) { return c->stream; }
 int ctx_fail(hymor_ctx* c, int code, const char* msg) { return fail(c, code, "%s", msg); }
+int ctx_check_waits(hymor_ctx* c) {
+  volatile unsigned* w = c->d.res_gave_up;
+  if (!w || !*w) return 0;
+  *w = 0;
+  return fail(c, HYMOR_ERR_TIMEOUT, "a bounded wait of a resident propagation for its neighbours' values gave up: its results are NaN");
+}
 std::vector<void*>& ctx_allocs(hymor_ctx* c) { return c->allocs; }
 void*& ctx_linear_state(hymor_ctx* c) { return c->linear_state; }
 int ctx_select_device(hymor_ctx* c) { return cudaSetDevice(c->device) == cudaSuccess ? 0 : HYMOR_ERR_CUDA; }

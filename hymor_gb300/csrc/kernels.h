@@ -63,6 +63,10 @@ struct DevCtx {
   int coef_version, coef_ff_version;  // writes of coef, and the write coef_ff was split from
   // the cooperative Taylor propagator in float-float (1, the default) or FP64 (0)
   int expm_ff;
+  // the resident propagation's bounded waits: polls after which a block gives up, and the word in
+  // page-locked host memory that it then sets (read and cleared by ctx_check_waits)
+  int res_polls;
+  unsigned* res_gave_up;
   double* jwork;   // linearisation workspace
   ShockJac sj;
   // prescribed per-column upstream state (4 x Nchi) of the shock chain, or null: set only

@@ -26,6 +26,7 @@ namespace hymor {
 DevCtx& ctx_dev(hymor_ctx* c);
 cudaStream_t ctx_stream(hymor_ctx* c);
 int ctx_fail(hymor_ctx* c, int code, const char* msg);
+int ctx_check_waits(hymor_ctx* c);  // reports (once) a resident propagation that gave up
 }  // namespace hymor
 
 using namespace hymor;
@@ -496,7 +497,8 @@ int hymor_eigs(hymor_ctx* ctx, const hymor_krylov_opts* o, double dt, int nsteps
     info[2] = ks.converged ? 1 : 0;
   }
   if (dvecs && (r = ks.ritz_vectors(dvecs))) return r;
-  return cu(ctx, cudaStreamSynchronize(ctx_stream(ctx)), "eigen solve");
+  if ((r = cu(ctx, cudaStreamSynchronize(ctx_stream(ctx)), "eigen solve"))) return r;
+  return ctx_check_waits(ctx);
 }
 
 int hymor_tg_gain(hymor_ctx* ctx, const hymor_krylov_opts* o, int nh, const double* T, const double* x0,
@@ -607,7 +609,8 @@ int hymor_tg_gain(hymor_ctx* ctx, const hymor_krylov_opts* o, int nh, const doub
         (r = cw.apply(ctx, 2, o->nev, ry.p, dvecs)))
       return r;
   }
-  return cu(ctx, cudaStreamSynchronize(st), "transient-growth solve");
+  if ((r = cu(ctx, cudaStreamSynchronize(st), "transient-growth solve"))) return r;
+  return ctx_check_waits(ctx);
 }
 
 int hymor_dense_schur(int n, const double* A, int nsel, double* T, double* Z, double* wr, double* wi, int32_t* nlead) {

@@ -24,6 +24,7 @@ namespace hymor {
 DevCtx& ctx_dev(hymor_ctx* c);
 cudaStream_t ctx_stream(hymor_ctx* c);
 int ctx_fail(hymor_ctx* c, int code, const char* msg);
+int ctx_check_waits(hymor_ctx* c);  // reports (once) a resident propagation that gave up
 std::vector<void*>& ctx_allocs(hymor_ctx* c);
 void*& ctx_linear_state(hymor_ctx* c);
 void launch_shock_bc_flags(const DevCtx& d, bool on_S, bool copy_pts, bool do_shock, bool do_bc, int a_mode,
@@ -1020,8 +1021,8 @@ __global__ void __launch_bounds__(MODE == 0 ? kFfThreads : kMvThreads, MODE == 0
 // seen, and the two words need no order between them. Two buffers take the terms
 // in turn: a block writes term s + 2 over term s only after it has read term s + 1 of all its
 // neighbours, which they form after they have read term s. The waits are bounded (kResPolls): a
-// block that gives up sets kBitTimeout, leaves NaN and stops, and so do its neighbours in turn;
-// the blocks are co-resident (a cooperative launch).
+// block that gives up sets the context's word in host memory (ctx_check_waits), leaves NaN and
+// stops, and so do its neighbours in turn; the blocks are co-resident (a cooperative launch).
 //
 // What bounds it: the latency of a term, i.e. 36 float-float products in a chain of nine blocks
 // (~3 instructions in four cycles with two warps per sub-partition), the write of a value and its
@@ -1031,13 +1032,13 @@ __global__ void __launch_bounds__(MODE == 0 ? kFfThreads : kMvThreads, MODE == 0
 // shared by groups of threads, so that neither their chains nor their polls follow one another in
 // one thread: 60 x 40, twelve vectors, us for the propagation 1660 with the blocks from L2, 1500
 // in one group, 762 so.
-constexpr int kResPolls = 1 << 20;
 constexpr int kResThreads = 512;  // of a block with several groups: two blocks' registers per SM
 
 struct ResTile {
   int tw, th, tx, ty;  // tile size in cells, tiles
   int groups;          // of threads, a thread per cell and component each, that share the vectors
-  unsigned* err;
+  int polls;           // of a value, after which its reader gives up (0: at the first wait)
+  unsigned* gave_up;   // set by a block that gave up (host memory)
 };
 
 long res_smem(const ResTile& t, int k) {
@@ -1046,13 +1047,13 @@ long res_smem(const ResTile& t, int k) {
 }
 // the tiling of at most `blocks` tiles with the fewest cells per tile (then the smallest halo)
 ResTile res_tiling(const Wrap& w, int blocks, int k) {
-  ResTile best{0, 0, 0, 0, 1, nullptr};
+  ResTile best{0, 0, 0, 0, 1, 0, nullptr};
   for (int tw = 4; tw <= 64; ++tw) {
     const int tx = (w.nchi + tw - 1) / tw;
     if (tx > blocks) continue;
     const int rows = blocks / tx, th = std::max(2, (w.neta + rows - 1) / rows), ty = (w.neta + th - 1) / th;
     const long c = (long)tw * th, b = (long)best.tw * best.th;
-    if (!best.tw || c < b || (c == b && tw + th < best.tw + best.th)) best = ResTile{tw, th, tx, ty, 1, nullptr};
+    if (!best.tw || c < b || (c == b && tw + th < best.tw + best.th)) best = ResTile{tw, th, tx, ty, 1, 0, nullptr};
   }
   best.groups = std::max(1, std::min(k, kResThreads / (4 * best.tw * best.th)));
   return best;
@@ -1108,7 +1109,7 @@ __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor
   auto exchange = [&](int ka) -> bool {
     const ulonglong2* g = seq & 1 ? g1 : g0;
     float2* x = xs + (long)(seq & 1) * kall * 4 * halo;
-    bool good = true;
+    bool good = rt.polls > 0;
     for (int r = tid; r < ring * 4 * ka; r += nt) {  // the vectors spread over the threads too: a poll is a wait
       const int ve = r / ring, v = ve >> 2, e = ve & 3, c = r - ve * ring;
       int hx, hy;
@@ -1130,12 +1131,12 @@ __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor
       int polls = 0;
       do {
         asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(uh), "=l"(ul) : "l"(p) : "memory");
-      } while ((res_term(uh) != seq || res_term(ul) != seq) && ++polls < kResPolls && good);
+      } while ((res_term(uh) != seq || res_term(ul) != seq) && ++polls < rt.polls && good);
       good = good && res_term(uh) == seq && res_term(ul) == seq;
       x[((long)v * 4 + e) * halo + hx + hy * hw] = make_float2(res_half(uh), res_half(ul));
     }
     if (!__syncthreads_and(good)) {
-      if (tid == 0) atomicOr(rt.err, kBitTimeout);
+      if (tid == 0) *reinterpret_cast<volatile unsigned*>(rt.gave_up) = 1u;
       return false;
     }
     ++seq;
@@ -1155,7 +1156,7 @@ __global__ void __launch_bounds__(1024) k_expm_res_ff(MvFf a, ResTile rt, Taylor
       stff(sum, v * items + t, x);
       put(v, x);
     }
-  // (a propagation that gave up leaves NaN beside its error bit)
+  // (a propagation that gave up leaves NaN)
   auto fail = [&]() {
     if (in)
       for (int v = vg; v < kall; v += rt.groups) yout[v * a.ld + comp * N + m] = __longlong_as_double(0x7ff8000000000000LL);
@@ -2780,7 +2781,8 @@ int expm_cooperative(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
                                                               (int)kResSmem))))
         return r;
       ready = true;
-      rt.err = d.err;
+      rt.polls = d.res_polls;
+      rt.gave_up = d.res_gave_up;
       // two buffers of 16 bytes per value: the four vectors of the other paths (v .. vout); no
       // term has number 0
       if ((r = cuda_check(ctx, cudaMemsetAsync(v, 0, sizeof(double) * 4 * n, st)))) return r;
@@ -3091,8 +3093,8 @@ int hymor_expm_apply(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
   if (!r) cudaMemcpyAsync(Y, dy, bytes, cudaMemcpyDeviceToHost, st);
   cudaFreeAsync(dx, st);
   cudaFreeAsync(dy, st);
-  if (r) return r;
-  return cuda_check(ctx, cudaStreamSynchronize(st));
+  if (r || (r = cuda_check(ctx, cudaStreamSynchronize(st)))) return r;
+  return ctx_check_waits(ctx);
 }
 
 }  // extern "C"
@@ -3140,7 +3142,8 @@ int hymor_dot_dev(hymor_ctx* ctx, int64_t n, int m, const double* dA, int64_t ld
   cudaStream_t st = ctx_stream(ctx);
   dots(dA, lda, m, dw, n, k.h, 0, k.partial, st);
   cudaMemcpyAsync(out, k.h, sizeof(double) * m, cudaMemcpyDeviceToHost, st);
-  return cuda_check(ctx, cudaStreamSynchronize(st));
+  if ((r = cuda_check(ctx, cudaStreamSynchronize(st)))) return r;
+  return ctx_check_waits(ctx);
 }
 
 int hymor_krylov_orthogonalize(hymor_ctx* ctx, int64_t n, int m, double* dV, int64_t ldv, double* dw, double* h,
@@ -3166,6 +3169,7 @@ int hymor_krylov_orthogonalize(hymor_ctx* ctx, int64_t n, int m, double* dV, int
   if (m > 0) cudaMemcpyAsync(hh.data(), h1, sizeof(double) * 2 * m, cudaMemcpyDeviceToHost, st);
   cudaMemcpyAsync(hh.data() + 2 * m, nrm, sizeof(double), cudaMemcpyDeviceToHost, st);
   if ((r = cuda_check(ctx, cudaStreamSynchronize(st)))) return r;
+  if ((r = ctx_check_waits(ctx))) return r;  // the vector came from a propagation that gave up
   for (int j = 0; j < m; ++j) h[j] = hh[j] + hh[m + j];
   h[m] = std::sqrt(hh[2 * m]);
   return cuda_check(ctx, cudaGetLastError());

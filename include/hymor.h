@@ -26,7 +26,8 @@ extern "C" {
 #define HYMOR_ERR_CUDA (-2)         /* CUDA runtime error                           */
 #define HYMOR_ERR_NUMERIC (-3)      /* NaN / non-positive density or pressure seen  */
 #define HYMOR_ERR_SHOCK_RANGE (-4)  /* shocked cell too close to the domain top     */
-#define HYMOR_ERR_TIMEOUT (-5)      /* a bounded device wait (TMA transfer) gave up        */
+#define HYMOR_ERR_TIMEOUT (-5)      /* a bounded device wait gave up: a TMA transfer of the
+                                       flux halo, or a propagation's wait for a neighbour  */
 #define HYMOR_ERR_NOT_READY (-6)    /* e.g. matvec before a Jacobian exists         */
 
 /* Boundary conditions (names of utils/Operators/APPLY_BOUNDARY_CONDITIONS.jl). */
@@ -144,6 +145,15 @@ int hymor_set_cfl_screen(hymor_ctx* ctx, int on);
  * the shock-position unknowns and the receptivity operator are FP64 in either mode. The
  * eigen and transient-growth solvers (hymor_eigs, hymor_tg_gain) use the context's mode. */
 int hymor_set_expm_arith(hymor_ctx* ctx, int mode);
+
+/* The float-float propagation of a small grid runs as blocks that wait for their neighbours'
+ * values, each wait for `polls` reads of a value at most (default 2^20, about a second; 0: the
+ * first wait gives up, with which the handling of the failure can be tried). A propagation that
+ * gave up leaves NaN in its results and the context usable; HYMOR_ERR_TIMEOUT comes, once, from
+ * hymor_expm_apply itself, and for the device-pointer entry points from the next
+ * hymor_synchronize, hymor_memcpy_d2h, hymor_dot_dev, hymor_krylov_orthogonalize, hymor_eigs or
+ * hymor_tg_gain. No counterpart in the reference. */
+int hymor_set_wait_limit(hymor_ctx* ctx, int polls);
 
 /* Tile-shape autotuner of the RK step's flux (no counterpart in the reference): times `steps`
  * steps (CUDA events, after a warm-up step) for each flux configuration — the tile halo staged
