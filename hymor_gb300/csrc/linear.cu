@@ -135,7 +135,8 @@ __global__ void k_perturb_thermo(PertArgs a) {
 // takes a cell and loops over its slots, so that a warp writes whole rows of a plane and its
 // reads of the three colours of a row of slots share their lines in L1; one colour at a time
 // every warp wrote a third of the sectors of three planes. Linearisation at 600 x 300: 3.29 ms
-// with a pass per colour, 2.70 ms so.
+// with a pass per colour, 2.70 ms so. PART: the lanes are some of a variable's colours (a device
+// without the memory for nine), one group after another on one stream.
 struct ScatArgs {
   const double* Fp[4];
   const double* Fb[4];
@@ -146,6 +147,7 @@ struct ScatArgs {
   long N;
   long lane;
   int first_var;
+  int colour0, colours;  // PART: the lanes' colours
 };
 
 // d / eps, correctly rounded. The FP64 division of the compiler takes ~25 FP64 instructions
@@ -176,6 +178,7 @@ double div_eps_reciprocal(double eps) {
   return 1.0 / eps;
 }
 
+template <bool PART>
 __global__ void __launch_bounds__(256) k_scatter(ScatArgs a) {
   const long N = a.N, off = 9L * blockIdx.z * a.lane;
   const int var = a.first_var + blockIdx.z;
@@ -193,7 +196,9 @@ __global__ void __launch_bounds__(256) k_scatter(ScatArgs a) {
         const long n = a.w.nbr(i, j, aa, b);
         if (n < 0) continue;
         const unsigned nj = (unsigned)n / nchi_u, ni = (unsigned)n - nj * nchi_u;
-        const long o = off + (long)(3 * (nj % 3u) + ni % 3u) * a.lane + m;  // the input cell's colour
+        const int colour = (int)(3 * (nj % 3u) + ni % 3u) - (PART ? a.colour0 : 0);  // of the input cell
+        if (PART && (colour < 0 || colour >= a.colours)) continue;
+        const long o = off + (long)colour * a.lane + m;
         const int q = (b + 1) * 3 + (aa + 1);
 #pragma unroll
         for (int vo = 0; vo < 4; ++vo) {
@@ -202,7 +207,7 @@ __global__ void __launch_bounds__(256) k_scatter(ScatArgs a) {
           a.coef[((long)(q * 4 + vo) * 4 + var) * N + m] = d;
         }
       }
-    a.nz[var * N + m] = any != 0;
+    a.nz[var * N + m] = any != 0 || (PART && a.colour0 && a.nz[var * N + m]);
   }
 }
 
@@ -2210,7 +2215,8 @@ void launch_expm(const DevCtx& d, int k, double dt, int nsteps, int order, const
 // every kernel launched once for all its lanes (grid z), and the other group's launches run
 // beside it. The base state, the mesh, the base flux and the assembled blocks are shared:
 // read-only, or written at entries no other perturbation writes, with the same arithmetic as
-// one after another, so the result does not depend on the lanes.
+// one after another, so the result does not depend on the lanes. Where the memory for the lanes is
+// missing, fewer serve (ensure_lanes), down to one group of three.
 // One launch per kernel and group instead of one per residual, because the ~9 launches of a
 // residual cost the host ~2 us each: the assembly with the shock unknowns at 200 x 100 (245
 // residuals) took 4.2 ms, bound by them, and takes 1.06 ms so (with its point residuals on the
@@ -2232,7 +2238,7 @@ struct JacLanes {
   cudaEvent_t fork = nullptr;
   double* mem = nullptr;
   long stride = 0;
-  int per_group = 0;
+  int groups = 0, per_group = 0;
 };
 int lanes_per_group(long N) {
   const long want = (1200000 + N - 1) / N;
@@ -2283,7 +2289,7 @@ template <class Run>
 static void for_groups(const JacLanes& L, int n, int most, Run run) {
   const int g = std::min(most, L.per_group);
   int group = 0;
-  for (int q = 0; q < n; q += g, group = (group + 1) % kLaneGroups) run(q, group, std::min(g, n - q));
+  for (int q = 0; q < n; q += g, group = (group + 1) % L.groups) run(q, group, std::min(g, n - q));
 }
 
 // The shock-position blocks (perturb_shock), after the A11 assembly has left the base
@@ -2401,7 +2407,8 @@ void launch_jacobian_assemble(DevCtx& d, cudaStream_t st, JacLanes& L, const int
   // the 36 colour x variable residuals over the lanes; the shock points of all are S's, so
   // the smoothing-spline fit of the base residual serves them
   lanes_fork(L, st);
-  for_groups(L, 36, L.per_group >= 18 ? 18 : 9, [&](int q, int group, int n) {
+  const int most = L.per_group >= 18 ? 18 : (L.per_group >= 9 ? 9 : 3);
+  for_groups(L, 36, most, [&](int q, int group, int n) {
     const DevCtx ld = lane_ctx(d, L, group, n);
     cudaStream_t ls = L.st[group];
     const JacLane& l = L.first[group];
@@ -2415,7 +2422,10 @@ void launch_jacobian_assemble(DevCtx& d, cudaStream_t st, JacLanes& L, const int
     ScatArgs sl = sa;
     for (int v = 0; v < 4; ++v) sl.Fp[v] = l.F[v];
     sl.first_var = q / 9;
-    k_scatter<<<dim3(grid_for(N, 256), 1, n / 9), 256, 0, ls>>>(sl);
+    sl.colour0 = q % 9;
+    sl.colours = n;
+    if (most < 9) k_scatter<true><<<grid_for(N, 256), 256, 0, ls>>>(sl);
+    else k_scatter<false><<<dim3(grid_for(N, 256), 1, n / 9), 256, 0, ls>>>(sl);
   });
   lanes_join(L, st);
   k_masks<<<grid_for(N, 256), 256, 0, st>>>(d.coef_nz, d.coef_nz + N, make_wrap(c), N);
@@ -2475,13 +2485,18 @@ void launch_b_assemble(DevCtx& d, cudaStream_t st, JacLanes& L) {
 using namespace hymor;
 
 namespace {
+// Device memory that the context's linear entry points keep: counted against
+// hymor_set_workspace_limit, and for the context's life unless lin_free gives it back.
+cudaError_t lin_malloc(hymor_ctx* ctx, void** p, size_t bytes);
+void lin_free(hymor_ctx* ctx, void* p, size_t bytes);
+
 // Storage of the shock-position blocks (one allocation of doubles, one of the rows).
 int ensure_shock(hymor_ctx* ctx) {
   DevCtx& d = ctx_dev(ctx);
   if (d.sj.a12) return 0;
   const long n = d.nchi;
   void* p = nullptr;
-  if (cudaMalloc(&p, sizeof(double) * (8 * n + 10 * n * n + 3 * n)) != cudaSuccess)
+  if (lin_malloc(ctx, &p, sizeof(double) * (8 * n + 10 * n * n + 3 * n)) != cudaSuccess)
     return ctx_fail(ctx, HYMOR_ERR_CUDA, "shock-block allocation failed");
   ctx_allocs(ctx).push_back(p);
   double* b = static_cast<double*>(p);
@@ -2493,7 +2508,7 @@ int ensure_shock(hymor_ctx* ctx) {
   j.a22t = j.a12t + 4 * n * n;
   j.rel_b = j.a22t + n * n;
   j.dir = j.rel_b + n;
-  if (cudaMalloc(&p, sizeof(int) * n) != cudaSuccess) return ctx_fail(ctx, HYMOR_ERR_CUDA, "shock-block allocation failed");
+  if (lin_malloc(ctx, &p, sizeof(int) * n) != cudaSuccess) return ctx_fail(ctx, HYMOR_ERR_CUDA, "shock-block allocation failed");
   ctx_allocs(ctx).push_back(p);
   j.rows = static_cast<int*>(p);
   // the transposed shock matvec stages 5 Nchi doubles per block
@@ -2521,13 +2536,13 @@ int ensure_b(hymor_ctx* ctx) {
   DevCtx& d = ctx_dev(ctx);
   if (d.bq) return 0;
   void* p = nullptr;
-  if (cudaMalloc(&p, sizeof(double) * 65 * (long)d.nchi) != cudaSuccess)
+  if (lin_malloc(ctx, &p, sizeof(double) * 65 * (long)d.nchi) != cudaSuccess)
     return ctx_fail(ctx, HYMOR_ERR_CUDA, "upstream-boundary operator allocation failed");
   ctx_allocs(ctx).push_back(p);
   d.bq = static_cast<double*>(p);
   d.bs = d.bq + 48 * d.nchi;
   d.bwork = d.bs + 12 * d.nchi;
-  if (cudaMalloc(&p, sizeof(int) * d.nchi) != cudaSuccess)
+  if (lin_malloc(ctx, &p, sizeof(int) * d.nchi) != cudaSuccess)
     return ctx_fail(ctx, HYMOR_ERR_CUDA, "upstream-boundary operator allocation failed");
   ctx_allocs(ctx).push_back(p);
   d.brows = static_cast<int*>(p);
@@ -2550,15 +2565,15 @@ int ensure_linear(hymor_ctx* ctx) {
   DevCtx& d = ctx_dev(ctx);
   if (!d.coef) {
     void* p = nullptr;
-    if (cudaMalloc(&p, sizeof(double) * 144 * d.N) != cudaSuccess)
+    if (lin_malloc(ctx, &p, sizeof(double) * 144 * d.N) != cudaSuccess)
       return ctx_fail(ctx, HYMOR_ERR_CUDA, "Jacobian allocation failed");
     ctx_allocs(ctx).push_back(p);
     double* coef = static_cast<double*>(p);
-    if (cudaMalloc(&p, 5 * d.N) != cudaSuccess)
+    if (lin_malloc(ctx, &p, 5 * d.N) != cudaSuccess)
       return ctx_fail(ctx, HYMOR_ERR_CUDA, "Jacobian row mask allocation failed");
     ctx_allocs(ctx).push_back(p);
     d.coef_nz = static_cast<unsigned char*>(p);
-    if (cudaMalloc(&p, sizeof(double) * 8 * d.N) != cudaSuccess)
+    if (lin_malloc(ctx, &p, sizeof(double) * 8 * d.N) != cudaSuccess)
       return ctx_fail(ctx, HYMOR_ERR_CUDA, "Jacobian workspace allocation failed");
     ctx_allocs(ctx).push_back(p);
     d.jwork = static_cast<double*>(p);
@@ -2590,6 +2605,7 @@ struct KrylovScratch {
 // Per-context state of the linear entry points, owned by the context (created on first
 // use, released by hymor_ctx_destroy).
 struct LinearState {
+  size_t used = 0, limit = 0;  // bytes of lin_malloc, and their limit (0: none)
   ExpmCache expm;
   KrylovScratch kry;
   bool res_ready = false;  // k_expm_res_ff's shared memory is set
@@ -2605,7 +2621,22 @@ LinearState& linear_state(hymor_ctx* ctx) {
 }
 ExpmCache& expm_cache(hymor_ctx* ctx) { return linear_state(ctx).expm; }
 
-// The linearisation lanes, made on first use (2 groups of 9 to 32 x ~(11 N + 7 ..) doubles).
+cudaError_t lin_malloc(hymor_ctx* ctx, void** p, size_t bytes) {
+  LinearState& s = linear_state(ctx);
+  const cudaError_t e = s.limit && s.used + bytes > s.limit ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
+  if (e == cudaSuccess) s.used += bytes;
+  else cudaGetLastError();  // (a later check of the launches would report it again)
+  return e;
+}
+void lin_free(hymor_ctx* ctx, void* p, size_t bytes) {
+  if (!p) return;
+  cudaFree(p);
+  linear_state(ctx).used -= bytes;
+}
+
+// The linearisation lanes, made on first use: two groups of 9 to 32 lanes of ~88 bytes a cell
+// (800 x 400: 18 lanes, 507 MB), or, where the memory is missing, the first of two groups of 9,
+// one of 9 and one of 3 that fits.
 int ensure_lanes(hymor_ctx* ctx, JacLanes** out) {
   JacLanes& L = linear_state(ctx).lanes;
   *out = &L;
@@ -2614,7 +2645,6 @@ int ensure_lanes(hymor_ctx* ctx, JacLanes** out) {
   const size_t G = d.G, N = d.N, n = d.nchi;
   auto pad = [](size_t k) { return (k + 31) & ~size_t(31); };  // 256-byte aligned parts
   const size_t total = 7 * pad(G) + 4 * pad(N) + 4 * pad(n) + pad(17 * n + 16) + 3 * pad(n) + pad(4 * n);
-  const int per = lanes_per_group(N);
   if (!L.fork && cudaEventCreateWithFlags(&L.fork, cudaEventDisableTiming) != cudaSuccess)
     return ctx_fail(ctx, HYMOR_ERR_CUDA, "linearisation lane event");
   for (int g = 0; g < kLaneGroups; ++g)
@@ -2622,16 +2652,29 @@ int ensure_lanes(hymor_ctx* ctx, JacLanes** out) {
         (!L.done[g] && cudaEventCreateWithFlags(&L.done[g], cudaEventDisableTiming) != cudaSuccess))
       return ctx_fail(ctx, HYMOR_ERR_CUDA, "linearisation lane stream");
   double* mem = nullptr;
-  const size_t bytes = sizeof(double) * total * per * kLaneGroups;
-  if (cudaMalloc(&mem, bytes) != cudaSuccess) return ctx_fail(ctx, HYMOR_ERR_CUDA, "linearisation lane allocation failed");
+  int groups = 0, per = 0;
+  size_t bytes = 0;
+  const int plans[][2] = {{kLaneGroups, lanes_per_group(N)}, {kLaneGroups, 9}, {1, 9}, {1, 3}};
+  for (const auto& p : plans) {
+    groups = p[0];
+    per = p[1];
+    bytes = sizeof(double) * total * per * groups;
+    void* q = nullptr;
+    if (lin_malloc(ctx, &q, bytes) == cudaSuccess) {
+      mem = static_cast<double*>(q);
+      break;
+    }
+  }
+  if (!mem) return ctx_fail(ctx, HYMOR_ERR_CUDA, "linearisation lane allocation failed");
   if (cudaMemsetAsync(mem, 0, bytes, ctx_stream(ctx)) != cudaSuccess) {
-    cudaFree(mem);
+    lin_free(ctx, mem, bytes);
     return ctx_fail(ctx, HYMOR_ERR_CUDA, "linearisation lane allocation failed");
   }
   L.mem = mem;
   L.stride = (long)total;
+  L.groups = groups;
   L.per_group = per;
-  for (int g = 0; g < kLaneGroups; ++g) {
+  for (int g = 0; g < groups; ++g) {
     JacLane& l = L.first[g];
     double* b = mem + total * per * g;
     auto take = [&](size_t k) {
@@ -2679,11 +2722,11 @@ int expm_cooperative(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
   int r;
   if (4 * n + 2 * k > c.cap) {
     if ((r = cuda_check(ctx, cudaStreamSynchronize(st)))) return r;
-    if (c.buf) cudaFree(c.buf);
+    lin_free(ctx, c.buf, sizeof(double) * c.cap);
     c.buf = nullptr;
     c.cap = 0;
     void* p = nullptr;
-    if ((r = cuda_check(ctx, cudaMalloc(&p, sizeof(double) * (4 * n + 2 * k))))) return r;
+    if ((r = cuda_check(ctx, lin_malloc(ctx, &p, sizeof(double) * (4 * n + 2 * k))))) return r;
     c.buf = static_cast<double*>(p);
     c.cap = 4 * n + 2 * k;
   }
@@ -2697,7 +2740,7 @@ int expm_cooperative(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
   if (ffp && (!d.coef_ff || d.coef_ff_version != d.coef_version)) {
     if (!d.coef_ff) {
       void* p = nullptr;
-      if ((r = cuda_check(ctx, cudaMalloc(&p, sizeof(float2) * 144 * d.N)))) return r;
+      if ((r = cuda_check(ctx, lin_malloc(ctx, &p, sizeof(float2) * 144 * d.N)))) return r;
       ctx_allocs(ctx).push_back(p);
       d.coef_ff = static_cast<float2*>(p);
     }
@@ -2829,7 +2872,8 @@ int hymor_linearize(hymor_ctx* ctx) {
   DevCtx& d = ctx_dev(ctx);
   cudaStream_t st = ctx_stream(ctx);
   const bool shock_blocks = d.cfg.shock_enabled && d.cfg.perturb_shock;
-  if (shock_blocks && (r = ensure_shock(ctx))) return r;
+  JacLanes* L = nullptr;
+  if ((shock_blocks && (r = ensure_shock(ctx))) || (r = ensure_lanes(ctx, &L))) return r;  // before S changes
   d.sj.on = 0;
   // LINEARIZE_L.jl:43-56: flow cells and shock BC, thermo, sound speed, boundary conditions
   if (d.cfg.shock_enabled) {
@@ -2846,12 +2890,16 @@ int hymor_linearize(hymor_ctx* ctx) {
     if ((r = cuda_check(ctx, cudaStreamSynchronize(st)))) return r;
     if ((r = check_shock_rows_for_blocks(ctx, rows.data(), d.nchi, d.neta))) return r;
   }
-  JacLanes* L = nullptr;
-  if ((r = ensure_lanes(ctx, &L))) return r;
   launch_jacobian_assemble(d, st, *L, rows.data());
   if ((r = cuda_check(ctx, cudaGetLastError()))) return r;
   if ((r = cuda_check(ctx, cudaStreamSynchronize(st)))) return r;
   d.sj.on = shock_blocks;
+  return 0;
+}
+
+int hymor_set_workspace_limit(hymor_ctx* ctx, uint64_t bytes) {
+  if (!ctx) return HYMOR_ERR_INVALID;
+  linear_state(ctx).limit = bytes;
   return 0;
 }
 
@@ -3105,11 +3153,11 @@ int ensure_scratch(hymor_ctx* ctx, int cols, long tmp_n) {
   KrylovScratch& k = kscratch(ctx);
   if (cols > k.cols) {
     void* p;
-    if (cudaMalloc(&p, sizeof(double) * (long)kDotBlocks * cols) != cudaSuccess)
+    if (lin_malloc(ctx, &p, sizeof(double) * (long)kDotBlocks * cols) != cudaSuccess)
       return ctx_fail(ctx, HYMOR_ERR_CUDA, "Krylov scratch allocation failed");
     ctx_allocs(ctx).push_back(p);
     k.partial = static_cast<double*>(p);
-    if (cudaMalloc(&p, sizeof(double) * (2 * cols + 4)) != cudaSuccess)
+    if (lin_malloc(ctx, &p, sizeof(double) * (2 * cols + 4)) != cudaSuccess)
       return ctx_fail(ctx, HYMOR_ERR_CUDA, "Krylov scratch allocation failed");
     ctx_allocs(ctx).push_back(p);
     k.h = static_cast<double*>(p);
@@ -3117,7 +3165,7 @@ int ensure_scratch(hymor_ctx* ctx, int cols, long tmp_n) {
   }
   if (tmp_n > k.tmp_n) {
     void* p;
-    if (cudaMalloc(&p, sizeof(double) * tmp_n) != cudaSuccess)
+    if (lin_malloc(ctx, &p, sizeof(double) * tmp_n) != cudaSuccess)
       return ctx_fail(ctx, HYMOR_ERR_CUDA, "Krylov scratch allocation failed");
     ctx_allocs(ctx).push_back(p);
     k.tmp = static_cast<double*>(p);

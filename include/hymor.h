@@ -224,6 +224,13 @@ int hymor_bench_steps(hymor_ctx* ctx, int nsteps, uint64_t flush_bytes, float* m
  * LINEARIZE_EQUATIONS_NO_DISCONTINUITY.jl:42-288): coloured finite-difference Jacobian of the
  * residual on the device, 36 perturbed residuals batched. Keeps the blocks on the device. */
 int hymor_linearize(hymor_ctx* ctx);
+/* Device memory, in bytes, that the linear entry points of the context may keep (0, the default:
+ * what the device has): the blocks and their copies, 1.2 kB a cell each, the linearisation's
+ * workspaces, 88 bytes a cell for each of 18 to 64 lanes of perturbed states (800 x 400: 507 MB;
+ * 60 000 cells: 190 MB), and the propagators' vectors. Workspaces that would not fit the limit, or
+ * the device, get smaller (18, 9 or 3 lanes: slower, the same bits); HYMOR_ERR_CUDA where nothing
+ * fits. No counterpart in the reference. */
+int hymor_set_workspace_limit(hymor_ctx* ctx, uint64_t bytes);
 /* Copy the blocks out (Nchi*Neta*144 doubles) / in. */
 int hymor_jacobian_get(hymor_ctx* ctx, double* coef);
 int hymor_jacobian_set(hymor_ctx* ctx, const double* coef);
