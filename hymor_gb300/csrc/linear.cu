@@ -2490,13 +2490,19 @@ namespace {
 cudaError_t lin_malloc(hymor_ctx* ctx, void** p, size_t bytes);
 void lin_free(hymor_ctx* ctx, void* p, size_t bytes);
 
-// Storage of the shock-position blocks (one allocation of doubles, one of the rows).
+// Storage of the shock-position blocks and their rows.
 int ensure_shock(hymor_ctx* ctx) {
   DevCtx& d = ctx_dev(ctx);
   if (d.sj.a12) return 0;
   const long n = d.nchi;
+  // the transposed shock matvec stages 5 Nchi doubles per block
+  const long smem = shock_mv_smem(d.nchi, 1);
+  if (smem > 48 * 1024 &&
+      cudaFuncSetAttribute(k_shock_mv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return ctx_fail(ctx, HYMOR_ERR_INVALID, "perturb_shock: Nchi too large for the shock matvec's shared memory");
+  const long doubles = 11 * n + 10 * n * n;
   void* p = nullptr;
-  if (lin_malloc(ctx, &p, sizeof(double) * (8 * n + 10 * n * n + 3 * n)) != cudaSuccess)
+  if (lin_malloc(ctx, &p, sizeof(double) * doubles + sizeof(int) * n) != cudaSuccess)
     return ctx_fail(ctx, HYMOR_ERR_CUDA, "shock-block allocation failed");
   ctx_allocs(ctx).push_back(p);
   double* b = static_cast<double*>(p);
@@ -2508,14 +2514,7 @@ int ensure_shock(hymor_ctx* ctx) {
   j.a22t = j.a12t + 4 * n * n;
   j.rel_b = j.a22t + n * n;
   j.dir = j.rel_b + n;
-  if (lin_malloc(ctx, &p, sizeof(int) * n) != cudaSuccess) return ctx_fail(ctx, HYMOR_ERR_CUDA, "shock-block allocation failed");
-  ctx_allocs(ctx).push_back(p);
-  j.rows = static_cast<int*>(p);
-  // the transposed shock matvec stages 5 Nchi doubles per block
-  const long smem = shock_mv_smem(d.nchi, 1);
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(k_shock_mv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return ctx_fail(ctx, HYMOR_ERR_INVALID, "perturb_shock: Nchi too large for the shock matvec's shared memory");
+  j.rows = reinterpret_cast<int*>(b + doubles);
   return 0;
 }
 
@@ -2536,16 +2535,13 @@ int ensure_b(hymor_ctx* ctx) {
   DevCtx& d = ctx_dev(ctx);
   if (d.bq) return 0;
   void* p = nullptr;
-  if (lin_malloc(ctx, &p, sizeof(double) * 65 * (long)d.nchi) != cudaSuccess)
+  if (lin_malloc(ctx, &p, (sizeof(double) * 65 + sizeof(int)) * (long)d.nchi) != cudaSuccess)
     return ctx_fail(ctx, HYMOR_ERR_CUDA, "upstream-boundary operator allocation failed");
   ctx_allocs(ctx).push_back(p);
   d.bq = static_cast<double*>(p);
   d.bs = d.bq + 48 * d.nchi;
   d.bwork = d.bs + 12 * d.nchi;
-  if (lin_malloc(ctx, &p, sizeof(int) * d.nchi) != cudaSuccess)
-    return ctx_fail(ctx, HYMOR_ERR_CUDA, "upstream-boundary operator allocation failed");
-  ctx_allocs(ctx).push_back(p);
-  d.brows = static_cast<int*>(p);
+  d.brows = reinterpret_cast<int*>(d.bq + 65 * (long)d.nchi);
   return 0;
 }
 
@@ -2564,20 +2560,18 @@ int check_b_rows(hymor_ctx* ctx, const int* rows, int nchi, int neta) {
 int ensure_linear(hymor_ctx* ctx) {
   DevCtx& d = ctx_dev(ctx);
   if (!d.coef) {
-    void* p = nullptr;
-    if (lin_malloc(ctx, &p, sizeof(double) * 144 * d.N) != cudaSuccess)
+    void *coef = nullptr, *nz = nullptr, *work = nullptr;
+    const size_t bc = sizeof(double) * 144 * d.N, bn = 5 * d.N, bw = sizeof(double) * 8 * d.N;
+    if (lin_malloc(ctx, &coef, bc) != cudaSuccess || lin_malloc(ctx, &nz, bn) != cudaSuccess ||
+        lin_malloc(ctx, &work, bw) != cudaSuccess) {
+      lin_free(ctx, coef, bc);
+      lin_free(ctx, nz, bn);
       return ctx_fail(ctx, HYMOR_ERR_CUDA, "Jacobian allocation failed");
-    ctx_allocs(ctx).push_back(p);
-    double* coef = static_cast<double*>(p);
-    if (lin_malloc(ctx, &p, 5 * d.N) != cudaSuccess)
-      return ctx_fail(ctx, HYMOR_ERR_CUDA, "Jacobian row mask allocation failed");
-    ctx_allocs(ctx).push_back(p);
-    d.coef_nz = static_cast<unsigned char*>(p);
-    if (lin_malloc(ctx, &p, sizeof(double) * 8 * d.N) != cudaSuccess)
-      return ctx_fail(ctx, HYMOR_ERR_CUDA, "Jacobian workspace allocation failed");
-    ctx_allocs(ctx).push_back(p);
-    d.jwork = static_cast<double*>(p);
-    d.coef = coef;
+    }
+    for (void* p : {coef, nz, work}) ctx_allocs(ctx).push_back(p);
+    d.coef_nz = static_cast<unsigned char*>(nz);
+    d.jwork = static_cast<double*>(work);
+    d.coef = static_cast<double*>(coef);
   }
   return 0;
 }
