@@ -15,6 +15,8 @@ namespace hymor {
 void flux_kernel_setup();
 void linear_state_release(void* p);
 int ctx_check_waits(hymor_ctx* c);
+bool linear_spare_release(hymor_ctx* ctx);
+cudaError_t ctx_malloc(hymor_ctx* ctx, void** p, size_t bytes);
 }
 
 using namespace hymor;
@@ -929,7 +931,7 @@ int hymor_set_upstream(hymor_ctx* ctx, const double* cols) {
     d.res_up = nullptr;
     return 0;
   }
-  if (!d.res_up) CU(cudaMalloc(&d.res_up, sizeof(double) * 4 * d.nchi));
+  if (!d.res_up) CU(ctx_malloc(ctx, (void**)&d.res_up, sizeof(double) * 4 * d.nchi));
   CU(cudaMemcpyAsync(d.res_up, cols, sizeof(double) * 4 * d.nchi, cudaMemcpyHostToDevice, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
   return 0;
@@ -973,7 +975,7 @@ int hymor_bench_steps(hymor_ctx* ctx, int nsteps, uint64_t flush_bytes, float* m
   if (flush_bytes > ctx->flush_bytes) {
     if (ctx->flush_buf) CU(cudaFree(ctx->flush_buf));
     ctx->flush_buf = nullptr;
-    CU(cudaMalloc(&ctx->flush_buf, flush_bytes));
+    CU(ctx_malloc(ctx, (void**)&ctx->flush_buf, flush_bytes));
     ctx->flush_bytes = flush_bytes;
   }
   if (nsteps > 0) refresh_sound(ctx, ctx->d.cfg.shock_enabled);
@@ -1029,7 +1031,7 @@ int hymor_autotune(hymor_ctx* ctx, int steps, int32_t* choice, float* ms_per_ste
   size_t total = 0;
   for (const Part& q : parts) total += (q.bytes + 255) & ~(size_t)255;
   unsigned char* save = nullptr;
-  CU(cudaMalloc(&save, total));
+  CU(ctx_malloc(ctx, (void**)&save, total));
   auto copy = [&](bool store) -> int {
     size_t off = 0;
     for (const Part& q : parts) {
@@ -1156,6 +1158,7 @@ int hymor_set_step_viscous(hymor_ctx* ctx, int mode) {
 int hymor_set_expm_arith(hymor_ctx* ctx, int mode) {
   if (!ctx || mode < 0 || mode > 1) return HYMOR_ERR_INVALID;
   ctx->d.expm_ff = mode;
+  if (!mode) linear_spare_release(ctx);
   return 0;
 }
 
@@ -1278,7 +1281,7 @@ int hymor_synchronize(hymor_ctx* ctx) {
 int hymor_device_alloc(hymor_ctx* ctx, uint64_t bytes, void** dptr) {
   if (!ctx || !dptr) return HYMOR_ERR_INVALID;
   TRY(set_device(ctx));
-  CU(cudaMalloc(dptr, bytes));
+  CU(ctx_malloc(ctx, dptr, bytes));
   return 0;
 }
 

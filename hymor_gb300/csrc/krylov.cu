@@ -27,6 +27,7 @@ DevCtx& ctx_dev(hymor_ctx* c);
 cudaStream_t ctx_stream(hymor_ctx* c);
 int ctx_fail(hymor_ctx* c, int code, const char* msg);
 int ctx_check_waits(hymor_ctx* c);  // reports (once) a resident propagation that gave up
+cudaError_t ctx_malloc(hymor_ctx* ctx, void** p, size_t bytes);
 }  // namespace hymor
 
 using namespace hymor;
@@ -51,7 +52,7 @@ struct DevBuf {
   DevBuf& operator=(const DevBuf&) = delete;
   int alloc(hymor_ctx* c, size_t doubles) {
     ctx = c;
-    return cu(c, cudaMalloc((void**)&p, sizeof(double) * std::max<size_t>(doubles, 1)), "Krylov buffer allocation");
+    return cu(c, ctx_malloc(c, (void**)&p, sizeof(double) * std::max<size_t>(doubles, 1)), "Krylov buffer allocation");
   }
   ~DevBuf() {
     if (p) {

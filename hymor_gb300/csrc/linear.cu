@@ -25,6 +25,10 @@ DevCtx& ctx_dev(hymor_ctx* c);
 cudaStream_t ctx_stream(hymor_ctx* c);
 int ctx_fail(hymor_ctx* c, int code, const char* msg);
 int ctx_check_waits(hymor_ctx* c);  // reports (once) a resident propagation that gave up
+int ctx_select_device(hymor_ctx* c);
+bool linear_spare_release(hymor_ctx* ctx);
+cudaError_t ctx_malloc(hymor_ctx* ctx, void** p, size_t bytes);
+cudaError_t ctx_malloc_async(hymor_ctx* ctx, void** p, size_t bytes);
 std::vector<void*>& ctx_allocs(hymor_ctx* c);
 void*& ctx_linear_state(hymor_ctx* c);
 void launch_shock_bc_flags(const DevCtx& d, bool on_S, bool copy_pts, bool do_shock, bool do_bc, int a_mode,
@@ -1974,9 +1978,9 @@ void launch_k_matvec(const DevCtx& d, int k, const MvArgs& a, int grid, int th, 
 // Batches that take the fixed-point matvec: those where even the first one after a write of the
 // blocks, which makes their parts (~0.35 ns a cell and their storage, against ~66 ps saved per
 // cell and vector), is no slower than in FP64. Repeated, smaller ones would gain too (300 x 200,
-// 16 vectors: 173 -> 125 us), but their first took 75 us longer.
+// 16 vectors: 173 -> 125 us), but their first took 75 us longer. hymor_set_expm_arith(0) keeps FP64.
 static bool fx_takes(const DevCtx& d, int k) {
-  return k >= 8 && (long)(k - 6) * d.N >= 1000000 && !mv_one(d.N, k, d.sms);
+  return d.expm_ff && k >= 8 && (long)(k - 6) * d.N >= 1000000 && !mv_one(d.N, k, d.sms);
 }
 
 // the integer parts of the blocks for one direction, made again after each write of the blocks
@@ -2486,8 +2490,9 @@ using namespace hymor;
 
 namespace {
 // Device memory that the context's linear entry points keep: counted against
-// hymor_set_workspace_limit, and for the context's life unless lin_free gives it back.
-cudaError_t lin_malloc(hymor_ctx* ctx, void** p, size_t bytes);
+// hymor_set_workspace_limit, and for the context's life unless lin_free gives it back. What is
+// not to be had at first is tried again without the fixed-point parts (spare: it is they).
+cudaError_t lin_malloc(hymor_ctx* ctx, void** p, size_t bytes, bool spare = false);
 void lin_free(hymor_ctx* ctx, void* p, size_t bytes);
 
 // Storage of the shock-position blocks and their rows.
@@ -2600,6 +2605,9 @@ struct KrylovScratch {
 // use, released by hymor_ctx_destroy).
 struct LinearState {
   size_t used = 0, limit = 0;  // bytes of lin_malloc, and their limit (0: none)
+  void* fx_mem[2] = {};        // the fixed-point parts of each direction and their size
+  size_t fx_bytes = 0;
+  int fx_refused[2] = {-1, -1};  // the write of the blocks whose parts did not fit
   ExpmCache expm;
   KrylovScratch kry;
   bool res_ready = false;  // k_expm_res_ff's shared memory is set
@@ -2615,11 +2623,30 @@ LinearState& linear_state(hymor_ctx* ctx) {
 }
 ExpmCache& expm_cache(hymor_ctx* ctx) { return linear_state(ctx).expm; }
 
-cudaError_t lin_malloc(hymor_ctx* ctx, void** p, size_t bytes) {
+// whether the context's stream is being captured (or in error)
+bool stream_captured(hymor_ctx* ctx) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(ctx_stream(ctx), &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+// an error reported here, and not again by a later check of the launches
+cudaError_t settled(cudaError_t e) {
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+// an allocation, and if there is no room for it another try without the fixed-point parts, which
+// then stay away until the next write of the blocks
+template <class Take>
+cudaError_t with_spare(hymor_ctx* ctx, Take take) {
+  const cudaError_t e = settled(take());
+  if (e != cudaErrorMemoryAllocation || !linear_spare_release(ctx)) return e;
+  for (int& v : linear_state(ctx).fx_refused) v = ctx_dev(ctx).coef_version;
+  return settled(take());
+}
+cudaError_t lin_malloc(hymor_ctx* ctx, void** p, size_t bytes, bool spare) {
   LinearState& s = linear_state(ctx);
-  const cudaError_t e = s.limit && s.used + bytes > s.limit ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
+  auto take = [&]() { return s.limit && s.used + bytes > s.limit ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes); };
+  const cudaError_t e = spare ? settled(take()) : with_spare(ctx, take);
   if (e == cudaSuccess) s.used += bytes;
-  else cudaGetLastError();  // (a later check of the launches would report it again)
   return e;
 }
 void lin_free(hymor_ctx* ctx, void* p, size_t bytes) {
@@ -2842,10 +2869,39 @@ int expm_cooperative(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
 }  // namespace
 
 namespace hymor {
+// Gives back the fixed-point parts of the blocks, which the FP64 matvec can do without; false
+// where there are none, or the context's stream is being captured.
+bool linear_spare_release(hymor_ctx* ctx) {
+  LinearState* s = static_cast<LinearState*>(ctx_linear_state(ctx));
+  if (!s || (!s->fx_mem[0] && !s->fx_mem[1]) || stream_captured(ctx)) return false;
+  DevCtx& d = ctx_dev(ctx);
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // another stream's capture may be under way
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  cudaStreamSynchronize(ctx_stream(ctx));
+  for (int t = 0; t < 2; ++t) {
+    lin_free(ctx, s->fx_mem[t], s->fx_bytes);
+    s->fx_mem[t] = nullptr;
+    d.fx_part[t] = nullptr;
+    d.fx_ex[t] = nullptr;
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return true;
+}
+// The context's other device memory, in and out of stream order: what is not to be had at first
+// is tried again without the fixed-point parts.
+cudaError_t ctx_malloc(hymor_ctx* ctx, void** p, size_t bytes) {
+  return with_spare(ctx, [&]() { return cudaMalloc(p, bytes); });
+}
+cudaError_t ctx_malloc_async(hymor_ctx* ctx, void** p, size_t bytes) {
+  return with_spare(ctx, [&]() { return cudaMallocAsync(p, bytes, ctx_stream(ctx)); });
+}
+
 // Called by hymor_ctx_destroy after its stream has drained.
 void linear_state_release(void* p) {
   if (!p) return;
   LinearState* s = static_cast<LinearState*>(p);
+  for (void* q : s->fx_mem)
+    if (q) cudaFree(q);
   if (s->expm.buf) cudaFree(s->expm.buf);
   for (int g = 0; g < kLaneGroups; ++g) {
     if (s->lanes.st[g]) cudaStreamDestroy(s->lanes.st[g]);
@@ -2893,7 +2949,9 @@ int hymor_linearize(hymor_ctx* ctx) {
 
 int hymor_set_workspace_limit(hymor_ctx* ctx, uint64_t bytes) {
   if (!ctx) return HYMOR_ERR_INVALID;
-  linear_state(ctx).limit = bytes;
+  LinearState& s = linear_state(ctx);
+  s.limit = bytes;
+  s.fx_refused[0] = s.fx_refused[1] = -1;
   return 0;
 }
 
@@ -2966,7 +3024,7 @@ int hymor_jacobian_get(hymor_ctx* ctx, double* coef) {
   cudaStream_t st = ctx_stream(ctx);
   double* tmp = nullptr;
   int r;
-  if ((r = cuda_check(ctx, cudaMallocAsync((void**)&tmp, sizeof(double) * 144 * d.N, st)))) return r;
+  if ((r = cuda_check(ctx, ctx_malloc_async(ctx, (void**)&tmp, sizeof(double) * 144 * d.N)))) return r;
   k_planes_to_blocks<<<grid_for(d.N * 144, 256), 256, 0, st>>>(d.coef, tmp, d.N);
   r = cuda_check(ctx, cudaMemcpyAsync(coef, tmp, sizeof(double) * 144 * d.N, cudaMemcpyDeviceToHost, st));
   cudaFreeAsync(tmp, st);
@@ -2981,7 +3039,7 @@ int hymor_jacobian_set(hymor_ctx* ctx, const double* coef) {
   DevCtx& d = ctx_dev(ctx);
   cudaStream_t st = ctx_stream(ctx);
   double* tmp = nullptr;
-  if ((r = cuda_check(ctx, cudaMallocAsync((void**)&tmp, sizeof(double) * 144 * d.N, st)))) return r;
+  if ((r = cuda_check(ctx, ctx_malloc_async(ctx, (void**)&tmp, sizeof(double) * 144 * d.N)))) return r;
   r = cuda_check(ctx, cudaMemcpyAsync(tmp, coef, sizeof(double) * 144 * d.N, cudaMemcpyHostToDevice, st));
   cudaMemsetAsync(d.coef_nz + d.N, 0, 4 * d.N, st);
   k_blocks_to_planes<<<grid_for(d.N * 144, 256), 256, 0, st>>>(tmp, d.coef, d.coef_nz + d.N, d.N);
@@ -2998,24 +3056,24 @@ int hymor_jacobian_set(hymor_ctx* ctx, const double* coef) {
 static bool fx_ready(hymor_ctx* ctx, int k, int transpose) {
   DevCtx& d = ctx_dev(ctx);
   const int t = transpose != 0;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (!fx_takes(d, k) || cudaStreamIsCapturing(ctx_stream(ctx), &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
-    return false;
+  if (!fx_takes(d, k) || stream_captured(ctx)) return false;
   if (!d.fx_part[t]) {
-    void *p = nullptr, *e = nullptr;
+    LinearState& s = linear_state(ctx);
+    if (s.fx_refused[t] == d.coef_version || ctx_select_device(ctx)) return false;
+    void* p = nullptr;
+    const size_t parts = sizeof(int2) * 144 * d.N, bytes = parts + sizeof(short) * 16 * d.N;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     cudaThreadExchangeStreamCaptureMode(&mode);
-    const bool ok = cudaMalloc(&p, sizeof(int2) * 144 * d.N) == cudaSuccess && cudaMalloc(&e, sizeof(short) * 16 * d.N) == cudaSuccess;
+    const cudaError_t e = lin_malloc(ctx, &p, bytes, true);
     cudaThreadExchangeStreamCaptureMode(&mode);
-    if (!ok) {
-      if (p) cudaFree(p);
-      cudaGetLastError();
+    if (e != cudaSuccess) {
+      s.fx_refused[t] = d.coef_version;  // tried again after the next write of the blocks
       return false;
     }
-    ctx_allocs(ctx).push_back(p);
-    ctx_allocs(ctx).push_back(e);
+    s.fx_mem[t] = p;
+    s.fx_bytes = bytes;
     d.fx_part[t] = static_cast<int2*>(p);
-    d.fx_ex[t] = static_cast<short*>(e);
+    d.fx_ex[t] = reinterpret_cast<short*>(static_cast<char*>(p) + parts);
     d.fx_version[t] = d.coef_version - 1;
   }
   launch_fx_build(d, t, ctx_stream(ctx));
@@ -3038,8 +3096,8 @@ int hymor_matvec(hymor_ctx* ctx, int k, const double* X, double* Y, int transpos
   const size_t bytes = sizeof(double) * op_size(d) * (size_t)k;
   double *dx = nullptr, *dy = nullptr;
   int r;
-  if ((r = cuda_check(ctx, cudaMallocAsync((void**)&dx, bytes, st)))) return r;
-  if ((r = cuda_check(ctx, cudaMallocAsync((void**)&dy, bytes, st)))) return r;
+  if ((r = cuda_check(ctx, ctx_malloc_async(ctx, (void**)&dx, bytes)))) return r;
+  if ((r = cuda_check(ctx, ctx_malloc_async(ctx, (void**)&dy, bytes)))) return r;
   cudaMemcpyAsync(dx, X, bytes, cudaMemcpyHostToDevice, st);
   launch_matvec(d, k, dx, dy, transpose, 1.0, st, 0, fx_ready(ctx, k, transpose));
   cudaMemcpyAsync(Y, dy, bytes, cudaMemcpyDeviceToHost, st);
@@ -3094,7 +3152,7 @@ int hymor_expm_apply_dev(hymor_ctx* ctx, int k, double dt, int nsteps, int order
   const size_t n = op_size(d) * (size_t)k;
   double* work = nullptr;
   int r;
-  if ((r = cuda_check(ctx, cudaMallocAsync((void**)&work, 3 * n * sizeof(double), st)))) return r;
+  if ((r = cuda_check(ctx, ctx_malloc_async(ctx, (void**)&work, 3 * n * sizeof(double))))) return r;
   launch_expm(d, k, dt, nsteps, order, dX, dY, transpose, work, st);
   cudaFreeAsync(work, st);
   return cuda_check(ctx, cudaGetLastError());
@@ -3128,8 +3186,8 @@ int hymor_expm_apply(hymor_ctx* ctx, int k, double dt, int nsteps, int order, co
   const size_t bytes = sizeof(double) * op_size(d) * (size_t)k;
   double *dx = nullptr, *dy = nullptr;
   int r;
-  if ((r = cuda_check(ctx, cudaMallocAsync((void**)&dx, bytes, st)))) return r;
-  if ((r = cuda_check(ctx, cudaMallocAsync((void**)&dy, bytes, st)))) return r;
+  if ((r = cuda_check(ctx, ctx_malloc_async(ctx, (void**)&dx, bytes)))) return r;
+  if ((r = cuda_check(ctx, ctx_malloc_async(ctx, (void**)&dy, bytes)))) return r;
   cudaMemcpyAsync(dx, X, bytes, cudaMemcpyHostToDevice, st);
   r = hymor_expm_apply_dev(ctx, k, dt, nsteps, order, dx, dy, transpose);
   if (!r) cudaMemcpyAsync(Y, dy, bytes, cudaMemcpyDeviceToHost, st);
@@ -3287,7 +3345,7 @@ static int recept_prep(hymor_ctx* ctx, int k, int nw, const double* w, const dou
   if (!d.bq) return ctx_fail(ctx, HYMOR_ERR_NOT_READY, "no upstream-boundary operator: call hymor_linearize_b");
   cudaStream_t st = ctx_stream(ctx);
   int r;
-  if ((r = cuda_check(ctx, cudaMallocAsync((void**)dw, sizeof(double) * nw, st)))) return r;
+  if ((r = cuda_check(ctx, ctx_malloc_async(ctx, (void**)dw, sizeof(double) * nw)))) return r;
   return cuda_check(ctx, cudaMemcpyAsync(*dw, w, sizeof(double) * nw, cudaMemcpyHostToDevice, st));
 }
 
@@ -3321,7 +3379,7 @@ int hymor_recept_expm_dev(hymor_ctx* ctx, int k, int nw, const double* w, double
     a.nw = nw;
     a.divide = 1;
     double* work = nullptr;
-    if (!(r = cuda_check(ctx, cudaMallocAsync((void**)&work, sizeof(double) * 2 * a.ld * a.k, st)))) {
+    if (!(r = cuda_check(ctx, ctx_malloc_async(ctx, (void**)&work, sizeof(double) * 2 * a.ld * a.k)))) {
       r = cuda_check(ctx, launch_expm_ext(d, a, adjoint, nsteps, order, dX, dY, work, st));
       cudaFreeAsync(work, st);
     }
@@ -3330,7 +3388,7 @@ int hymor_recept_expm_dev(hymor_ctx* ctx, int k, int nw, const double* w, double
   }
   double* work = nullptr;
   const long n = 2L * k * recept_size(d, nw);
-  if ((r = cuda_check(ctx, cudaMallocAsync((void**)&work, sizeof(double) * 2 * n, st)))) return r;
+  if ((r = cuda_check(ctx, ctx_malloc_async(ctx, (void**)&work, sizeof(double) * 2 * n)))) return r;
   launch_recept_expm(d, k, nw, dw, dt, nsteps, order, dX, dY, adjoint, work, st);
   cudaFreeAsync(work, st);
   cudaFreeAsync(dw, st);

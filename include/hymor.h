@@ -141,8 +141,9 @@ int hymor_set_cfl_screen(hymor_ctx* ctx, int on);
  * propagations that run as one cooperative launch (the stencil operator, Taylor degree >= 2,
  * 16 launches or more) keep their Taylor terms and running sum as float-float pairs and
  * multiply by a float-float copy of the blocks on the FP32 pipe, ~2^-47 per operation (the
- * input and output vectors stay FP64); mode 0: FP64. hymor_matvec_dev, the propagators with
- * the shock-position unknowns and the receptivity operator are FP64 in either mode. The
+ * input and output vectors stay FP64); mode 0: FP64. The propagators with the shock-position
+ * unknowns and the receptivity operator are FP64 in either mode; large batches of hymor_matvec
+ * form their FP64 results in fixed point in mode 1 and with FP64 instructions in mode 0 (there). The
  * eigen and transient-growth solvers (hymor_eigs, hymor_tg_gain) use the context's mode. */
 int hymor_set_expm_arith(hymor_ctx* ctx, int mode);
 
@@ -262,7 +263,15 @@ int hymor_shock_fields(hymor_ctx* ctx, double* beta, double* rel_vel);
  * hymor_operator_size), host pointers. Replaces the CuSparse SpMV `mul!(term, A, v)` of
  * Eigenvalues/ARNOLDI_POWER_GPU.jl:73 (and its transpose, TRANSIENT_GROWTH_DOWNSTREAM.jl:75). */
 int hymor_matvec(hymor_ctx* ctx, int k, const double* X, double* Y, int transpose);
-/* Same on device pointers (no copies). */
+/* Same on device pointers (no copies). k vectors with k >= 8 and (k - 6) Nchi Neta >= 1e6 have
+ * their products formed in fixed point (58-bit factors, exact sums of nine; no further from the
+ * exact sums than an FP64 chain) unless hymor_set_expm_arith(0) asks for FP64 instructions. The
+ * first such batch of each direction allocates the blocks' integer parts, 1184 bytes a cell
+ * (800 x 400: 379 MB), which the context keeps; a write of the blocks makes them again with the
+ * next batch. FP64 instructions serve, with results that differ in the last places, where that
+ * memory is not to be had (device, hymor_set_workspace_limit) and while the context's stream is
+ * captured; the parts give way to any other allocation of the context that would fail beside
+ * them, and hymor_set_expm_arith(0) frees them. Smaller batches allocate nothing. */
 int hymor_matvec_dev(hymor_ctx* ctx, int k, const double* dX, double* dY, int transpose);
 /* Timing of hymor_matvec_dev (no counterpart in the reference): reps repetitions of one
  * launch over the k vectors (per_vector 0), or of k launches of one vector each
