@@ -2715,8 +2715,9 @@ void launch_flux_class(const DevCtx& d, bool on_S, double* const out[4], int til
   // its own (180 x 60, the residual without its copy to the host, with k_thermo_sound and
   // k_bc_edges_one: 48 -> 36 us; with WIDE blocks too, and its copy: 59.4 -> 46.3 us)
   const long halves = (long)flux_tiles_x(d) * ((d.neta + TY / 2 - 1) / (TY / 2));
+  // (under the split tiling, the default: the tilings of 31 x 8 and 31 x 16 cells are used as set)
   const bool few = tile_class < 0 && !ffv && d.lanes == 1 && halves <= d.sms;
-  const bool half = (flux_split(d) && tile_class >= 0 && d.tiles) || few;
+  const bool half = flux_split(d) && ((tile_class >= 0 && d.tiles) || few);
   const int rows = half ? TY / 2 : flux_rows(d);
   const bool wide = half && d.lanes == 1 && halves <= kWideTiles * d.sms;
   const bool tma = d.tma && !half;

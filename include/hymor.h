@@ -169,7 +169,7 @@ int hymor_set_wait_limit(hymor_ctx* ctx, int polls);
  * tile computes it, and the staged halo holds the same values). hymor_set_flux_tiling sets one
  * directly (default: the split tiling, 1 spare slot, TMA when Nchi is even: with the split
  * tiling only the whole-grid flux of the residual and of the classical RK4 scheme stages its
- * halo by TMA). */
+ * halo by TMA, and a residual whose half tiles are no more than the SMs runs as those). */
 int hymor_autotune(hymor_ctx* ctx, int steps, int32_t* choice, float* ms_per_step);
 int hymor_set_flux_tiling(hymor_ctx* ctx, int rows, int spare, int tma);
 
