@@ -447,10 +447,12 @@ __device__ __forceinline__ void matvec_multi(const MvArgs& a) {
 // entries (L e_i stays exact: an entry above the line has all its 53 bits within the 58), for
 // tiles with an infinity or a NaN, and for exponents beyond +-900 (subnormal factors among them).
 //
-// What bounds it: the integer multiply pipe, 432 wide multiply-adds per cell and vector (FP64:
-// 144 multiply-adds at a fifteenth of that rate, 0.98 of the pipe by ncu), 51 % busy beside the
-// shifts of the alignment and the parts (42 %) and the FP64 rows (11 %). 800 x 400, 64 vectors:
-// 3.64 -> 2.29 ms. Error against sums in 113 bits, relative in the 2-norm, random rows of
+// What bounds it: waiting, with four warps per sub-partition (124 registers a thread): 48 % of the
+// issue slots are used, and the stalls are the multiplies' fixed latency (2.3 cycles an issue) and
+// the loads of the blocks' parts (1.7). No pipe is full: the integer multiplies, 432 wide
+// multiply-adds per cell and vector (FP64: 144 multiply-adds at a fifteenth of that rate, 0.98 of
+// the pipe), keep the heavy half of the FMA pipe 52 % busy, the shifts of the alignment and the
+// parts the ALU 44 %, the FP64 rows that pipe 11 %. 800 x 400, 64 vectors: 3.64 -> 2.29 ms. Error against sums in 113 bits, relative in the 2-norm, random rows of
 // magnitudes 1e-4 .. 2 and component scales 1e-2 .. 1e2: 5.3e-17 (the FP64 chain: 2.1e-16).
 constexpr int kFxVecs = 4, kFxRows = 4;
 constexpr int kFxHx = 34, kFxHalo = kFxHx * (kFxRows + 2);
@@ -873,10 +875,10 @@ __device__ __forceinline__ void matvec_cell_ff(const MvFf& a) {
 
 // A batch of vectors: a block takes a tile of 32 x kFfRows cells and a chunk of up to kVecChunk
 // vectors, stages the vectors' tile and halo in shared memory, and a thread forms the outputs of
-// its cell for the chunk (four components each). What bounds it is the FP32 pipe (~1950
-// instructions per cell and vector, 16 independent chains per thread) and the latency of the 16
-// pairs of a neighbour block, which four blocks of four warps on an SM, each at its own place,
-// hide in part (FP32 pipe 36 %, issue slots 46 % busy by ncu). Before, a thread per component
+// its cell for the chunk (four components each). What bounds it is the latency of the 16 pairs of a
+// neighbour block (4.0 of 8.7 cycles an issue wait for loads), which four blocks of four warps on
+// an SM, each at its own place, hide in part: the ~1950 FP32 instructions per cell and vector, 16
+// independent chains per thread, keep that pipe 36 % and the issue slots 46 % busy. Before, a thread per component
 // read the inputs from global memory for every neighbour: 38 x 4 loads of L2 per cell and vector.
 // 600 x 300, 8 vectors, adjoint, us per matvec of the batch: 279 before; 178 in tiles of 32 x 8
 // cells; 159 in tiles of 32 x 4 with the cells without entries left out (187 with the pairs by
