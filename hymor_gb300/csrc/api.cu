@@ -205,7 +205,8 @@ void face_geometry(const hymor_config& c, const hymor_mesh& m, std::vector<doubl
 }
 
 int enqueue_step(hymor_ctx* ctx, bool with_events) {
-  DevCtx& d = ctx->d;
+  DevCtx d = ctx->d;  // as the captured launches see it
+  d.spl_stored = d.cfg.rk_variant == 0 && step_stores_fitted(d);
   cudaStream_t st = ctx->stream, sx = ctx->side;
   const hymor_config& c = d.cfg;
   const bool shock = c.shock_enabled;
@@ -768,6 +769,7 @@ int hymor_ctx_create(const hymor_config* cfg, const hymor_mesh* mesh, hymor_ctx*
   d.lanes = 1;
   d.lane_stride = 0;
   d.spl_shared = 0;
+  d.spl_stored = 0;
   d.flux_rows = 4;  // the split tiling
   d.flux_spare = 1;
   d.tma = make_flux_maps(d);

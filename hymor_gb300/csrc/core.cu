@@ -406,7 +406,7 @@ __device__ void edge_bc_point(const hymor_config& c, const EdgeCtx& e, const Dev
 //   k_bc_edges       the two boundary phases (chi edges, then eta edges, whose corners
 //                    read the chi ghosts), one launch each, one thread per edge point
 // Spline workspace (units of n = Nchi doubles): 0 knots, 1-2 ordinates x/y, 3-4
-// second derivatives x/y, 5-6 unused, 7-11 per-row d0 d1 d2 rhs_x rhs_y,
+// second derivatives x/y, 5-6 fitted values x/y (DevCtx::spl_stored), 7-11 per-row d0 d1 d2 rhs_x rhs_y,
 // 12-14 FP64 Cholesky factors of the fallback solve, 15 interval reciprocals
 // 1/(x[k+1] - x[k]).
 
@@ -425,7 +425,7 @@ struct SplineArgs {
   ShockPts pts, pS;
   double* ws;
   double lam;
-  int n, copy_pts;
+  int n, copy_pts, stored;
   long lane;  // offset of the next lane's ws and pts (grid z; kernels.h, DevCtx::lane_stride)
 };
 
@@ -739,7 +739,6 @@ __global__ void __launch_bounds__(kSplineThreads) k_spline_fit(SplineArgs A) {
   float* ey = ex + mp;
   const double lam = A.lam;
   for (int i = tid; i < n; i += nt) { cx[i] = 0; cy[i] = 0; }
-  if (m <= 0) return;
   const double* ih = ws + 15 * n;
   float qloc = 0.f, yloc = 0.f;  // max 2 (1/h_{k-1} + 1/h_k) and max |y| over this thread's rows
   for (int j = tid; j < m; j += nt) {
@@ -819,6 +818,10 @@ __global__ void __launch_bounds__(kSplineThreads) k_spline_fit(SplineArgs A) {
       chol_solve_f64(m, d0, d1, d2, rx, ry, ws + 12 * n, ws + 13 * n, ws + 14 * n, cx, cy);
     __syncthreads();
   }
+  if (A.stored && tid < n) {
+    ws[5 * n + tid] = spline_g(n, ih, yx, cx, lam, tid);
+    ws[6 * n + tid] = spline_g(n, ih, yy, cy, lam, tid);
+  }
 }
 
 struct ColArgs {
@@ -834,6 +837,7 @@ struct ColArgs {
   DevMesh m;
   double cY, cS;
   double lam;                             // of the spline fit
+  int stored;                             // the fit left the fitted values (DevCtx::spl_stored)
   const double* up_cols;                  // per-column upstream state (4 x Nchi) or null
   int move, on_S;
   int disturbed;                          // any freestream disturbance amplitude non-zero
@@ -844,13 +848,17 @@ struct ColArgs {
   long lane, ws_lane;  // offsets of the next lane's buffers and spline workspace (grid z)
 };
 
-// value and slope of the fitted spline at t (Linear() extrapolation outside the knots); the
-// fitted values of the two knots it needs are formed here, by every column's threads, not by the
-// one block of the fit
-__device__ void spline_at(int n, const double* xs, const double* ys, const double* gam, const double* ih, double lam,
-                          double t, int guess, double& val, double& der) {
+// value and slope of the fitted spline at t (Linear() extrapolation outside the knots), from the
+// fitted values gs or, without them, from the ordinates
+__device__ void spline_at(int n, const double* xs, const double* ys, const double* gs, const double* gam,
+                          const double* ih, double lam, double t, int guess, double& val, double& der) {
   double g0, g1;  // of knots k, k + 1
   auto fitted = [&](int k) {
+    if (gs) {
+      g0 = gs[k];
+      g1 = gs[k + 1];
+      return;
+    }
     g0 = spline_g(n, ih, ys, gam, lam, k);
     g1 = spline_g(n, ih, ys, gam, lam, k + 1);
   };
@@ -921,6 +929,8 @@ __global__ void __launch_bounds__(kColThreads) k_shock_columns(ColArgs A) {
   const double* cys = xs + 4 * nchi;
   const double* yxs = xs + nchi;
   const double* yys = xs + 2 * nchi;
+  const double* gxs = A.stored ? xs + 5 * nchi : nullptr;
+  const double* gys = A.stored ? xs + 6 * nchi : nullptr;
   const double* ih = xs + 15 * nchi;
   const ShockPts pts = lane_pts(A.pts, off);
   const Cons q = lane_cons(A.tgt, off);
@@ -930,7 +940,7 @@ __global__ void __launch_bounds__(kColThreads) k_shock_columns(ColArgs A) {
   // and its slope at the column's abscissa
   if (act && w < 2) {
     double v, dv;
-    spline_at(nchi, xs, w == 0 ? yxs : yys, w == 0 ? cxs : cys, ih, A.lam, A.m.chi1[i], i - 1, v, dv);
+    spline_at(nchi, xs, w == 0 ? yxs : yys, w == 0 ? gxs : gys, w == 0 ? cxs : cys, ih, A.lam, A.m.chi1[i], i - 1, v, dv);
     (w == 0 ? sh.xv : sh.yv)[lane] = v;
     (w == 0 ? sh.xd : sh.yd)[lane] = dv;
   } else if (act) {
@@ -2458,6 +2468,21 @@ void launch_update_thermo(const DevCtx& d, int mode, double cY, double cS, cudaS
   k_update_thermo<<<grid_for(d.G, 256), 256, 0, st>>>(upd_args(d, mode, cY, cS));
 }
 
+// Who forms the fitted values g = y - lam Q gamma that the columns read (the same bits either way):
+// every column its own two, or in the step, by this rule, the fit, a knot per thread. In the one block of the fit they cost up
+// to 4 us on the chain of a large grid's or a very small one's stage; in the columns their ~14 FP64
+// instructions wait for the FP64 pipe behind an interior flux that starts with them, which a flux
+// of two to four half tiles per SM does not outlast. us for four steps, in the fit and in the
+// columns, cylinder (cone): 300 x 150 933 (1050) and 943 (1094), 420 x 100 930 (1032) and 977
+// (1115), 500 x 120 979 (1071) and 1006 (1155), 382 x 187 1013 (1099) and 1047 (1154); fewer half
+// tiles: 500 x 60 936 (1039) and 910 (1020); more: 420 x 200 1049 (1200) and 1010 (1121), 1024 x 300
+// 1557 and 1532, 1200 x 400 (2237) and (2023); more columns: 800 x 60 1022 (1146) and 989 (1102).
+// (A residual has no flux beside its chain: 420 x 100 96.8 and 94.2.)
+bool step_stores_fitted(const DevCtx& d) {
+  const long halves = flux_tiles_max(d);
+  return d.nchi <= kSplineThreads / 2 && halves > 2 * d.sms && 5 * halves <= 21 * d.sms;
+}
+
 void launch_spline(const DevCtx& d, bool on_S, bool copy_pts, cudaStream_t st) {
   const hymor_config& c = d.cfg;
   if (!c.shock_enabled) return;
@@ -2468,6 +2493,7 @@ void launch_spline(const DevCtx& d, bool on_S, bool copy_pts, cudaStream_t st) {
   sa.lam = (1 - c.spline_param) / c.spline_param;
   sa.n = d.nchi;
   sa.copy_pts = copy_pts;
+  sa.stored = d.spl_stored;
   sa.lane = d.lane_stride;
   // (the single-lane kernels without the lane offsets: the RK step's serial chain waits for them)
   const bool ln = d.lanes > 1;
@@ -2490,6 +2516,7 @@ void launch_columns_bc(const DevCtx& d, bool on_S, bool move, double cY, double 
     ca.pS = d.Sp;
     ca.ws = d.spl;
     ca.lam = (1 - c.spline_param) / c.spline_param;
+    ca.stored = d.spl_stored;
     ca.cell_idx = d.cell_idx;
     ca.beta = d.beta;
     ca.speed_x = d.speed_x;

@@ -101,6 +101,7 @@ struct DevCtx {
   int lanes;
   long lane_stride;
   int spl_shared;
+  int spl_stored;  // the fit leaves the fitted values and the columns read them (step_stores_fitted)
 };
 
 // Unknowns of the linearised operator: 4N, plus Nchi with the shock blocks.
@@ -141,6 +142,7 @@ void launch_classify_tiles(const DevCtx& d, cudaStream_t st);
 // the ghosted rows jlo <= j < jhi their flux reads.
 void launch_band_tiles(const DevCtx& d, const int* rows, int& jlo, int& jhi, cudaStream_t st);
 int flux_tiles(const DevCtx& d);
+bool step_stores_fitted(const DevCtx& d);
 int flux_tiles_max(const DevCtx& d);  // the tile count of the smallest tile height (list sizes)
 // UPDATE_FLOW_CELLS part 1: detect shocked cells, upstream fill, extrapolation (on S).
 void launch_flow_cells(const DevCtx& d, cudaStream_t st);
